@@ -10,6 +10,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "rt_fast_math.h"
+
 namespace relsim {
 
 // Dormand-Prince 5(4) tableau (rk45_adaptive.hpp:196-203).
@@ -59,12 +61,18 @@ __device__ __forceinline__ float rt_sqrt<float>(float v) {  // MUFU rsqrt based
 }
 
 // Boyer-Lindquist r of a Kerr-Schild point (kerr_schild_null_integrator.hpp:32-36).
-template <typename T>
+// FAST (FP64): the root without special cases (rt_fast_math.h); a NaN stays one.
+template <typename T, bool FAST = false>
 __device__ __forceinline__ T bl_r2(T x, T y, T z, T a2) {
     const T z2 = z * z;
     const T diff = x * x + y * y + z2 - a2;
-    const T r2 = T(0.5) * (diff + rt_sqrt<T>(diff * diff + T(4) * a2 * z2));
-    return fmax(r2, T(1e-24));
+    if constexpr (FAST) {
+        const T r2 = T(0.5) * (diff + fast_sqrt(diff * diff + T(4) * a2 * z2));
+        return (r2 < T(1e-24)) ? T(1e-24) : r2;
+    } else {
+        const T r2 = T(0.5) * (diff + rt_sqrt<T>(diff * diff + T(4) * a2 * z2));
+        return fmax(r2, T(1e-24));
+    }
 }
 
 // Hamiltonian RHS.  y = (x, y, z, p_x, p_y, p_z); returns r_BL and, through
@@ -74,12 +82,17 @@ __device__ __forceinline__ T bl_r2(T x, T y, T z, T a2) {
 // with dk/dx_i . p = dr_i * A + B_i (A, B below) and dH/dx_i = C dr_i (+ D for z).
 // With GRAV = true the position part returns only the gravitational term
 // -2 H s k (the mixed-precision step keeps the free-streaming p in FP64).
-template <typename T, bool GRAV = false>
+// With FAST = true (FP64) the square root and the reciprocal are the straight-line
+// forms of rt_fast_math.h: the same values where their arguments lie between
+// 2^-900 and 2^1020, and all six outputs NaN where one does not (sv, a factor of
+// every gravitational term, takes k and with it r, 1/r and 1/(r^2 + a^2)).  A
+// caller looks for that NaN and evaluates again with FAST = false.
+template <typename T, bool GRAV = false, bool FAST = false>
 __device__ __forceinline__ T ks_rhs(const T* __restrict__ y, T M, T a, T* __restrict__ dy, T& hf, T& s) {
     const T x = y[0], yy = y[1], z = y[2], px = y[3], py = y[4], pz = y[5];
     const T a2 = a * a;
     const T z2 = z * z;
-    const T r2 = bl_r2<T>(x, yy, z, a2);
+    const T r2 = bl_r2<T, FAST>(x, yy, z, a2);
     const T inv_r = rt_rsqrt<T>(r2);
     const T r = r2 * inv_r;
     const T rpa = r2 + a2;
@@ -88,7 +101,9 @@ __device__ __forceinline__ T ks_rhs(const T* __restrict__ y, T M, T a, T* __rest
     T inv_rpa, inv_den;
     if constexpr (sizeof(T) == 8) {
         // one reciprocal for both denominators (r^6 stays far from overflow in FP64)
-        const T q = rt_rcp<T>(rpa * den);
+        T q;
+        if constexpr (FAST) q = fast_rcp(rpa * den);
+        else q = rt_rcp<T>(rpa * den);
         inv_rpa = den * q;
         inv_den = rpa * q;
     } else {

@@ -210,6 +210,77 @@ __device__ __forceinline__ void fp64_stages_rolled(const double* __restrict__ y,
     }
 }
 
+// FP64 stages 2..7, straight-line (rk45_adaptive.hpp:210-252).  A root evaluation
+// stops at y5.  DENSE: a step that crosses z = 0 also gets its dense-output term.
+template <bool FAST, bool DENSE>
+__device__ __forceinline__ void fp64_stages(const double* __restrict__ y, const double* __restrict__ k1, double hh,
+                                            double M, double a, bool root, double* __restrict__ y5,
+                                            double* __restrict__ kA, double* __restrict__ est,
+                                            double* __restrict__ dense5, double& r5, double& hf5, double& s5) {
+    double k3[6], k4[6], k5[6], k6[6];
+    double in[6], hf, sv;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A21 * k1[i]);
+    ks_rhs<double, false, FAST>(in, M, a, kA, hf, sv);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A31 * k1[i] + DP::A32 * kA[i]);
+    ks_rhs<double, false, FAST>(in, M, a, k3, hf, sv);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A41 * k1[i] + DP::A42 * kA[i] + DP::A43 * k3[i]);
+    ks_rhs<double, false, FAST>(in, M, a, k4, hf, sv);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        in[i] = y[i] + hh * (DP::A51 * k1[i] + DP::A52 * kA[i] + DP::A53 * k3[i] + DP::A54 * k4[i]);
+    ks_rhs<double, false, FAST>(in, M, a, k5, hf, sv);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        in[i] = y[i] + hh * (DP::A61 * k1[i] + DP::A62 * kA[i] + DP::A63 * k3[i] + DP::A64 * k4[i] + DP::A65 * k5[i]);
+    ks_rhs<double, false, FAST>(in, M, a, k6, hf, sv);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        y5[i] = y[i] + hh * (DP::B1 * k1[i] + DP::B3 * k3[i] + DP::B4 * k4[i] + DP::B5 * k5[i] + DP::B6 * k6[i]);
+    if (!root) {
+        r5 = ks_rhs<double, false, FAST>(y5, M, a, kA, hf5, s5);
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+            est[i] = fabs(hh) * fabs(DP::E1 * k1[i] + DP::E3 * k3[i] + DP::E4 * k4[i] + DP::E5 * k5[i] +
+                                     DP::E6 * k6[i] + DP::E7 * kA[i]);
+        if constexpr (DENSE) {
+            if (y[2] * y5[2] <= 0.0) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+                    dense5[i] = hh * (DP::D1 * k1[i] + DP::D3 * k3[i] + DP::D4 * k4[i] + DP::D5 * k5[i] +
+                                      DP::D6 * k6[i] + DP::D7 * kA[i]);
+            }
+        }
+    }
+}
+
+// The same attempt with the compiler's division and square root, for an attempt whose
+// stages leave the fast forms' range: out of line, y and k1 in io[0..11], then y5, k7,
+// est, the dense-output term, r, H and s.
+template <bool DENSE>
+__device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double hh, double M, double a, bool root) {
+    double y[6], k1[6], y5[6], kA[6], est[6], dense5[6], r5 = 0.0, hf5 = 0.0, s5 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        y[i] = io[i];
+        k1[i] = io[6 + i];
+        kA[i] = est[i] = dense5[i] = 0.0;
+    }
+    fp64_stages<false, DENSE>(y, k1, hh, M, a, root, y5, kA, est, dense5, r5, hf5, s5);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        io[12 + i] = y5[i];
+        io[18 + i] = kA[i];
+        io[24 + i] = est[i];
+        io[30 + i] = dense5[i];
+    }
+    io[36] = r5;
+    io[37] = hf5;
+    io[38] = s5;
+}
+
 }  // namespace
 
 // 384 / BLOCK resident CTAs per SM caps the kernel at 168 registers per thread
@@ -589,45 +660,26 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) trace_kernel_t(TraceArgs a
                     }
                 }
             } else {
-                double k3[6], k4[6], k5[6], k6[6];
-                double in[6], hf, sv;
+                fp64_stages<true, NEAR_PASS>(y, k1, hh, M, a, root, y5, kA, est, dense5, r5, hf5, s5);
+                const double probe = root ? y5[2] : est[2];
+                if (probe != probe) {  // a stage left the fast forms' range (or the state is NaN)
+                    double io[39];
 #pragma unroll
-                for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A21 * k1[i]);
-                ks_rhs<double>(in, M, a, kA, hf, sv);
-#pragma unroll
-                for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A31 * k1[i] + DP::A32 * kA[i]);
-                ks_rhs<double>(in, M, a, k3, hf, sv);
-#pragma unroll
-                for (int i = 0; i < 6; ++i)
-                    in[i] = y[i] + hh * (DP::A41 * k1[i] + DP::A42 * kA[i] + DP::A43 * k3[i]);
-                ks_rhs<double>(in, M, a, k4, hf, sv);
-#pragma unroll
-                for (int i = 0; i < 6; ++i)
-                    in[i] = y[i] + hh * (DP::A51 * k1[i] + DP::A52 * kA[i] + DP::A53 * k3[i] + DP::A54 * k4[i]);
-                ks_rhs<double>(in, M, a, k5, hf, sv);
-#pragma unroll
-                for (int i = 0; i < 6; ++i)
-                    in[i] = y[i] + hh * (DP::A61 * k1[i] + DP::A62 * kA[i] + DP::A63 * k3[i] + DP::A64 * k4[i] +
-                                         DP::A65 * k5[i]);
-                ks_rhs<double>(in, M, a, k6, hf, sv);
-#pragma unroll
-                for (int i = 0; i < 6; ++i)
-                    y5[i] = y[i] + hh * (DP::B1 * k1[i] + DP::B3 * k3[i] + DP::B4 * k4[i] + DP::B5 * k5[i] +
-                                         DP::B6 * k6[i]);
-                if (!root) {
-                    r5 = ks_rhs<double>(y5, M, a, kA, hf5, s5);
-#pragma unroll
-                    for (int i = 0; i < 6; ++i)
-                        est[i] = fabs(hh) * fabs(DP::E1 * k1[i] + DP::E3 * k3[i] + DP::E4 * k4[i] +
-                                                 DP::E5 * k5[i] + DP::E6 * k6[i] + DP::E7 * kA[i]);
-                    if constexpr (NEAR_PASS) {
-                        if (y[2] * y5[2] <= 0.0) {
-#pragma unroll
-                            for (int i = 0; i < 6; ++i)
-                                dense5[i] = hh * (DP::D1 * k1[i] + DP::D3 * k3[i] + DP::D4 * k4[i] +
-                                                  DP::D5 * k5[i] + DP::D6 * k6[i] + DP::D7 * kA[i]);
-                        }
+                    for (int i = 0; i < 6; ++i) {
+                        io[i] = y[i];
+                        io[6 + i] = k1[i];
                     }
+                    fp64_stages_special<NEAR_PASS>(io, hh, M, a, root);
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        y5[i] = io[12 + i];
+                        kA[i] = io[18 + i];
+                        est[i] = io[24 + i];
+                        dense5[i] = io[30 + i];
+                    }
+                    r5 = io[36];
+                    hf5 = io[37];
+                    s5 = io[38];
                 }
             }
         }

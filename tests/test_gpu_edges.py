@@ -124,3 +124,43 @@ def test_host_wait_times_out_and_recovers(tracer):
     part = tracer.dispatch(small, fields=["status", "r_hit"], pixels=False)
     np.testing.assert_array_equal(part["status"], st[2000 * side:2008 * side])
     np.testing.assert_array_equal(part["r_hit"], dev["r_hit"].cpu().numpy()[2000 * side:2008 * side])
+
+
+@pytest.mark.parametrize("precision", [relsim.PRECISION_FP64, relsim.PRECISION_MIXED])
+@pytest.mark.parametrize("mass", [1e-3, 1e5])
+def test_mass_scales(tracer, precision, mass):
+    """The record of a scaled scene is the unit scene's, scaled."""
+    tracer.set_launch_config()
+    kw = dict(width=32, height=32, incl_deg=60.0, fov_deg=25.0, precision=precision, atol=1e-13)
+    one = tracer.dispatch(relsim.make_camera(spin=0.7, r_obs=40.0, **kw))
+    out = tracer.dispatch(relsim.make_camera(spin=0.7 * mass, mass=mass, r_obs=40.0 * mass, escape_radius=1000.0 * mass,
+                                             disk_outer=20.0 * mass, **kw))
+    np.testing.assert_array_equal(out["status"], one["status"])
+    hit = one["status"] == relsim.RAY_DISK
+    assert hit.sum() > 50
+    rel = np.abs(out["r_hit"][hit] / mass / one["r_hit"][hit] - 1.0)
+    assert rel.max() < 1e-5, rel.max()
+
+
+@pytest.mark.parametrize("precision", [relsim.PRECISION_FP64, relsim.PRECISION_MIXED])
+def test_attempts_outside_the_fast_range(tracer, precision):
+    """r^6 beyond the largest double: the stages' straight-line reciprocal has no value there and
+    the attempt is taken again with the compiler's division, which gives 0 (no field).  A ray then
+    runs straight along its initial momentum; after the first step (0.01 r_obs) the longest one,
+    1e13, is nothing at that radius, and every ray uses up its attempts one first step from the
+    observer, instead of ending on a state that is not finite."""
+    tracer.set_launch_config()
+    m = 1e52
+    cam = relsim.make_camera(spin=0.5 * m, mass=m, r_obs=100.0 * m, incl_deg=20.0, fov_deg=10.0,
+                             escape_radius=1000.0 * m, disk_outer=20.0 * m, width=24, height=24, max_steps=30,
+                             early_capture=False, precision=precision)
+    out = tracer.dispatch(cam)
+    assert np.all(out["status"] == relsim.RAY_UNFINISHED)
+    assert np.all(out["steps_accepted"] + out["steps_rejected"] == 30)
+    d = relsim.camera_dict(cam)
+    for i in range(24 * 24):
+        y, _ = O.initial_state(d, i % 24, i // 24)
+        x = (y[:3] - 0.01 * 100.0 * m * y[3:6]) / m
+        w = x @ x - 0.25
+        r = np.sqrt(0.5 * (w + np.sqrt(w * w + x[2] ** 2)))
+        assert abs(out["r"][i] / m / r - 1.0) < 1e-9, (i, out["r"][i] / m, r)
