@@ -242,9 +242,8 @@ rt_status launch(rt_handle* h, uint32_t n_bundles, uint64_t total, const OutPtrs
     args.cont = h->cur_cont;
     RT_CUDA(h, cudaMemsetAsync(h->queue.ptr, 0, sizeof(unsigned long long), s));
     RT_CUDA(h, cudaMemsetAsync(h->stats.ptr, 0, sizeof(unsigned long long) * ST_COUNT, s));
-    const uint32_t grid = static_cast<uint32_t>(h->sm_count) * c.ctas_per_sm;
     if (!capturing) RT_CUDA(h, cudaEventRecord(h->ev0, s));
-    launch_trace(args, grid, c.block_size, mixed, c.fp64_rolled != 0, s);
+    launch_trace(args, h->sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, s);
     RT_CUDA(h, cudaGetLastError());
     if (!capturing) {
         RT_CUDA(h, cudaEventRecord(h->ev1, s));
@@ -667,8 +666,7 @@ rt_status launch_banded_single(rt_handle* h, const rt_camera* cam, uint32_t col0
             args.stats = static_cast<unsigned long long*>(h->stats.ptr);
             args.out = out;
             args.cont = h->cur_cont;
-            launch_trace(args, static_cast<uint32_t>(h->sm_count) * c.ctas_per_sm, c.block_size, mixed,
-                         c.fp64_rolled != 0, sb);
+            launch_trace(args, h->sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, sb);
         }
         RT_CUDA(h, cudaGetLastError());
         if (prev_stream) RT_CUDA(h, static_cast<cudaError_t>(band_copy_hook(&ctx, prev_begin, prev_count, prev_stream)));
@@ -1323,6 +1321,7 @@ rt_status noalloc_setup(int dev, NoAllocDevice& out, char* err, size_t len) {
         for (uint32_t block : {64u, 128u, 256u})
             for (bool mixed : {false, true})
                 for (bool rolled : {false, true}) trace_occupancy(kernel_block(block, mixed, rolled), mixed, rolled);
+        trace_wide_occupancy();
         if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_cuda_fail(err, len, e, "kernel set-up");
         d.scratch = static_cast<unsigned char*>(p);
         d.sm_count = sms;
@@ -1417,8 +1416,7 @@ extern "C" rt_status rt_trace_bundles_noalloc(int device_ordinal, const rt_camer
     args.queue = reinterpret_cast<unsigned long long*>(dev.scratch);
     args.stats = reinterpret_cast<unsigned long long*>(dev.scratch + kNoAllocStatsOffset);
     args.out = OutPtrs{pixels, rays ? *rays : rt_ray_out{}};
-    const uint32_t grid = static_cast<uint32_t>(dev.sm_count) * c.ctas_per_sm;
-    launch_trace(args, grid, c.block_size, mixed, c.fp64_rolled != 0, s);
+    launch_trace(args, dev.sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_cuda_fail(error, error_len, e, "tracer launch");
     return RT_OK;
 }

@@ -435,8 +435,7 @@ bool launch_epoch(rt_server* s, Slot& slot) {
         e = static_cast<cudaError_t>(
             enqueue_two_pass(args, buf, s->sm_count, c.block_size, st, nullptr, nullptr, nullptr, 1));
     } else {
-        launch_trace(args, static_cast<uint32_t>(s->sm_count) * c.ctas_per_sm, c.block_size, mixed,
-                     c.fp64_rolled != 0, st);
+        launch_trace(args, s->sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaEventRecord(slot.done, st);

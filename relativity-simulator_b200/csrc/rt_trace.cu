@@ -283,8 +283,8 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 
 }  // namespace
 
-// 384 / BLOCK resident CTAs per SM caps the kernel at 168 registers per thread
-// (12 warps per SM).
+// Resident warps per SM set the registers per thread: 12 warps at 168 registers, or
+// with WIDE 16 at 128.
 //
 // PASS selects the single-kernel tracer or one pass of the two-pass mixed
 // tracer.  The far pass (FP32 stages only) parks a ray when it enters the FP64
@@ -292,10 +292,15 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 // again.  Both passes solve disk crossings on the step's dense output.  Parked
 // rays resume from their saved state, so a ray's arithmetic does not depend on
 // which rays share its warp.
-// Every form runs 12 warps per SM (168 registers); the pass kernels spill a
-// little there, which measured faster than 8 warps without spills.
-template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0>
-__global__ void __launch_bounds__(BLOCK, 384 / BLOCK) trace_kernel_t(TraceArgs args) {
+// Twelve warps: the pass kernels spill a little there, which measured faster than 8
+// warps without spills.  Sixteen serve the plain FP64 tracer over many rays: FP64
+// latency is what bounds it, and a third more warps hide more of it than the
+// spills cost (2048^2 34.0 / 31.9 ms; the FP64 pipe is busy 65 % of the time).
+// The far, near and critical passes lose by it (1279x717: 4.53 / 4.71, 0.89 / 1.19
+// and 1.73 / 2.01 ms): their warps run few rays or few lanes, and there a longer
+// attempt is a longer tail.
+template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, bool WIDE = false>
+__global__ void __launch_bounds__(BLOCK, (WIDE ? 512 : 384) / BLOCK) trace_kernel_t(TraceArgs args) {
     __shared__ Cold<BLOCK> S;
     __shared__ KStore<ROLLED ? BLOCK : 1> K;
     const unsigned FULL = 0xffffffffu;
@@ -960,6 +965,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) trace_kernel_t(TraceArgs a
 template __global__ void trace_kernel_t<64, false, false>(TraceArgs);
 template __global__ void trace_kernel_t<128, false, false>(TraceArgs);
 template __global__ void trace_kernel_t<256, false, false>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, true>(TraceArgs);
 template __global__ void trace_kernel_t<64, false, true>(TraceArgs);
 template __global__ void trace_kernel_t<128, false, true>(TraceArgs);
 template __global__ void trace_kernel_t<64, true, true>(TraceArgs);
@@ -1006,7 +1012,26 @@ const void* kernel_for(uint32_t block, bool mixed, bool rolled, int cont = 0) {
     if (cont == 2) return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 2>);
     return (cont == 1) ? kernel_for_t<1>(block, mixed, rolled) : kernel_for_t<0>(block, mixed, rolled);
 }
+
+// The plain FP64 tracer with 16 warps per SM.
+const void* wide_kernel() { return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, true>); }
+
+// Rays per SM from which the plain FP64 tracer takes it.  More warps raise the rate
+// and lengthen one attempt, so the longest rays' tail has to be a small part of the
+// launch.  12 / 16 warps, three cameras (face-on, grazing, wide view): 1448^2
+// 17.2 / 16.2, 22.3 / 23.3, 12.9 / 12.4 ms; 1740^2 24.7 / 23.2, 32.8 / 34.3,
+// 18.4 / 17.5; 2048^2 34.0 / 31.9, 43.4 / 42.0, 25.3 / 24.0.  The line is at 3.6 M rays.
+constexpr uint64_t kWideRaysPerSm = 24576;
 }  // namespace
+
+int trace_wide_occupancy() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wide_kernel(), 128, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
 
 uint32_t kernel_block(uint32_t block, bool mixed, bool rolled) {
     if ((mixed || rolled) && block > 128) return 128;
@@ -1114,7 +1139,7 @@ uint64_t two_pass_state_bytes(uint64_t n) {
 namespace {
 cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t begin, uint64_t count, char* qb,
                          uint32_t far_grid, uint32_t far_block, uint32_t near_grid, uint32_t finish_grid,
-                         uint32_t crit_grid, bool crit_beside, cudaStream_t s) {
+                         int sm_count, uint32_t crit_ctas, bool crit_beside, cudaStream_t s) {
     uint32_t* near_q = buf.queues + 4 * begin;
     uint32_t* far_q = near_q + count;
     uint32_t* crit_q = far_q + 2 * count;
@@ -1158,7 +1183,7 @@ cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t beg
                 if ((e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_fork), s)) != cudaSuccess) break;
                 if ((e = cudaStreamWaitEvent(cs, static_cast<cudaEvent_t>(buf.crit_fork), 0)) != cudaSuccess) break;
             }
-            launch_trace(c, crit_grid, kCriticalBlock, false, false, cs);
+            launch_trace(c, sm_count, crit_ctas, kCriticalBlock, false, false, cs);
             if ((e = cudaGetLastError()) != cudaSuccess) break;
             if (crit_beside && (e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_join), cs)) != cudaSuccess) break;
         }
@@ -1202,7 +1227,7 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
     const uint32_t near_grid = static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(near_occ > 1 ? near_occ : 1);
     const uint32_t finish_grid = static_cast<uint32_t>(sm_count) * 8u;
     const int crit_occ = trace_occupancy(kCriticalBlock, false, false);
-    const uint32_t crit_grid = static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(crit_occ > 1 ? crit_occ : 1);
+    const uint32_t crit_ctas = static_cast<uint32_t>(crit_occ > 1 ? crit_occ : 1);
     cudaError_t e = cudaSuccess;
     if (bands > 1) {
         if ((e = cudaEventRecord(static_cast<cudaEvent_t>(fork), s)) != cudaSuccess) return static_cast<int>(e);
@@ -1218,7 +1243,7 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
         cudaStream_t sb = (b & 1u) ? s2 : s;
         const bool crit_beside = bands == 1 && buf.crit_stream && buf.crit_fork && buf.crit_join;
         e = enqueue_band(base, buf, begin, count, buf.counters + kBandCounterBytes * b, far_grid, far_block, near_grid,
-                         finish_grid, crit_grid, crit_beside, sb);
+                         finish_grid, sm_count, crit_ctas, crit_beside, sb);
         if (e == cudaSuccess && after_band && prev_stream)
             e = static_cast<cudaError_t>(after_band(hook_ctx, prev_begin, prev_count, prev_stream));
         prev_begin = begin;
@@ -1236,12 +1261,20 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
     return static_cast<int>(e);
 }
 
-void launch_trace(const TraceArgs& args, uint32_t grid, uint32_t block, bool mixed, bool rolled, void* stream) {
+void launch_trace(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, uint32_t block, bool mixed, bool rolled,
+                  void* stream) {
     void* params[] = {const_cast<TraceArgs*>(&args)};
     // hydro model 2: the FP64 straight-line tracer in 128-thread blocks
     const int cont = args.cont.vol ? 2 : (args.cont.cross ? 1 : 0);
     block = (cont == 2) ? 128u : kernel_block(block, mixed, rolled);
-    cudaLaunchKernel(kernel_for(block, mixed, rolled, cont), dim3(grid), dim3(block), params, 0,
+    const void* kernel = kernel_for(block, mixed, rolled, cont);
+    // only where the caller left the CTAs per SM at the occupancy maximum
+    if (!mixed && !rolled && cont == 0 && !args.in_queue && block == 128u && ctas_per_sm >= 3u &&
+        args.total_rays >= kWideRaysPerSm * static_cast<uint64_t>(sm_count)) {
+        kernel = wide_kernel();
+        ctas_per_sm = 4;
+    }
+    cudaLaunchKernel(kernel, dim3(static_cast<uint32_t>(sm_count) * ctas_per_sm), dim3(block), params, 0,
                      static_cast<cudaStream_t>(stream));
 }
 
