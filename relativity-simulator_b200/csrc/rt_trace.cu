@@ -38,112 +38,13 @@
 #include <cstdint>
 
 #include "rt_device.cuh"
+#include "rt_far_step.cuh"
 #include "rt_internal.h"
 #include "rt_ray.cuh"
 
 namespace relsim {
 
 namespace {
-
-// Mixed-precision DP45 step for the far zone.  The state y and the result y5
-// are FP64; the stages run in FP32 on the deviation from free streaming:
-//   x_j = x + h c_j p + h sum_m a_jm dx_m,   dx_m = (p_m - p) - 2 H s k (at stage m)
-//   p_j = p + h sum_m a_jm kp_m,             kp_m = dp/dlambda (at stage m)
-// so the large h p term of every position increment stays FP64 and FP32 only
-// carries the gravitational part.  y5 = y + h p (FP64) + h sum b_j dx_j (FP32).
-// The error estimate uses sum_j e_j = 0: E_x = h sum e_j dx_j.  Outputs k7 in
-// FP64 (FSAL), |E| per component, and the FP32 BL radius, H and s of the FSAL
-// stage at y5 (the step's bookkeeping: step cap, termination, projection).
-// When the step crosses z = 0 it also writes the dense-output term
-// e = h sum_j D_j k_j; sum_j D_j = 0 makes its position part h sum_j D_j dx_j,
-// so it too comes from the FP32 deviations.
-__device__ __forceinline__ void mixed_stages(const double* __restrict__ y, const double* __restrict__ k1, double hh,
-                                             double M, double a, double* __restrict__ y5, double* __restrict__ k7,
-                                             double* __restrict__ est, float& r7, float& hf7, float& s7,
-                                             double* __restrict__ dense_e) {
-    const float h = static_cast<float>(hh);
-    const float Mf = static_cast<float>(M), af = static_cast<float>(a);
-    float x0[3], p0[3];
-    float dx1[3], kp1[3], dx2[3], kp2[3], dx3[3], kp3[3], dx4[3], kp4[3], dx5[3], kp5[3], dx6[3], kp6[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        x0[i] = static_cast<float>(y[i]);
-        p0[i] = static_cast<float>(y[3 + i]);
-        dx1[i] = static_cast<float>(k1[i] - y[3 + i]);
-        kp1[i] = static_cast<float>(k1[3 + i]);
-    }
-    constexpr float C2 = 1.0f / 5.0f, C3 = 3.0f / 10.0f, C4 = 4.0f / 5.0f, C5 = 8.0f / 9.0f;
-    float in[6], g[6], hf, sv;
-#define RT_STAGE(DXO, KPO, CC, SUMX, SUMP)                          \
-    _Pragma("unroll") for (int i = 0; i < 3; ++i) {                 \
-        const float dp = h * (SUMP);                                \
-        in[i] = x0[i] + h * ((CC) * p0[i] + (SUMX));                \
-        in[3 + i] = p0[i] + dp;                                     \
-        g[i] = dp;                                                  \
-    }                                                               \
-    {                                                               \
-        float dpv[3] = {g[0], g[1], g[2]};                          \
-        ks_rhs<float, true>(in, Mf, af, g, hf, sv);                 \
-        _Pragma("unroll") for (int i = 0; i < 3; ++i) {             \
-            DXO[i] = dpv[i] + g[i];                                 \
-            KPO[i] = g[3 + i];                                      \
-        }                                                           \
-    }
-    RT_STAGE(dx2, kp2, C2, float(DP::A21) * dx1[i], float(DP::A21) * kp1[i])
-    RT_STAGE(dx3, kp3, C3, float(DP::A31) * dx1[i] + float(DP::A32) * dx2[i],
-             float(DP::A31) * kp1[i] + float(DP::A32) * kp2[i])
-    RT_STAGE(dx4, kp4, C4, float(DP::A41) * dx1[i] + float(DP::A42) * dx2[i] + float(DP::A43) * dx3[i],
-             float(DP::A41) * kp1[i] + float(DP::A42) * kp2[i] + float(DP::A43) * kp3[i])
-    RT_STAGE(dx5, kp5, C5,
-             float(DP::A51) * dx1[i] + float(DP::A52) * dx2[i] + float(DP::A53) * dx3[i] + float(DP::A54) * dx4[i],
-             float(DP::A51) * kp1[i] + float(DP::A52) * kp2[i] + float(DP::A53) * kp3[i] + float(DP::A54) * kp4[i])
-    RT_STAGE(dx6, kp6, 1.0f,
-             float(DP::A61) * dx1[i] + float(DP::A62) * dx2[i] + float(DP::A63) * dx3[i] + float(DP::A64) * dx4[i] +
-                 float(DP::A65) * dx5[i],
-             float(DP::A61) * kp1[i] + float(DP::A62) * kp2[i] + float(DP::A63) * kp3[i] + float(DP::A64) * kp4[i] +
-                 float(DP::A65) * kp5[i])
-#undef RT_STAGE
-    // 5th-order solution: FP64 accumulation of the FP32 increments
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float sx = float(DP::B1) * dx1[i] + float(DP::B3) * dx3[i] + float(DP::B4) * dx4[i] +
-                         float(DP::B5) * dx5[i] + float(DP::B6) * dx6[i];
-        const float sp = float(DP::B1) * kp1[i] + float(DP::B3) * kp3[i] + float(DP::B4) * kp4[i] +
-                         float(DP::B5) * kp5[i] + float(DP::B6) * kp6[i];
-        y5[i] = y[i] + hh * y[3 + i] + static_cast<double>(h * sx);
-        y5[3 + i] = y[3 + i] + static_cast<double>(h * sp);
-    }
-    // stage 7 (FSAL) at y5
-#pragma unroll
-    for (int i = 0; i < 6; ++i) in[i] = static_cast<float>(y5[i]);
-    r7 = ks_rhs<float, true>(in, Mf, af, g, hf, sv);
-    hf7 = hf;
-    s7 = sv;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float dx7 = static_cast<float>(y5[3 + i] - y[3 + i]) + g[i];
-        const float ex = float(DP::E1) * dx1[i] + float(DP::E3) * dx3[i] + float(DP::E4) * dx4[i] +
-                         float(DP::E5) * dx5[i] + float(DP::E6) * dx6[i] + float(DP::E7) * dx7;
-        const float ep = float(DP::E1) * kp1[i] + float(DP::E3) * kp3[i] + float(DP::E4) * kp4[i] +
-                         float(DP::E5) * kp5[i] + float(DP::E6) * kp6[i] + float(DP::E7) * g[3 + i];
-        est[i] = static_cast<double>(fabsf(h * ex));
-        est[3 + i] = static_cast<double>(fabsf(h * ep));
-        k7[i] = y5[3 + i] + static_cast<double>(g[i]);
-        k7[3 + i] = static_cast<double>(g[3 + i]);
-    }
-    if (y[2] * y5[2] <= 0.0) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const float dx7 = static_cast<float>(y5[3 + i] - y[3 + i]) + g[i];
-            const float sx = float(DP::D1) * dx1[i] + float(DP::D3) * dx3[i] + float(DP::D4) * dx4[i] +
-                             float(DP::D5) * dx5[i] + float(DP::D6) * dx6[i] + float(DP::D7) * dx7;
-            const float sp = float(DP::D1) * kp1[i] + float(DP::D3) * kp3[i] + float(DP::D4) * kp4[i] +
-                             float(DP::D5) * kp5[i] + float(DP::D6) * kp6[i] + float(DP::D7) * g[3 + i];
-            dense_e[i] = static_cast<double>(h * sx);
-            dense_e[3 + i] = static_cast<double>(h * sp);
-        }
-    }
-}
 
 // Dormand-Prince tableau rows for the rolled FP64 step: row s gives the
 // coefficients of k1..k(s+1) in the input of stage s + 2 (row 5 = b, the
