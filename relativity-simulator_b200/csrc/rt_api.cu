@@ -20,6 +20,7 @@
 
 #include "relsim_cuda.h"
 #include "rt_internal.h"
+#include "rt_planck.h"
 
 namespace relsim {
 double measure_fma_peak(bool fp64, int sm_count, cudaStream_t stream, float* ms_out);
@@ -53,6 +54,7 @@ struct rt_handle {
     DevBuf bl_desc;                      // Boyer-Lindquist camera
     DevBuf band_desc, band_queue;        // banded single-kernel host dispatches: per-band camera and counter
     DevBuf shade_desc;                   // pixel shading constants of the last shaded camera
+    DevBuf planck;                       // the blackbody colour's table, uploaded at the first shaded dispatch
     bool shade_on = false;               // rt_set_shading
     // translucent-disk continuation of a shaded dispatch: each ray's disk crossings
     // and how it ended, and what the launches pass the tracer
@@ -314,11 +316,29 @@ rt_status add_shade_fields(rt_handle* h, rt_ray_out& dev, size_t n) {
     return RT_OK;
 }
 
+// The blackbody colour's table on the device: 57 KB, the same for every camera,
+// uploaded once and waited for, since later dispatches may use other streams.
+rt_status ensure_planck(rt_handle* h, cudaStream_t s) {
+    if (h->planck.ptr) return RT_OK;
+    const rt_status st = ensure(h, h->planck, sizeof(double) * kPlanckTableDoubles);
+    if (st != RT_OK) return st;
+    cudaError_t e = cudaMemcpyAsync(h->planck.ptr, planck_table_host(), sizeof(double) * kPlanckTableDoubles,
+                                    cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        release(h->planck);
+        return cuda_fail(h, e, "spectral table upload");
+    }
+    return RT_OK;
+}
+
 // Upload the shading constants of a camera (before the trace, on its stream).
 rt_status shade_prepare(rt_handle* h, const rt_camera* cam, cudaStream_t s) {
     ShadeDesc d;
     if (!build_shade_desc(*cam, h->shading, d)) return fail(h, RT_ERR_INVALID_ARG, "unsupported shading settings");
     rt_status st;
+    if ((st = ensure_planck(h, s)) != RT_OK) return st;
+    d.planck = static_cast<const double*>(h->planck.ptr);
     if ((st = ensure(h, h->shade_desc, sizeof(ShadeDesc))) != RT_OK) return st;
     // pageable descriptor: the copy is staged before the call returns
     RT_CUDA(h, cudaMemcpyAsync(h->shade_desc.ptr, &d, sizeof d, cudaMemcpyHostToDevice, s));
@@ -699,11 +719,13 @@ rt_status ms_shade_prepare(rt_handle* h, const rt_camera* cam, const rt_source* 
     ShadeDesc d[kMaxSources];
     ShadeDesc base;
     if (!build_shade_desc(*cam, h->shading, base)) return fail(h, RT_ERR_INVALID_ARG, "unsupported shading settings");
+    rt_status st;
+    if ((st = ensure_planck(h, s)) != RT_OK) return st;
+    base.planck = static_cast<const double*>(h->planck.ptr);
     build_source_shade_desc(base, nullptr, table[0].m, table[0].a, table[0].disk_in, table[0].disk_out, d[0]);
     for (uint32_t i = 1; i < count; ++i)
         build_source_shade_desc(base, reinterpret_cast<const float*>(&sources[i - 1].disk), table[i].m, table[i].a,
                                 table[i].disk_in, table[i].disk_out, d[i]);
-    rt_status st;
     if ((st = ensure(h, h->ms_shade, sizeof(ShadeDesc) * kMaxSources)) != RT_OK) return st;
     // pageable descriptors: the copy is staged before the call returns
     RT_CUDA(h, cudaMemcpyAsync(h->ms_shade.ptr, d, sizeof(ShadeDesc) * count, cudaMemcpyHostToDevice, s));
@@ -848,6 +870,7 @@ void rt_destroy(rt_handle* h) {
     release(h->band_desc);
     release(h->band_queue);
     release(h->shade_desc);
+    release(h->planck);
     release(h->ms_shade);
     release(h->cont_cross);
     release(h->cont_info);

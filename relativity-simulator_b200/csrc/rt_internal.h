@@ -241,7 +241,7 @@ struct alignas(16) ShadeDesc {
     double pattern_omega;                 // orbital angular velocity at sqrt(inner outer)
     double nt_flux_peak, nt_rate_factor;  // Novikov-Thorne: peak flux over the disk, rate^(1/4)
     double nt_m, nt_a_star, nt_x0, nt_x1, nt_x2, nt_x3, nt_r_isco;
-    uint32_t hydro_model, tonemap, sky_on, pad1;
+    uint32_t hydro_model, tonemap, sky_on, fm_valid;
     double lambda_um[33];
     double weight[33][3];
     double fov;      // the camera's field of view (the sky's level of detail)
@@ -251,12 +251,14 @@ struct alignas(16) ShadeDesc {
     // exponent 1 / (gamma - 1), kappa (optical depth per M at peak enthalpy) and
     // samples per M of chord
     double fm_m, fm_a, fm_rh, fm_l, fm_w_in, fm_h_max, fm_inner, fm_outer, fm_exponent, fm_kappa, fm_density;
-    uint32_t fm_valid, pad2;
+    const double* planck;  // device: the blackbody colour's table (rt_planck.h); null: not at hand
 };
 
 // Build the shading constants of a camera; false if the settings are not
 // supported (hydro model above 2, sky_enabled above 1).
 bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d);
+// The blackbody colour's table (rt_planck.h), built at the first call.
+const double* planck_table_host();
 void build_source_shade_desc(const ShadeDesc& base, const float* profile, double mass, double spin, double inner,
                              double outer, ShadeDesc& d);
 // Shade n rays: pixels[i].rgba from the record's status, r_hit, phi and g.

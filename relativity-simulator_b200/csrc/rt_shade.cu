@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <vector>
 
 #include "rt_device.cuh"
 #include "rt_internal.h"
@@ -224,20 +225,35 @@ double temperature_shape_peak(double exponent, double zero_torque) {
 
 }  // namespace
 
-bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d) {
-    if (s.hydro_model > 2u || s.sky_enabled > 1u || s.tonemapping_mode > 3u) return false;
-    d = ShadeDesc{};
-    // spectral table (accretion_disk_model.hpp:52-69)
+// The spectral table of the blackbody colour (accretion_disk_model.hpp:52-69).
+static void spectral_table(double* lambda_um, double (*weight)[3]) {
     const double step = (780.0 - 380.0) / 32.0;
     for (int i = 0; i <= 32; ++i) {
         const double lnm = 380.0 + static_cast<double>(i) * step;
         const double trap = (i == 0 || i == 32) ? 0.5 : 1.0;
-        d.lambda_um[i] = lnm * 1e-3;
-        d.weight[i][0] = trap * (lobe(lnm, 1.056, 599.8, 37.9, 31.0) + lobe(lnm, 0.362, 442.0, 16.0, 26.7) -
-                                 lobe(lnm, 0.065, 501.1, 20.4, 26.2));
-        d.weight[i][1] = trap * (lobe(lnm, 0.821, 568.8, 46.9, 40.5) + lobe(lnm, 0.286, 530.9, 16.3, 31.1));
-        d.weight[i][2] = trap * (lobe(lnm, 1.217, 437.0, 11.8, 36.0) + lobe(lnm, 0.681, 459.0, 26.0, 13.8));
+        lambda_um[i] = lnm * 1e-3;
+        weight[i][0] = trap * (lobe(lnm, 1.056, 599.8, 37.9, 31.0) + lobe(lnm, 0.362, 442.0, 16.0, 26.7) -
+                               lobe(lnm, 0.065, 501.1, 20.4, 26.2));
+        weight[i][1] = trap * (lobe(lnm, 0.821, 568.8, 46.9, 40.5) + lobe(lnm, 0.286, 530.9, 16.3, 31.1));
+        weight[i][2] = trap * (lobe(lnm, 1.217, 437.0, 11.8, 36.0) + lobe(lnm, 0.681, 459.0, 26.0, 13.8));
     }
+}
+
+const double* planck_table_host() {
+    static const std::vector<double> table = [] {
+        double lambda_um[33], weight[33][3];
+        spectral_table(lambda_um, weight);
+        std::vector<double> t(kPlanckTableDoubles);
+        planck_table_fill(lambda_um, weight, t.data());
+        return t;
+    }();
+    return table.data();
+}
+
+bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d) {
+    if (s.hydro_model > 2u || s.sky_enabled > 1u || s.tonemapping_mode > 3u) return false;
+    d = ShadeDesc{};
+    spectral_table(d.lambda_um, d.weight);
     // resolve_primary_profile + finalize (accretion_disk_model.hpp:180-196)
     static_assert(sizeof(rt_disk_profile) == 32 * sizeof(float), "GpuDiskProfile layout");
     std::copy_n(reinterpret_cast<const float*>(&s.disk), 32, d.profile);
@@ -251,7 +267,7 @@ bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d) {
     const double peak = temperature_shape_peak(static_cast<double>(P[DP_T_EXPONENT]), static_cast<double>(P[DP_ZERO_TORQUE]));
     P[DP_T_NORMALIZATION] = static_cast<float>(1.0 / mxd(peak, 1e-6));
     double xyz[3];
-    planck_xyz(d.lambda_um, d.weight, static_cast<double>(P[DP_PEAK_T]), xyz);
+    planck_sum(d.lambda_um, d.weight, static_cast<double>(P[DP_PEAK_T]), xyz);
     P[DP_REF_LUMINANCE] = static_cast<float>(mxd(xyz[1], 1e-30));
 
     // disk geometry and the camera's detail factor (software_compute_engine.hpp:3800-3836)

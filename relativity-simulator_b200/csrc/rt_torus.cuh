@@ -57,35 +57,47 @@ RT_FM_HD double potential(double m, double a, double rh, double l, double r, dou
 }
 RT_FM_HD double potential(const Torus& t, double r, double theta) { return potential(t.m, t.a, t.rh, t.l, r, theta); }
 
-// Specific enthalpy h = exp(W_in - W), at least 1 (:152-159).
-RT_FM_HD double enthalpy(const Torus& t, double r, double theta) {
-    const double w = potential(t, r, theta);
-    if (w >= t.w_in) return 1.0;
-    return fmx(1.0, exp(t.w_in - w));
+// The fluid at radius r with c2 = cos^2 theta and s2 = sin^2 theta (s2 >= 1e-30 is
+// imposed): false outside the torus (no such orbit, or an enthalpy h = exp(W_in - W)
+// of 1 + 1e-9 or less, :152-159), else h and the four-velocity's u^t and u^phi
+// (:210-224: u_t = -e^W, u_phi = -l u_t, raised with the Boyer-Lindquist Kerr inverse
+// metric, metrics/kerr.hpp:151-177).  W = log(X) / 2, so e^W = sqrt(X) and no
+// logarithm or exponential is taken; e_in = exp(W_in).
+RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_in, double& h, double& ut, double& uphi) {
+    if (r <= t.rh * 1.0001) return false;
+    const double s2 = fmx(s2_in, 1e-30);
+    const double r2 = r * r, a2 = t.a * t.a, mra = 2.0 * t.m * r * t.a;
+    const double rho2 = r2 + a2 * c2;
+    const double delta = r2 - 2.0 * t.m * r + a2;
+    const double sigma = (r2 + a2) * (r2 + a2) - a2 * delta * s2;
+    const double ds = delta - a2 * s2;
+    const double denom = sigma * s2 - 2.0 * mra * t.l * s2 - t.l * t.l * ds;
+    if (denom <= 0.0 || delta <= 0.0) return false;
+    const double rd = rho2 * delta;
+    const double ew = sqrt(fmx((rd * s2) / denom, 1e-30));
+    h = e_in / ew;
+    if (!(h > 1.0 + 1e-9)) return false;
+    const double q = ew / rd;
+    ut = q * (sigma - mra * t.l);
+    uphi = q * (mra + t.l * ds / s2);
+    return true;
 }
 
-// The fluid's u^t and u^phi (:210-224): u_t = -e^W, u_phi = -l u_t, raised
-// with the Boyer-Lindquist Kerr inverse metric (metrics/kerr.hpp:151-177).
+// Specific enthalpy at (r, theta), 1 outside the torus.
+RT_FM_HD double enthalpy(const Torus& t, double r, double theta) {
+    const double st = sin(theta), ct = cos(theta);
+    double h, ut, uphi;
+    return fluid(t, exp(t.w_in), r, ct * ct, st * st, h, ut, uphi) ? h : 1.0;
+}
+
+// The fluid's u^t and u^phi at (r, theta); at rest (1, 0) outside the torus.
 RT_FM_HD void four_velocity(const Torus& t, double r, double theta, double& ut, double& uphi) {
-    const double w = potential(t, r, theta);
-    if (w >= 1e20) {
+    const double st = sin(theta), ct = cos(theta);
+    double h;
+    if (!fluid(t, exp(t.w_in), r, ct * ct, st * st, h, ut, uphi)) {
         ut = 1.0;
         uphi = 0.0;
-        return;
     }
-    const double lt = -exp(w), lphi = -t.l * lt;
-    const double rr = fmx(r, 1e-12);
-    const double st = sin(theta), ct = cos(theta);
-    const double s2 = fmx(st * st, 1e-30), c2 = ct * ct;
-    const double a2 = t.a * t.a, r2 = rr * rr;
-    const double rho2 = r2 + a2 * c2;
-    const double delta = r2 - 2.0 * t.m * rr + a2;
-    const double sigma = (r2 + a2) * (r2 + a2) - a2 * delta * s2;
-    const double gtt = -sigma / (rho2 * delta);
-    const double gtp = -(2.0 * t.m * rr * t.a) / (rho2 * delta);
-    const double gpp = (delta - a2 * s2) / (rho2 * delta * s2);
-    ut = gtt * lt + gtp * lphi;
-    uphi = gtp * lt + gpp * lphi;
 }
 
 // The torus of a hole (mass, spin clamped as the shading context does) with its
