@@ -39,7 +39,12 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr double kHalfPi = 0.5 * kPi;
 constexpr double kEarlyCaptureMargin = 1e-4;  // M, distance to the critical curve
 constexpr int NB = 7;
-enum BlMode : int { BL_IDLE = 0, BL_STEP = 1 };
+// BL_ENDED: the ray has ended; its end is worked out and written when the warp refills.
+enum BlMode : int { BL_IDLE = 0, BL_STEP = 1, BL_ENDED = 2 };
+// What is left to do for an ended ray: nothing (the record at y), place the end on the
+// threshold radius inside the last step, find the disk crossing of the last step, or
+// the record at the crossing found.
+enum BlEnd : uint32_t { BE_POINT = 0, BE_TARGET = 16, BE_CROSSING = 32, BE_DISK = 48 };
 
 // Dormand-Prince rows (rk45_adaptive.hpp:196-203), error and dense-output weights.
 __constant__ double kBlA[6][6] = {
@@ -72,7 +77,9 @@ struct KnGeom {
     double irho2, idelta, idet, grr_inv, sin2, cos1;
 };
 
-template <bool DERIV>
+// FAST: that reciprocal in its straight-line form (rt_fast_math.h), for cameras whose
+// stages stay within its range (BF_FAST_RANGE).
+template <bool DERIV, bool FAST = false>
 __device__ __forceinline__ void kn_geometry(double m, double a, double q2, double r, double th, KnGeom& G) {
     double s, c;
     sincos(th, &s, &c);
@@ -81,7 +88,9 @@ __device__ __forceinline__ void kn_geometry(double m, double a, double q2, doubl
     const double rho2 = r2 + a2 * (c * c);
     const double delta = r2 - 2.0 * m * r + a2 + q2;
     const double s2c = fmax(s2, 1e-30);
-    const double qinv = 1.0 / (rho2 * delta * s2c);
+    double qinv;
+    if constexpr (FAST) qinv = fast_rcp(rho2 * delta * s2c);
+    else qinv = 1.0 / (rho2 * delta * s2c);
     const double irho2 = delta * s2c * qinv;
     const double idelta = rho2 * s2c * qinv;
     const double F = (2.0 * m * r - q2) * irho2;
@@ -117,10 +126,11 @@ __device__ __forceinline__ void kn_geometry(double m, double a, double q2, doubl
 // du/dl = -Gamma u u from d(g_mu nu u^nu)/dl = (1/2) d_mu g_ab u^a u^b:
 //   r, theta: g_rr a^r = (1/2) d_r g(u,u) - (d_r g_rr u^r + d_th g_rr u^th) u^r (same for theta);
 //   t, phi:   the t-phi block times (a^t, a^phi) = -(dg/dl) (u^t, u^phi).
+template <bool FAST = false>
 __device__ __forceinline__ void bl_rhs(double m, double a, double q2, const double* __restrict__ y,
                                        double* __restrict__ dy) {
     KnGeom G;
-    kn_geometry<true>(m, a, q2, y[0], y[1], G);
+    kn_geometry<true, FAST>(m, a, q2, y[0], y[1], G);
     const double ut = y[3], ur = y[4], uth = y[5], up = y[6];
     const double half_r = 0.5 * (G.dr[0] * ut * ut + 2.0 * G.dr[1] * ut * up + G.dr[2] * ur * ur +
                                  G.dr[3] * uth * uth + G.dr[4] * up * up);
@@ -141,8 +151,9 @@ __device__ __forceinline__ void bl_rhs(double m, double a, double q2, const doub
 }
 
 // Stages 2..7 around one RHS copy; S.k holds k2..k7 on return (k7 = S.k[5]).
-// Returns the max-norm error (rk45_adaptive.hpp:254-261, with |h|).
-template <int BLOCK>
+// Returns the max-norm error (rk45_adaptive.hpp:254-261, with |h|).  FAST: the
+// right-hand sides' straight-line reciprocal.
+template <int BLOCK, bool FAST>
 __device__ __forceinline__ double bl_stages(const BlDesc& B, const double* __restrict__ y,
                                             const double* __restrict__ k1, double hh, BlCold<BLOCK>& S, int tid,
                                             double* __restrict__ y5) {
@@ -164,7 +175,7 @@ __device__ __forceinline__ double bl_stages(const BlDesc& B, const double* __res
             for (int i = 0; i < NB; ++i) y5[i] = in[i];
         }
         double out[NB];
-        bl_rhs(B.m, B.a, B.q2, in, out);
+        bl_rhs<FAST>(B.m, B.a, B.q2, in, out);
 #pragma unroll
         for (int i = 0; i < NB; ++i) S.k[st][i][tid] = out[i];
     }
@@ -427,7 +438,10 @@ __device__ __noinline__ void bl_finish(const BlDesc* __restrict__ Bp, BlCold<BLO
 
 // VOL: hydro model 2, each accepted step's chord through the Fishbone-Moncrief
 // torus gathered into the ray's record (args.cont.vol)
-template <int BLOCK, bool VOL = false>
+// FAST: the straight-line reciprocal of the step's right-hand sides, the same values
+// without a special-case test and branch in each (1024^2 Kerr-Newman image 22.7 / 22.0
+// ms); every camera of the launch has BF_FAST_RANGE.
+template <int BLOCK, bool VOL, bool FAST>
 __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs args) {
     __shared__ BlCold<BLOCK> S;
     const unsigned FULL = 0xffffffffu;
@@ -443,6 +457,17 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
     uint32_t acc = 0, rej = 0, flags = 0, bidx = 0, guard = 0;
     uint32_t n_cross = 0;  // disk crossings so far (translucent-disk continuation)
     int mode = BL_IDLE;
+    // A ray's end (a root on the dense output, the invariants, sin and cos of the
+    // point, the record) is a good part of a step attempt, and rays of a warp end one
+    // or two at a time.  The lane keeps its last step instead (y, k1 and h in place,
+    // k2..k7 in shared memory, y5 in local memory) and waits; the warp works the ends
+    // out together when it refills.  Measured one by one /
+    // together: 1024^2 Kerr-Newman image 24.9 / 22.7 ms.
+    uint32_t end_kind = 0;   // class of the end | BlEnd
+    bool past_disk = false;  // the current step's crossing was found off the disk
+    double end_y5_mem[NB];
+    double* end_y5 = end_y5_mem;
+    asm volatile("" : "+l"(end_y5));  // addressed memory, not seven more register pairs
 #pragma unroll
     for (int i = 0; i < NB; ++i) y[i] = k1[i] = 0.0;
     bool queue_open = true;
@@ -450,6 +475,67 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
     uint32_t n_att = 0, n_acc = 0, n_rays = 0;
 
     for (;;) {
+        {
+            // the ends waiting in this warp, when it can refill or has nothing else to do
+            const unsigned ended = __ballot_sync(FULL, mode == BL_ENDED);
+            const int n_free = __popc(__ballot_sync(FULL, mode == BL_IDLE) | ended);
+            if (ended && (n_free == 32 || ((queue_open || chunk_next < chunk_end) &&
+                                           n_free >= static_cast<int>(args.refill_threshold)))) {
+                if (mode == BL_ENDED) {
+                    const BlDesc* Bp = args.bundles + bidx;
+                    const BlDesc& B = *Bp;
+                    const uint32_t cls = end_kind & 15u, todo = end_kind & ~15u;
+                    double yt[NB], r_hit = NAN, g = 1.0;
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) yt[i] = (todo == BE_POINT) ? y[i] : end_y5[i];
+                    mode = BL_IDLE;
+                    if (todo == BE_TARGET || todo == BE_CROSSING) {
+                        const bool crossing = todo == BE_CROSSING;
+                        const double target = crossing                                  ? kHalfPi
+                                              : (cls == RT_RAY_ESCAPED)                 ? B.r_esc
+                                              : (flags & RT_RAYFLAG_EARLY_CAPTURE) != 0 ? B.r_early
+                                                                                        : B.r_capture;
+                        const int comp = crossing ? 1 : 0;
+                        const double f0 = (crossing ? y[1] : y[0]) - target, f1 = (crossing ? yt[1] : yt[0]) - target;
+                        const double lambda_step = S.lambda[tid];
+                        if (crossing || (f0 > 0.0) != (f1 > 0.0)) {
+                            double co[4][NB], k7[NB];
+#pragma unroll
+                            for (int i = 0; i < NB; ++i) k7[i] = S.k[5][i][tid];
+                            bl_dense_coeffs<BLOCK>(y, yt, k1, k7, h, S, tid, co);
+                            const double t = bl_dense_root(y, co, comp, target, f0, f1, crossing ? 1e-15 : 1e-13 * target);
+#pragma unroll
+                            for (int i = 0; i < NB; ++i) yt[i] = bl_dense_at(y, co, i, t);
+                            S.lambda[tid] = fma(t, h, lambda_step);
+                        } else {
+                            S.lambda[tid] = lambda_step + h;
+                        }
+                        if (crossing && !(yt[0] >= B.r_in && yt[0] <= B.r_out && yt[0] > B.rh * 1.02)) {
+                            // off the disk after all: the step again, past its crossing
+                            S.lambda[tid] = lambda_step;
+                            past_disk = true;
+                            --acc;
+                            --n_acc;
+                            --n_att;
+                            --guard;
+                            mode = BL_STEP;
+                        }
+                    }
+                    if (mode == BL_IDLE) {
+                        if (todo >= BE_CROSSING) {
+                            double E, L, Q;
+                            bl_invariants(B, yt, E, L, Q);
+                            r_hit = yt[0];
+                            g = disk_redshift(B.m, B.a, r_hit, L / E);
+                        }
+                        if (n_cross == 0) bl_finish<BLOCK>(Bp, S, tid, yt, cls, flags, acc, rej, r_hit, g, args.out);
+                        if (args.cont.cross)
+                            bl_cont_finish(args.cont, B, B.out_offset + S.local[tid], n_cross, cls, yt);
+                    }
+                }
+                __syncwarp();
+            }
+        }
         // refill idle lanes from the warp's chunk, then from a new chunk (one atomic)
         const unsigned idle = __ballot_sync(FULL, mode == BL_IDLE);
         const int n_idle = __popc(idle);
@@ -509,7 +595,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
             if (!queue_open && chunk_next >= chunk_end) break;
             continue;
         }
-        if (mode == BL_IDLE) continue;
+        if (mode == BL_IDLE || mode == BL_ENDED) continue;
 
         const BlDesc* Bp = args.bundles + bidx;
         const BlDesc& B = *Bp;
@@ -534,15 +620,14 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
             }
         }
         if (term) {
-            if (n_cross == 0) bl_finish<BLOCK>(Bp, S, tid, y, term & 15u, flags, acc, rej, NAN, 1.0, args.out);
-            if (args.cont.cross) bl_cont_finish(args.cont, B, B.out_offset + S.local[tid], n_cross, term & 15u, y);
-            mode = BL_IDLE;
+            end_kind = (term & 15u) | BE_POINT;
+            mode = BL_ENDED;
             continue;
         }
 
         const double hh = h;
         double y5[NB];
-        double err = bl_stages<BLOCK>(B, y, k1, hh, S, tid, y5);
+        double err = bl_stages<BLOCK, FAST>(B, y, k1, hh, S, tid, y5);
         if (!(err <= 1e300)) err = 1e300;
         ++n_att;
         if (err > 1.0) {
@@ -563,21 +648,26 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
 #pragma unroll
         for (int i = 0; i < NB; ++i) finite = finite && isfinite(y5[i]);
         if (!finite) {
-            if (n_cross == 0)
-                bl_finish<BLOCK>(Bp, S, tid, y, RT_RAY_CAPTURED, flags | RT_RAYFLAG_NONFINITE, acc, rej, NAN, 1.0,
-                                 args.out);
-            if (args.cont.cross)
-                bl_cont_finish(args.cont, B, B.out_offset + S.local[tid], n_cross, RT_RAY_CAPTURED, y);
-            mode = BL_IDLE;
+            flags |= RT_RAYFLAG_NONFINITE;
+            end_kind = RT_RAY_CAPTURED | BE_POINT;
+            mode = BL_ENDED;
             continue;
         }
         // disk: the theta = pi/2 crossing of this step, when its root lies on the disk
-        if (B.flags & BF_DISK) {
+        if ((B.flags & BF_DISK) && !past_disk) {
             const double f0 = y[1] - kHalfPi, f1 = y5[1] - kHalfPi;
             if (f0 * f1 <= 0.0 && f0 != f1) {
                 const double sl = f0 / (f0 - f1);
                 const double re = y[0] + sl * (y5[0] - y[0]);
                 const double margin = 0.05 * re + 0.5 * B.m;
+                if (!args.cont.cross && re >= B.r_in + margin && re <= B.r_out - margin) {
+                    // well on the disk by the chord: the root with the other ends
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) end_y5[i] = y5[i];
+                    end_kind = static_cast<uint32_t>(RT_RAY_DISK) | BE_CROSSING;
+                    mode = BL_ENDED;
+                    continue;
+                }
                 if (re >= B.r_in - margin && re <= B.r_out + margin) {
                     double co[4][NB];
                     bl_dense_coeffs<BLOCK>(y, y5, k1, k7, hh, S, tid, co);
@@ -587,6 +677,14 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
                     for (int i = 0; i < NB; ++i) yr[i] = bl_dense_at(y, co, i, t);
                     const double rr = yr[0];
                     if (rr >= B.r_in && rr <= B.r_out && rr > B.rh * 1.02) {
+                        if (!args.cont.cross) {
+                            S.lambda[tid] = fma(t, hh, S.lambda[tid]);
+#pragma unroll
+                            for (int i = 0; i < NB; ++i) end_y5[i] = yr[i];
+                            end_kind = RT_RAY_DISK | BE_DISK;
+                            mode = BL_ENDED;
+                            continue;
+                        }
                         double E, L, Q;
                         bl_invariants(B, yr, E, L, Q);
                         const double g = disk_redshift(B.m, B.a, rr, L / E);
@@ -598,7 +696,6 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
                             S.lambda[tid] = lambda_step;
                         }
                         mode = BL_IDLE;
-                        if (!args.cont.cross) continue;
                         // translucent disk: record the crossing (at the record's azimuth,
                         // that of the reflected root point) and go on through it
                         double yp[NB];
@@ -617,18 +714,16 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
                 }
             }
         }
+        past_disk = false;
         // capture / escape / certain capture inside this step: the terminal point on
         // the dense output at the threshold radius
         {
-            double target = 0.0;
             uint32_t tterm = 0;
             const double rn = y5[0];
             if (rn < B.r_capture) {
                 tterm = RT_RAY_CAPTURED;
-                target = B.r_capture;
             } else if (rn > B.r_esc) {
                 tterm = RT_RAY_ESCAPED;
-                target = B.r_esc;
             } else if (can_early != 0 && rn < B.r_early) {
                 if (can_early < 0) {
                     const double e0 = S.e0[tid];
@@ -639,27 +734,13 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
                 if (can_early > 0 && y5[4] > 0.0) {
                     tterm = RT_RAY_CAPTURED;
                     flags |= RT_RAYFLAG_EARLY_CAPTURE;
-                    target = B.r_early;
                 }
             }
             if (tterm) {
-                double yt[NB];
-                const double f0 = y[0] - target, f1 = rn - target;
-                if ((f0 > 0.0) != (f1 > 0.0)) {
-                    double co[4][NB];
-                    bl_dense_coeffs<BLOCK>(y, y5, k1, k7, hh, S, tid, co);
-                    const double t = bl_dense_root(y, co, 0, target, f0, f1, 1e-13 * target);
 #pragma unroll
-                    for (int i = 0; i < NB; ++i) yt[i] = bl_dense_at(y, co, i, t);
-                    S.lambda[tid] += t * hh;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < NB; ++i) yt[i] = y5[i];
-                    S.lambda[tid] += hh;
-                }
-                if (n_cross == 0) bl_finish<BLOCK>(Bp, S, tid, yt, tterm, flags, acc, rej, NAN, 1.0, args.out);
-                if (args.cont.cross) bl_cont_finish(args.cont, B, B.out_offset + S.local[tid], n_cross, tterm, yt);
-                mode = BL_IDLE;
+                for (int i = 0; i < NB; ++i) end_y5[i] = y5[i];
+                end_kind = tterm | BE_TARGET;
+                mode = BL_ENDED;
                 continue;
             }
         }
@@ -704,14 +785,16 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
     }
 }
 
-template __global__ void bl_trace_kernel<128, false>(BlArgs);
-template __global__ void bl_trace_kernel<128, true>(BlArgs);
+template __global__ void bl_trace_kernel<128, false, false>(BlArgs);
+template __global__ void bl_trace_kernel<128, false, true>(BlArgs);
+template __global__ void bl_trace_kernel<128, true, false>(BlArgs);
+template __global__ void bl_trace_kernel<128, true, true>(BlArgs);
 
 }  // namespace
 
 uint32_t bl_trace_grid(int sm_count) {
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bl_trace_kernel<128, false>, 128, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bl_trace_kernel<128, false, true>, 128, 0) != cudaSuccess) {
         cudaGetLastError();
         occ = 1;
     }
@@ -719,10 +802,14 @@ uint32_t bl_trace_grid(int sm_count) {
 }
 
 void launch_bl_trace(const BlArgs& args, uint32_t grid, void* stream) {
-    if (args.cont.vol)
-        bl_trace_kernel<128, true><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(args);
-    else
-        bl_trace_kernel<128, false><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(args);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (args.cont.vol) {
+        if (args.fast_range) bl_trace_kernel<128, true, true><<<grid, 128, 0, s>>>(args);
+        else bl_trace_kernel<128, true, false><<<grid, 128, 0, s>>>(args);
+    } else {
+        if (args.fast_range) bl_trace_kernel<128, false, true><<<grid, 128, 0, s>>>(args);
+        else bl_trace_kernel<128, false, false><<<grid, 128, 0, s>>>(args);
+    }
 }
 
 }  // namespace relsim

@@ -214,7 +214,12 @@ void build_bl_bundle(const rt_camera& cam, uint32_t col0, uint32_t ncols, uint32
     b.cap_c = cam.step_cap_fraction;
     b.h0 = cam.initial_step_fraction * r_obs;
     b.proj_tol = cam.projection_tol;
-    b.flags = (disk ? BF_DISK : 0u) | (cam.early_capture ? BF_EARLY_CAPTURE : 0u);
+    // The stages divide by rho^2 Delta sin^2(theta).  A step is at most cap_c (r - r_+),
+    // so a stage stays near its step's start: r^4 below 1e130, Delta as far from zero as
+    // the capture radius keeps it, and sin^2 is held above 1e-30.
+    const bool fast = r_obs <= 1e30 && b.r_esc <= 1e30 && m <= 1e30 && cam.capture_scale >= 1.0 + 1e-6 &&
+                      b.cap_c <= 0.5;
+    b.flags = (disk ? BF_DISK : 0u) | (cam.early_capture ? BF_EARLY_CAPTURE : 0u) | (fast ? BF_FAST_RANGE : 0u);
 }
 
 // Source table of a multi-source scene (software_compute_engine.hpp:2738-2798):

@@ -19,7 +19,9 @@ static_assert(sizeof(rt_ray_out) == kRayFields * sizeof(void*), "rt_ray_out is a
 enum : uint32_t {
     BF_DISK = 1u << 0,          // thin disk present
     BF_EARLY_CAPTURE = 1u << 1, // Carter early capture allowed
-    BF_MIXED = 1u << 2          // mixed-precision stages
+    BF_MIXED = 1u << 2,         // mixed-precision stages
+    BF_FAST_RANGE = 1u << 3     // Boyer-Lindquist: the stages' reciprocal stays far from the ends of the
+                                // range (the straight-line form of rt_fast_math.h gives the same values)
 };
 
 // Mixed mode: the near-critical band (M, distance of a ray's constants from
@@ -221,7 +223,7 @@ struct BlArgs {
     uint32_t n_bundles;
     uint32_t refill_threshold;
     uint32_t claim;
-    uint32_t pad;
+    uint32_t fast_range;  // every bundle has BF_FAST_RANGE
     uint64_t total_rays;
     unsigned long long* queue;
     unsigned long long* stats;

@@ -10,7 +10,6 @@
 // (de / 4)^9 / 9! for the bluest node's exponent change de = 0.3 over a piece is
 // 4e-16; the rest is rounding).  27 fused operations and one reciprocal replace the
 // sum.  Colder than 500 K, where the sum drops nodes, it is evaluated as it stands.
-// MEASURED
 #pragma once
 
 #include <cmath>

@@ -415,6 +415,9 @@ bool launch_epoch(rt_server* s, Slot& slot) {
         BlArgs ba{};
         ba.bundles = slot.dev_bl;
         ba.n_bundles = nb;
+        ba.fast_range = 1u;
+        for (uint32_t b = 0; b < nb; ++b)
+            if (!(slot.host_bl[b].flags & BF_FAST_RANGE)) ba.fast_range = 0u;
         ba.refill_threshold = c.refill_threshold;
         ba.claim = 32u * c.rays_per_thread;
         ba.total_rays = total;

@@ -249,3 +249,21 @@ def test_charge_sign_does_not_matter(tracer):
     b = tracer.dispatch(neg, fields=FIELDS, pixels=True)
     for k in a:
         np.testing.assert_array_equal(a[k], b[k])
+
+
+@pytest.mark.parametrize("kw", [dict(step_cap=0.1), dict(step_cap=0.1, capture_scale=1.0), dict(step_cap=0.500001)])
+def test_range_rule_of_the_reciprocal(tracer, kw):
+    """Cameras on both sides of the rule that picks the stages' reciprocal (step cap, capture
+    radius) against the oracle, at the bars of the full images."""
+    tracer.set_launch_config()
+    cam = relsim.make_camera(metric_form=relsim.METRIC_BOYER_LINDQUIST, spin=0.7, charge=0.4, r_obs=30.0, incl_deg=70.0,
+                             fov_deg=30.0, width=40, height=30, **kw)
+    out = tracer.dispatch(cam)
+    ref = O.bl_trace(relsim.camera_dict(cam), 0.4)
+    ok = np.abs(ref["db_shadow"]) > 1e-3
+    np.testing.assert_array_equal(out["status"][ok], ref["status"][ok])
+    done = ok & ((ref["status"] == O.DISK) | (ref["status"] == O.ESCAPED))
+    assert done.sum() > 600
+    for f in ("r", "theta"):
+        rel = np.abs(out[f][done] / ref[f][done] - 1.0)
+        assert np.mean(rel < 1e-9) > 0.995 and rel.max() < 1e-6, (f, rel.max())
