@@ -567,6 +567,7 @@ rt_status ms_launch(rt_handle* h, const rt_camera* cam, const rt_source* src, ui
     args.bundles = static_cast<const MsDesc*>(h->ms_desc.ptr);
     args.sources = static_cast<const MsSource*>(h->ms_sources.ptr);
     args.n_bundles = 1;
+    args.sources_per_ray = count;
     args.refill_threshold = c.refill_threshold;
     args.claim = 32u * c.rays_per_thread;
     args.total_rays = static_cast<uint64_t>(cam->screen_width) * nrows;
@@ -575,7 +576,7 @@ rt_status ms_launch(rt_handle* h, const rt_camera* cam, const rt_source* src, ui
     args.out = out;
     args.cont = h->cur_cont;
     RT_CUDA(h, cudaEventRecord(h->ev0, s));
-    launch_ms_trace(args, ms_trace_grid(h->sm_count), s);
+    launch_ms_trace(args, h->sm_count, s);
     RT_CUDA(h, cudaGetLastError());
     RT_CUDA(h, cudaEventRecord(h->ev1, s));
     h->timed = true;

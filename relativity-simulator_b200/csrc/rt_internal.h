@@ -191,7 +191,7 @@ struct MsArgs {
     uint32_t n_bundles;
     uint32_t refill_threshold;
     uint32_t claim;
-    uint32_t pad;
+    uint32_t sources_per_ray;  // mean over the launch's rays (chooses the launch's shape)
     uint64_t total_rays;
     unsigned long long* queue;
     unsigned long long* stats;
@@ -331,8 +331,7 @@ uint32_t kernel_block(uint32_t block, bool mixed, bool rolled);
 rt_launch_config resolve_launch_config(rt_launch_config c, bool mixed);
 
 // Multi-source tracer (rt_multi.cu).
-void launch_ms_trace(const MsArgs& args, uint32_t grid, void* stream);
-uint32_t ms_trace_grid(int sm_count);
+void launch_ms_trace(const MsArgs& args, int sm_count, void* stream);
 
 // Boyer-Lindquist Kerr-Newman tracer (rt_bl.cu).
 void launch_bl_trace(const BlArgs& args, uint32_t grid, void* stream);

@@ -18,7 +18,8 @@
 //     trace_multi_source (:3155).
 // Sources live in global memory per bundle (at most 16, read through L1 by
 // whole warps of one bundle).  The stage loop is rolled around one copy of the
-// N-source RHS, its stage derivatives in shared memory.
+// N-source RHS, its stage derivatives in shared memory.  In launches of few rays
+// several lanes share a ray (Group).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -59,57 +60,201 @@ struct MsCold {
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
+// ---- the superposed right-hand side ----
+//
+// A source's term is a chain of some 60 dependent FP64 operations, and a ray takes six
+// of them per source and attempt in turn: latency bounds the kernel, not the FP64
+// pipe.  Two ways to overlap terms: one lane interleaves U sources, or G lanes of a
+// warp share a ray, each evaluating every G-th source.  The terms are always added up
+// in source order, and every product and sum is written with its rounding (no
+// contraction is left to the compiler), so a ray's steps depend on neither G nor U.
+template <int G>
+struct Group {
+    unsigned mask;  // the group's lanes
+    int sub;        // this lane's place among them
+    __device__ __forceinline__ double from(double v, int q) const {
+        if constexpr (G == 1) return v;
+        else return __shfl_sync(mask, v, q, G);
+    }
+};
+
+// a . b, the first product fused into the second
+__device__ __forceinline__ double dot3x(const double* a, const double* b) {
+    return __fma_rn(a[2], b[2], __fma_rn(a[0], b[0], __dmul_rn(a[1], b[1])));
+}
+
+// Component k in the world frame of a vector with local components v.
+__device__ __forceinline__ double ms_world(const MsSource& s, const double* v, int k) {
+    return __fma_rn(v[2], s.axis[k], __fma_rn(v[0], s.fx[k], __dmul_rn(v[1], s.fy[k])));
+}
+
+// r^2 of a local Kerr-Schild point and the pieces that share it.
+template <bool FAST>
+__device__ __forceinline__ double ms_r2(const double* x, double a2, double z2, bool square_fused) {
+    double d = __fma_rn(x[0], x[0], __dmul_rn(x[1], x[1]));
+    d = __dadd_rn(__dadd_rn(d, z2), -a2);
+    const double t4 = __dmul_rn(4.0, a2);
+    const double v = square_fused ? __fma_rn(d, d, __dmul_rn(t4, z2)) : __fma_rn(t4, z2, __dmul_rn(d, d));
+    if constexpr (FAST) {
+        const double r2 = __dmul_rn(0.5, __dadd_rn(d, fast_sqrt(v)));
+        return (r2 < 1e-24) ? 1e-24 : r2;
+    } else {
+        return fmax(__dmul_rn(0.5, __dadd_rn(d, __dsqrt_rn(v))), 1e-24);
+    }
+}
+
+// U sources' terms of the right-hand side in the world frame (the gravitational part
+// of ks_rhs in each local frame), with r_BL in that frame.  The reciprocal roots sit
+// between two straight-line halves, each of which interleaves the sources.
+template <int U, bool FAST>
+__device__ __forceinline__ void ms_terms(const MsSource* __restrict__ const* sp, const double* __restrict__ y,
+                                         double (*__restrict__ term)[6], double* __restrict__ rout) {
+    double X[U][3], P[U][3], R2[U], IR[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const MsSource& s = *sp[u];
+        const double rel[3] = {__dadd_rn(y[0], -s.pos[0]), __dadd_rn(y[1], -s.pos[1]), __dadd_rn(y[2], -s.pos[2])};
+        X[u][0] = dot3x(rel, s.fx);
+        X[u][1] = dot3x(rel, s.fy);
+        X[u][2] = dot3x(rel, s.axis);
+        P[u][0] = dot3x(y + 3, s.fx);
+        P[u][1] = dot3x(y + 3, s.fy);
+        P[u][2] = dot3x(y + 3, s.axis);
+        R2[u] = ms_r2<FAST>(X[u], __dmul_rn(s.a, s.a), __dmul_rn(X[u][2], X[u][2]), true);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) IR[u] = rsqrt(R2[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const MsSource& s = *sp[u];
+        const double* x = X[u];
+        const double px = P[u][0], py = P[u][1], pz = P[u][2];
+        const double M = s.m, a = s.a;
+        const double a2 = __dmul_rn(a, a), z2 = __dmul_rn(x[2], x[2]);
+        const double r2 = R2[u], inv_r = IR[u];
+        const double r = __dmul_rn(r2, inv_r);
+        const double rpa = __dadd_rn(r2, a2);
+        const double r4 = __dmul_rn(r2, r2);
+        const double den = __fma_rn(a2, z2, r4);
+        double q;
+        if constexpr (FAST) q = fast_rcp(__dmul_rn(rpa, den));
+        else q = __drcp_rn(__dmul_rn(rpa, den));
+        const double inv_rpa = __dmul_rn(den, q), inv_den = __dmul_rn(rpa, q);
+        const double r3 = __dmul_rn(r2, r);
+        const double H = __dmul_rn(__dmul_rn(M, r3), inv_den);
+        const double k[3] = {__dmul_rn(__fma_rn(a, x[1], __dmul_rn(r, x[0])), inv_rpa),
+                             __dmul_rn(__fma_rn(r, x[1], -__dmul_rn(a, x[0])), inv_rpa), __dmul_rn(x[2], inv_r)};
+        const double sv = __fma_rn(k[2], pz, __fma_rn(k[1], py, __fma_rn(k[0], px, 1.0)));
+        const double th = __dmul_rn(__dmul_rn(2.0, H), sv);
+        const double r3d = __dmul_rn(r3, inv_den);
+        const double drz = __dmul_rn(__dmul_rn(__dmul_rn(r, rpa), x[2]), inv_den);
+        const double c = __fma_rn(__dmul_rn(3.0, a2), z2, -r4);
+        const double C = __dmul_rn(__dmul_rn(__dmul_rn(M, r2), inv_den), __dmul_rn(c, inv_den));
+        const double D = __dmul_rn(__dmul_rn(-2.0, H), __dmul_rn(__dmul_rn(a2, x[2]), inv_den));
+        const double tr = __dmul_rn(2.0, r);
+        const double U = __fma_rn(-tr, k[0], x[0]), V = __fma_rn(-tr, k[1], x[1]);
+        const double W = __fma_rn(U, px, __dmul_rn(V, py));
+        const double A = __fma_rn(inv_rpa, W, -__dmul_rn(__dmul_rn(inv_r, k[2]), pz));
+        const double B0 = __dmul_rn(inv_rpa, __fma_rn(r, px, -__dmul_rn(a, py)));
+        const double B1 = __dmul_rn(inv_rpa, __fma_rn(a, px, __dmul_rn(r, py)));
+        const double B2 = __dmul_rn(inv_r, pz);
+        const double s2 = __dmul_rn(sv, sv);
+        const double Gd = __fma_rn(s2, C, __dmul_rn(th, A));
+        const double dx[3] = {-__dmul_rn(th, k[0]), -__dmul_rn(th, k[1]), -__dmul_rn(th, k[2])};
+        const double dp[3] = {__fma_rn(th, B0, __dmul_rn(__dmul_rn(r3d, x[0]), Gd)),
+                              __fma_rn(th, B1, __dmul_rn(__dmul_rn(r3d, x[1]), Gd)),
+                              __fma_rn(s2, D, __fma_rn(th, B2, __dmul_rn(drz, Gd)))};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            term[u][i] = ms_world(s, dx, i);
+            term[u][3 + i] = ms_world(s, dp, i);
+        }
+        rout[u] = r;
+    }
+}
+
 // Superposed RHS; returns min_i max(r_i - r_+i, 0.01 m_i) and the first source
 // whose local r_BL < capture_scale r_+ (-1: none).
-__device__ double ms_rhs(const MsSource* __restrict__ src, uint32_t n, const double* __restrict__ y,
-                         double* __restrict__ dy, double cap_scale, int& inside) {
+template <int G, int U, bool FAST>
+__device__ __forceinline__ double ms_rhs(const MsSource* __restrict__ src, uint32_t n, const double* __restrict__ y,
+                                         double* __restrict__ dy, double cap_scale, int& inside, const Group<G>& grp) {
     double cap = 1e300;
-    int in = -1;
+    int in = 0x7fffffff;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         dy[k] = y[3 + k];
         dy[3 + k] = 0.0;
     }
+    uint32_t base = 0;
+    if constexpr (U > 1) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < n; ++i) {
-        const MsSource& s = src[i];
-        const double rel[3] = {y[0] - s.pos[0], y[1] - s.pos[1], y[2] - s.pos[2]};
-        double ly[6];
-        ly[0] = dot3(rel, s.fx);
-        ly[1] = dot3(rel, s.fy);
-        ly[2] = dot3(rel, s.axis);
-        ly[3] = dot3(y + 3, s.fx);
-        ly[4] = dot3(y + 3, s.fy);
-        ly[5] = dot3(y + 3, s.axis);
-        double ld[6], hf, sv;
-        const double r = ks_rhs<double, true>(ly, s.m, s.a, ld, hf, sv);
+        for (; base + U <= n; base += U) {
+            double term[U][6], r[U];
+            const MsSource* sp[U];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            dy[k] += ld[0] * s.fx[k] + ld[1] * s.fy[k] + ld[2] * s.axis[k];
-            dy[3 + k] += ld[3] * s.fx[k] + ld[4] * s.fy[k] + ld[5] * s.axis[k];
+            for (int u = 0; u < U; ++u) sp[u] = src + base + u;
+            ms_terms<U, FAST>(sp, y, term, r);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) dy[k] = __dadd_rn(dy[k], term[u][k]);
+                cap = fmin(cap, fmax(r[u] - sp[u]->rh, 0.01 * sp[u]->m));
+                if (r[u] < cap_scale * sp[u]->rh && in == 0x7fffffff) in = static_cast<int>(base + u);
+            }
         }
-        cap = fmin(cap, fmax(r - s.rh, 0.01 * s.m));
-        if (in < 0 && r < cap_scale * s.rh) in = static_cast<int>(i);
     }
-    inside = in;
+#pragma unroll 1
+    for (; base < n; base += G) {
+        double term[1][6], r[1];
+        const uint32_t i = base + grp.sub;
+        if (i < n) {
+            const MsSource* sp[1] = {src + i};
+            ms_terms<1, FAST>(sp, y, term, r);
+            cap = fmin(cap, fmax(r[0] - sp[0]->rh, 0.01 * sp[0]->m));
+            if (r[0] < cap_scale * sp[0]->rh && in == 0x7fffffff) in = static_cast<int>(i);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) term[0][k] = 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            double t[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) t[k] = grp.from(term[0][k], q);
+            if (base + q < n) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) dy[k] = __dadd_rn(dy[k], t[k]);
+            }
+        }
+    }
+    if constexpr (G > 1) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            cap = fmin(cap, __shfl_xor_sync(grp.mask, cap, o, G));
+            in = min(in, __shfl_xor_sync(grp.mask, in, o, G));
+        }
+    }
+    inside = (in == 0x7fffffff) ? -1 : in;
     return cap;
 }
 
-// Stages 2..7 around one RHS copy; K holds k2..k7 on return.
-template <int BLOCK>
+// Stages 2..7 around one RHS copy; K holds k2..k7 on return.  The stage sums are
+// unrolled over j (predicated), so their shared-memory loads issue together.
+template <int BLOCK, int G, int U, bool FAST>
 __device__ __forceinline__ void ms_stages(const MsSource* __restrict__ src, uint32_t n, const double* __restrict__ y,
                                           const double* __restrict__ k1, double hh, MsCold<BLOCK>& S, int tid,
                                           double cap_scale, double* __restrict__ y5, double* __restrict__ k7,
-                                          double* __restrict__ est, double& cap5, int& inside5) {
+                                          double* __restrict__ est, double& cap5, int& inside5, const Group<G>& grp) {
 #pragma unroll 1
     for (int st = 0; st < 6; ++st) {
         double in[6];
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-            double acc = kMsA[st][0] * k1[i];
-#pragma unroll 1
-            for (int j = 1; j <= st; ++j) acc += kMsA[st][j] * S.k[j - 1][i][tid];
-            in[i] = y[i] + hh * acc;
+            double acc = __dmul_rn(kMsA[st][0], k1[i]);
+#pragma unroll
+            for (int j = 1; j < 6; ++j)
+                if (j <= st) acc = __fma_rn(kMsA[st][j], S.k[j - 1][i][tid], acc);
+            in[i] = __fma_rn(hh, acc, y[i]);
         }
         if (st == 5) {
 #pragma unroll
@@ -117,7 +262,7 @@ __device__ __forceinline__ void ms_stages(const MsSource* __restrict__ src, uint
         }
         double out[6];
         int ins;
-        const double c = ms_rhs(src, n, in, out, cap_scale, ins);
+        const double c = ms_rhs<G, U, FAST>(src, n, in, out, cap_scale, ins, grp);
 #pragma unroll
         for (int i = 0; i < 6; ++i) S.k[st][i][tid] = out[i];
         if (st == 5) {
@@ -129,11 +274,36 @@ __device__ __forceinline__ void ms_stages(const MsSource* __restrict__ src, uint
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-        double acc = kMsE[0] * k1[i];
-#pragma unroll 1
-        for (int j = 2; j < 7; ++j) acc += kMsE[j] * S.k[j - 1][i][tid];
-        est[i] = fabs(hh) * fabs(acc);
+        double acc = __dmul_rn(kMsE[0], k1[i]);
+#pragma unroll
+        for (int j = 2; j < 7; ++j) acc = __fma_rn(kMsE[j], S.k[j - 1][i][tid], acc);
+        est[i] = __dmul_rn(fabs(hh), fabs(acc));
     }
+}
+
+// The attempt with the compiler's division and root, for an attempt whose stages
+// leave the fast forms' range (its error estimate is NaN: one NaN term makes all six
+// sums NaN).  Out of line: y and k1 in io[0..11], then y5, k7, est and cap5.
+template <int BLOCK, int G>
+__device__ __noinline__ int ms_stages_special(const MsSource* __restrict__ src, uint32_t n, double* __restrict__ io,
+                                              double hh, MsCold<BLOCK>& S, int tid, double cap_scale,
+                                              const Group<G> grp) {
+    double y[6], k1[6], y5[6], k7[6], est[6], cap5 = 0.0;
+    int inside5 = -1;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        y[i] = io[i];
+        k1[i] = io[6 + i];
+    }
+    ms_stages<BLOCK, G, 1, false>(src, n, y, k1, hh, S, tid, cap_scale, y5, k7, est, cap5, inside5, grp);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        io[12 + i] = y5[i];
+        io[18 + i] = k7[i];
+        io[24 + i] = est[i];
+    }
+    io[30] = cap5;
+    return inside5;
 }
 
 // Coefficients of the step's dense output y(t) = y0 + t (d + (1-t)(b + t(c + (1-t) e))).
@@ -214,55 +384,100 @@ __device__ double ms_radius_crossing(const double* y0, const double* f0, const d
     return t;
 }
 
-// Projection of p onto H = 0 along n = dH/dp, closest root; returns |H| before.
-// Two passes over the sources (n needs all of them first).
-__device__ double ms_project(const MsSource* __restrict__ src, uint32_t n, double* y, double tol) {
+// Kerr-Schild field of one source at a world point: k in the world frame, H.
+template <bool FAST>
+__device__ __forceinline__ double ms_field(const MsSource& s, const double* __restrict__ at, double* __restrict__ kw) {
+    const double rel[3] = {__dadd_rn(at[0], -s.pos[0]), __dadd_rn(at[1], -s.pos[1]), __dadd_rn(at[2], -s.pos[2])};
+    const double x[3] = {dot3x(rel, s.fx), dot3x(rel, s.fy), dot3x(rel, s.axis)};
+    const double a = s.a, a2 = __dmul_rn(a, a);
+    const double r2 = ms_r2<FAST>(x, a2, __dmul_rn(x[2], x[2]), false);
+    const double inv_r = rsqrt(r2);
+    const double r = __dmul_rn(r2, inv_r);
+    const double rpa = __dadd_rn(r2, a2);
+    const double den = __fma_rn(__dmul_rn(a2, x[2]), x[2], __dmul_rn(r2, r2));
+    double q;
+    if constexpr (FAST) q = fast_rcp(__dmul_rn(rpa, den));
+    else q = __drcp_rn(__dmul_rn(rpa, den));
+    const double inv_rpa = __dmul_rn(den, q);
+    const double k[3] = {__dmul_rn(__fma_rn(a, x[1], __dmul_rn(r, x[0])), inv_rpa),
+                         __dmul_rn(__fma_rn(r, x[1], -__dmul_rn(a, x[0])), inv_rpa), __dmul_rn(x[2], inv_r)};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) kw[i] = ms_world(s, k, i);
+    return __dmul_rn(__dmul_rn(__dmul_rn(s.m, r2), r), __dmul_rn(rpa, q));
+}
+
+// Projection of p onto H = 0 along n = dH/dp, closest root; returns |H| before (NaN,
+// with p as it was, where a field leaves the fast forms' range).  Two passes over
+// the sources (n needs all of them first).
+template <int G, bool FAST>
+__device__ __forceinline__ double ms_project(const MsSource* __restrict__ src, uint32_t n, double* y, double tol,
+                                             const Group<G>& grp) {
     double* p = y + 3;
     double nv[3] = {p[0], p[1], p[2]};
     double sum = 0.0;
 #pragma unroll 1
-    for (uint32_t i = 0; i < n; ++i) {
-        const MsSource& s = src[i];
-        const double rel[3] = {y[0] - s.pos[0], y[1] - s.pos[1], y[2] - s.pos[2]};
-        const double lx[3] = {dot3(rel, s.fx), dot3(rel, s.fy), dot3(rel, s.axis)};
-        double kl[3], hf;
-        ks_field64(lx, s.m, s.a, kl, hf);
-        double kw[3];
+    for (uint32_t base = 0; base < n; base += G) {
+        const uint32_t i = base + grp.sub;
+        double kw[3] = {0.0, 0.0, 0.0}, hs = 0.0, sv = 0.0, c = 0.0;
+        if (i < n) {
+            const double hf = ms_field<FAST>(src[i], y, kw);
+            sv = __dadd_rn(1.0, dot3x(kw, p));
+            hs = __dmul_rn(hf, sv);
+            c = __dmul_rn(__dmul_rn(2.0, hf), sv);
+        }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) kw[k] = kl[0] * s.fx[k] + kl[1] * s.fy[k] + kl[2] * s.axis[k];
-        const double sv = 1.0 + dot3(kw, p);
-        sum += hf * sv * sv;
+        for (int q = 0; q < G; ++q) {
+            const double hq = grp.from(hs, q), sq = grp.from(sv, q), cq = grp.from(c, q);
+            double kq[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) nv[k] -= 2.0 * hf * sv * kw[k];
+            for (int k = 0; k < 3; ++k) kq[k] = grp.from(kw[k], q);
+            if (base + q < n) {
+                sum = __fma_rn(hq, sq, sum);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) nv[k] = __fma_rn(-cq, kq[k], nv[k]);
+            }
+        }
     }
-    const double res = 0.5 * (dot3(p, p) - 1.0) - sum;
+    const double res = __fma_rn(0.5, __dadd_rn(dot3x(p, p), -1.0), -sum);
     if (!(fabs(res) >= tol)) return fabs(res);
-    double qa = 0.5 * dot3(nv, nv), qb = dot3(p, nv);
+    double qa = __dmul_rn(0.5, dot3x(nv, nv)), qb = dot3x(p, nv);
 #pragma unroll 1
-    for (uint32_t i = 0; i < n; ++i) {
-        const MsSource& s = src[i];
-        const double rel[3] = {y[0] - s.pos[0], y[1] - s.pos[1], y[2] - s.pos[2]};
-        const double lx[3] = {dot3(rel, s.fx), dot3(rel, s.fy), dot3(rel, s.axis)};
-        double kl[3], hf;
-        ks_field64(lx, s.m, s.a, kl, hf);
-        double kw[3];
+    for (uint32_t base = 0; base < n; base += G) {
+        const uint32_t i = base + grp.sub;
+        double kn = 0.0, ha = 0.0, hb = 0.0;
+        if (i < n) {
+            double kw[3];
+            const double hf = ms_field<FAST>(src[i], y, kw);
+            const double sv = __dadd_rn(1.0, dot3x(kw, p));
+            kn = dot3x(kw, nv);
+            ha = __dmul_rn(hf, kn);
+            hb = __dmul_rn(__dmul_rn(2.0, hf), sv);
+        }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) kw[k] = kl[0] * s.fx[k] + kl[1] * s.fy[k] + kl[2] * s.axis[k];
-        const double sv = 1.0 + dot3(kw, p);
-        const double kn = dot3(kw, nv);
-        qa -= hf * kn * kn;
-        qb -= 2.0 * hf * sv * kn;
+        for (int q = 0; q < G; ++q) {
+            const double kq = grp.from(kn, q), aq = grp.from(ha, q), bq = grp.from(hb, q);
+            if (base + q < n) {
+                qa = __fma_rn(-aq, kq, qa);
+                qb = __fma_rn(-bq, kq, qb);
+            }
+        }
     }
-    const double disc = qb * qb - 4.0 * qa * res;
+    const double disc = __fma_rn(qb, qb, -__dmul_rn(__dmul_rn(4.0, qa), res));
     if (disc >= 0.0) {
-        const double q = -0.5 * (qb + copysign(sqrt(disc), qb));
+        const double q = __dmul_rn(-0.5, __dadd_rn(qb, copysign(__dsqrt_rn(disc), qb)));
         if (q != 0.0) {
-            const double alpha = res / q;
+            const double alpha = __ddiv_rn(res, q);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) p[k] += alpha * nv[k];
+            for (int k = 0; k < 3; ++k) p[k] = __fma_rn(alpha, nv[k], p[k]);
         }
     }
     return fabs(res);
+}
+
+template <int G>
+__device__ __noinline__ double ms_project_special(const MsSource* __restrict__ src, uint32_t n, double* y, double tol,
+                                                  const Group<G> grp) {
+    return ms_project<G, false>(src, n, y, tol, grp);
 }
 
 // Static observer's null momentum in the superposed metric (ms_initial_momentum,
@@ -387,7 +602,7 @@ __device__ __noinline__ void ms_finish(const MsDesc* __restrict__ Bp, const MsSo
         if (status == RT_RAY_ESCAPED) {
             double dy[6];
             int ins;
-            ms_rhs(src, Bp->src_count, y, dy, Bp->capture_scale, ins);
+            ms_rhs<1, 1, false>(src, Bp->src_count, y, dy, Bp->capture_scale, ins, Group<1>{0u, 0});
             const double len = sqrt(dot3(dy, dy));
             if (len > 1e-12) {
 #pragma unroll
@@ -441,7 +656,7 @@ __device__ __noinline__ void ms_cont_finish(const ContOut& C, uint64_t o, uint32
         // superposed RHS, (0, 0, -1) where it vanishes (:3220-3224)
         double dy[6], e[3] = {0.0, 0.0, -1.0};
         int ins;
-        ms_rhs(src, n, x, dy, 1.0, ins);
+        ms_rhs<1, 1, false>(src, n, x, dy, 1.0, ins, Group<1>{0u, 0});
         const double len = sqrt(dot3(dy, dy));
         if (len > 1e-12)
             for (int i = 0; i < 3; ++i) e[i] = -dy[i] / len;
@@ -457,13 +672,18 @@ __device__ __forceinline__ void ms_unwrap(double& phi, const double* y) {
     phi += d;
 }
 
-template <int BLOCK, bool CONT>
-__global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs args) {
+// Eight warps per SM: at 12 (168 registers) the two interleaved sources spill, and the
+// chain of an attempt, which is what bounds this kernel, gets longer (5 holes: 480x270
+// 23.9 ms at 12 warps and one source at a time, 20.3 at 8 and two; 160x90 17.8 / 13.0).
+template <int BLOCK, bool CONT, int G, int U>
+__global__ void __launch_bounds__(BLOCK, 256 / BLOCK) ms_trace_kernel(MsArgs args) {
     __shared__ MsCold<BLOCK> S;
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
+    const Group<G> grp{((1u << G) - 1u) << (lane & ~(G - 1)), lane & (G - 1)};
+    const bool leader = grp.sub == 0;
 
     double y[6], k1[6];
     double h = 0.0, cap_len = 0.0;
@@ -488,7 +708,8 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
             const uint64_t avail = chunk_end - chunk_next;
             uint64_t base2 = 0;
             bool got2 = false;
-            if (avail < static_cast<uint64_t>(n_idle) && queue_open) {
+            const int n_want = n_idle / G;  // idle groups: rays to take
+            if (avail < static_cast<uint64_t>(n_want) && queue_open) {
                 const int leader = __ffs(idle) - 1;
                 unsigned long long b = 0;
                 if (lane == leader) b = atomicAdd(args.queue, static_cast<unsigned long long>(args.claim));
@@ -501,9 +722,9 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
                     if (b + args.claim >= args.total_rays) queue_open = false;
                 }
             }
-            const uint64_t used_old = (avail < static_cast<uint64_t>(n_idle)) ? avail : n_idle;
+            const uint64_t used_old = (avail < static_cast<uint64_t>(n_want)) ? avail : n_want;
             if (mode == MS_IDLE) {
-                const uint64_t rank = static_cast<uint64_t>(__popc(idle & lt_mask));
+                const uint64_t rank = static_cast<uint64_t>(__popc(idle & lt_mask) / G);
                 uint64_t rid = ~0ull;
                 if (rank < avail) rid = chunk_next + rank;
                 else if (got2) rid = base2 + (rank - avail);
@@ -519,7 +740,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
                     S.local[tid] = rid - Bp->ray_begin;
                     ms_init_ray(Bp, src, S.local[tid], y);
                     int ins;
-                    cap_len = ms_rhs(src, Bp->src_count, y, k1, Bp->capture_scale, ins);
+                    cap_len = ms_rhs<G, 1, false>(src, Bp->src_count, y, k1, Bp->capture_scale, ins, grp);
                     inside = ins;
                     h = -Bp->h0;
                     lnp = 0.0f;
@@ -530,11 +751,11 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
                     S.phi[tid] = Bp->phi0;
                     n_cross = bodies = 0;
                     mode = MS_STEP;
-                    ++n_rays;
+                    if (leader) ++n_rays;
                 }
             }
             if (got2) {
-                chunk_next = base2 + (static_cast<uint64_t>(n_idle) - used_old);
+                chunk_next = base2 + (static_cast<uint64_t>(n_want) - used_old);
                 chunk_end = base2 + args.claim;
                 if (chunk_end > args.total_rays) chunk_end = args.total_rays;
             } else {
@@ -553,10 +774,12 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
         // the end of a ray: its record (with the continuation only when it crossed
         // no disk: the record describes the first hit) and its continuation end
         auto end_ray = [&](const double* yend, uint32_t status, uint32_t fl, uint32_t body) {
-            if (!CONT || n_cross == 0)
+            if (leader && (!CONT || n_cross == 0))
                 ms_finish<BLOCK>(Bp, src, S, tid, yend, status, fl, acc, rej, NAN, 1.0, body, args.out);
-            if constexpr (CONT)
-                ms_cont_finish(args.cont, Bp->out_offset + S.local[tid], n_cross, bodies, status, src, ns, yend);
+            if constexpr (CONT) {
+                if (leader)
+                    ms_cont_finish(args.cont, Bp->out_offset + S.local[tid], n_cross, bodies, status, src, ns, yend);
+            }
             mode = MS_IDLE;
         };
         // backstop on loop iterations per ray (one attempt per iteration)
@@ -592,7 +815,23 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
         const double hh = h;
         double y5[6], k7[6], est[6], cap5;
         int inside5;
-        ms_stages<BLOCK>(src, ns, y, k1, hh, S, tid, Bp->capture_scale, y5, k7, est, cap5, inside5);
+        ms_stages<BLOCK, G, U, true>(src, ns, y, k1, hh, S, tid, Bp->capture_scale, y5, k7, est, cap5, inside5, grp);
+        if (est[2] != est[2]) {  // a stage left the fast forms' range (or the state is NaN)
+            double io[31];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                io[i] = y[i];
+                io[6 + i] = k1[i];
+            }
+            inside5 = ms_stages_special<BLOCK, G>(src, ns, io, hh, S, tid, Bp->capture_scale, grp);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                y5[i] = io[12 + i];
+                k7[i] = io[18 + i];
+                est[i] = io[24 + i];
+            }
+            cap5 = io[30];
+        }
         double err;
         {
             double num = 0.0, den = 1.0;
@@ -607,7 +846,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
             err = num / den;
         }
         if (!(err <= 1e300)) err = 1e300;
-        ++n_att;
+        if (leader) ++n_att;
         if (err > 1.0) {
             ++rej;
             const float le = __log2f(fmaxf(static_cast<float>(err), 1e-12f));
@@ -618,7 +857,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
             continue;
         }
         ++acc;
-        ++n_acc;
+        if (leader) ++n_acc;
         bool finite = true;
 #pragma unroll
         for (int i = 0; i < 6; ++i) finite = finite && isfinite(y5[i]);
@@ -683,7 +922,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
                     double ph = ph0;
                     ms_unwrap(ph, yr);
                     S.phi[tid] = ph;
-                    ms_finish<BLOCK>(Bp, src, S, tid, yr, RT_RAY_DISK, flags, acc, rej, best_r, g, best_i, args.out);
+                    if (leader) ms_finish<BLOCK>(Bp, src, S, tid, yr, RT_RAY_DISK, flags, acc, rej, best_r, g, best_i, args.out);
                 }
                 if constexpr (!CONT) {
                     mode = MS_IDLE;
@@ -693,13 +932,15 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
                     // the crossing recorded; the ray goes on through the disk
                     S.lambda[tid] = lam;
                     S.phi[tid] = ph0;
-                    ms_cont_record(args.cont, Bp->out_offset + S.local[tid], n_cross, best_r, best_az, g);
+                    if (leader)
+                        ms_cont_record(args.cont, Bp->out_offset + S.local[tid], n_cross, best_r, best_az, g);
                     bodies |= best_i << (4u * n_cross);
                     ++n_cross;
                     t_prev = best;
                     if (n_cross >= kMaxCrossings) {
-                        ms_cont_finish(args.cont, Bp->out_offset + S.local[tid], n_cross, bodies, RT_RAY_UNFINISHED,
-                                       src, ns, yr);
+                        if (leader)
+                            ms_cont_finish(args.cont, Bp->out_offset + S.local[tid], n_cross, bodies,
+                                           RT_RAY_UNFINISHED, src, ns, yr);
                         mode = MS_IDLE;
                         ended = true;
                         break;
@@ -727,7 +968,11 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
             end_ray(yt, RT_RAY_ESCAPED, flags, RT_BODY_NONE);
             continue;
         }
-        S.dH[tid] = fmax(S.dH[tid], ms_project(src, ns, y5, Bp->proj_tol));
+        {
+            double drift = ms_project<G, true>(src, ns, y5, Bp->proj_tol, grp);
+            if (drift != drift) drift = ms_project_special<G>(src, ns, y5, Bp->proj_tol, grp);
+            S.dH[tid] = fmax(S.dH[tid], drift);
+        }
         {
             double ph = S.phi[tid];
             ms_unwrap(ph, y5);
@@ -765,25 +1010,48 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) ms_trace_kernel(MsArgs arg
     }
 }
 
-template __global__ void ms_trace_kernel<128, false>(MsArgs);
-template __global__ void ms_trace_kernel<128, true>(MsArgs);
+template __global__ void ms_trace_kernel<128, false, 1, 2>(MsArgs);
+template __global__ void ms_trace_kernel<128, true, 1, 2>(MsArgs);
+template __global__ void ms_trace_kernel<128, false, 4, 1>(MsArgs);
+template __global__ void ms_trace_kernel<128, true, 4, 1>(MsArgs);
+template __global__ void ms_trace_kernel<128, false, 8, 1>(MsArgs);
+template __global__ void ms_trace_kernel<128, true, 8, 1>(MsArgs);
 
-}  // namespace
-
-uint32_t ms_trace_grid(int sm_count) {
+template <int G, int U>
+void launch_group(MsArgs args, int sm_count, cudaStream_t s) {
+    args.claim = args.claim / G > 0 ? args.claim / G : 1u;  // a warp holds 32 / G rays
+    auto* kernel = args.cont.cross ? ms_trace_kernel<128, true, G, U> : ms_trace_kernel<128, false, G, U>;
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ms_trace_kernel<128, false>, 128, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 128, 0) != cudaSuccess) {
         cudaGetLastError();
         occ = 1;
     }
-    return static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(occ > 1 ? occ : 1);
+    kernel<<<static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(occ > 1 ? occ : 1), 128, 0, s>>>(args);
 }
 
-void launch_ms_trace(const MsArgs& args, uint32_t grid, void* stream) {
-    if (args.cont.cross)
-        ms_trace_kernel<128, true><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(args);
-    else
-        ms_trace_kernel<128, false><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(args);
+// Lanes a ray: one, or with few rays (the launch then lasts as long as its longest
+// ray's chain of attempts, each a chain of source terms) four or eight.  The lanes of
+// a group repeat everything but the source terms, so this pays only while a ray has
+// several sources and the groups about fit on the device at once.  FP64 at 1 / 4 / 8
+// lanes (ms), 5 holes: 64x64 11.4 / 9.4 / 6.8, 160x120 12.7 / 10.8 / 12.4, 200x150
+// 13.5 / 13.7 / 17.2; 16 holes: 64x64 39.0 / 19.0 / 14.3, 160x120 41.8 / 29.9 / 33.1,
+// 200x150 42.2 / 39.9 / 47.6, 240x180 47.6 / 52.4 / 64.5; 2 holes: 160x120 6.8 / 7.2.
+int group_lanes(uint64_t rays, uint32_t sources, int sm_count) {
+    const uint64_t sm = static_cast<uint64_t>(sm_count);
+    if (sources >= 5 && rays <= 32 * sm) return 8;
+    if (sources >= 8 ? rays <= 192 * sm : (sources >= 3 && rays <= 160 * sm)) return 4;
+    return 1;
+}
+
+}  // namespace
+
+void launch_ms_trace(const MsArgs& args, int sm_count, void* stream) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    switch (group_lanes(args.total_rays, args.sources_per_ray, sm_count)) {
+        case 8: launch_group<8, 1>(args, sm_count, s); break;
+        case 4: launch_group<4, 1>(args, sm_count, s); break;
+        default: launch_group<1, 2>(args, sm_count, s); break;
+    }
 }
 
 }  // namespace relsim

@@ -409,7 +409,11 @@ bool launch_epoch(rt_server* s, Slot& slot) {
         const int ms_sms = (s->cfg.multi_source_sms > 0 && s->cfg.multi_source_sms < static_cast<uint32_t>(s->sm_count))
                                ? static_cast<int>(s->cfg.multi_source_sms)
                                : s->sm_count;
-        launch_ms_trace(ma, ms_trace_grid(ms_sms), st);
+        uint64_t ray_sources = 0;
+        for (uint32_t b = 0; b < nb; ++b)
+            ray_sources += static_cast<uint64_t>(slot.host_ms[b].nrows) * slot.host_ms[b].ncols * slot.host_ms[b].src_count;
+        ma.sources_per_ray = static_cast<uint32_t>(ray_sources / total);
+        launch_ms_trace(ma, ms_sms, st);
         e = cudaGetLastError();
     } else if (bl) {
         BlArgs ba{};

@@ -286,3 +286,30 @@ def test_multi_source_with_the_torus_model_drops_the_primary_disk(tracer):
     print(f"torus model, multi-source: {int(crossed.sum())} rays cross a body's disk; sRGB within 1e-5 "
           f"{np.mean(d < 1e-5):.4f}, max {d.max():.2e}")
     assert np.mean(d < 1e-5) >= 0.99
+
+
+@pytest.mark.parametrize("holes", [2, 3, 5, 8, 13, 16])
+def test_lanes_per_ray_do_not_change_a_ray(tracer, holes):
+    """A scene traced as a whole (one lane a ray) against its first rows alone, in windows small
+    enough for four and for eight lanes a ray: classes, steps, drift and disk hits bit for bit,
+    the ends of escaped rays within 1e-12."""
+    import torch
+
+    tracer.set_launch_config()
+    reqs = [r for r in scenes.request_stream() if len(r.sources) + 1 == holes]
+    srcs = scenes.rt_sources(reqs[0].sources)
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    width = 149  # groups that straddle rows, ragged last claims
+    rows = {8: 30 * sm // width, 4: 150 * sm // width, 1: 200 * sm // width}
+    base = dict(spin=0.6, r_obs=60.0, incl_deg=70.0, fov_deg=30.0, width=width, height=400, rtol=1e-8)
+    fields = ["status", "flags", "steps_accepted", "steps_rejected", "body", "r_hit", "g", "dH", "r", "theta", "phi"]
+    got = {}
+    for lanes, n_rows in rows.items():
+        cam = relsim.make_camera(**base, row_offset=100, row_count=n_rows)
+        got[lanes] = tracer.dispatch_multi(cam, srcs, fields=fields, pixels=False)
+    n = rows[8] * width
+    for lanes in (8, 4):
+        for f in fields[:8]:
+            np.testing.assert_array_equal(got[lanes][f][:n], got[1][f][:n], err_msg=f"{lanes} lanes, {f}")
+        for f in fields[8:]:
+            np.testing.assert_allclose(got[lanes][f][:n], got[1][f][:n], rtol=1e-12, err_msg=f"{lanes} lanes, {f}")
