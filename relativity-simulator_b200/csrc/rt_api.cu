@@ -1347,7 +1347,7 @@ rt_status noalloc_setup(int dev, NoAllocDevice& out, char* err, size_t len) {
         for (uint32_t block : {64u, 128u, 256u})
             for (bool mixed : {false, true})
                 for (bool rolled : {false, true}) trace_occupancy(kernel_block(block, mixed, rolled), mixed, rolled);
-        trace_wide_occupancy();
+        preload_trace_shapes();
         if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_cuda_fail(err, len, e, "kernel set-up");
         d.scratch = static_cast<unsigned char*>(p);
         d.sm_count = sms;

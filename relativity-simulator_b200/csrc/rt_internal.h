@@ -287,10 +287,7 @@ void row_window(const rt_camera& c, uint32_t& row0, uint32_t& nrows);
 
 // Tracer launch helpers implemented in rt_trace.cu.
 void launch_trace(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, uint32_t block, bool mixed, bool rolled,
-                  void* stream);
-// One pass of the two-pass mixed tracer (PASS_FAR or PASS_NEAR).
-void launch_trace_pass(const TraceArgs& args, int pass, uint32_t grid, uint32_t block, void* stream);
-int trace_pass_occupancy(int pass, uint32_t block);
+                  void* stream, bool lean = false);
 
 // Device buffers of the two-pass mixed tracer for n rays.
 struct TwoPassBuffers {
@@ -325,7 +322,7 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
                      void* stream, void* stream2, void* fork, void* join, uint32_t bands,
                      BandHook after_band = nullptr, void* hook_ctx = nullptr);
 int trace_occupancy(uint32_t block, bool mixed, bool rolled);
-int trace_wide_occupancy();  // of the plain FP64 tracer's 16-warp form
+void preload_trace_shapes();
 uint32_t kernel_block(uint32_t block, bool mixed, bool rolled);
 // Launch shape with defaults filled in and limits applied for one precision.
 rt_launch_config resolve_launch_config(rt_launch_config c, bool mixed);

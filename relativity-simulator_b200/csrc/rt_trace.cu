@@ -184,8 +184,16 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 
 }  // namespace
 
-// Resident warps per SM set the registers per thread: 12 warps at 168 registers, or
-// with WIDE 16 at 128.
+// WARPS resident warps per SM set the registers per thread: 8 warps at up to 255
+// registers, 12 at 168, 16 at 128.  Fewer warps spill less and an attempt takes less
+// time; more warps hide more of the FP64 latency that bounds the step loop.
+//
+//   12: the general case; it spills a little.
+//   16: the plain FP64 tracer over many rays (kWideRaysPerSm).  In the far, near and
+//       critical passes it loses (1279x717: 4.53 / 4.71, 0.89 / 1.19 and 1.73 / 2.01
+//       ms at 12 / 16): their warps run few rays or few lanes.
+//    8: launches of few rays, which last as long as their longest ray
+//       (kLeanRaysPerSm, kLeanMixedRaysPerSm).
 //
 // PASS selects the single-kernel tracer or one pass of the two-pass mixed
 // tracer.  The far pass (FP32 stages only) parks a ray when it enters the FP64
@@ -193,15 +201,8 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 // again.  Both passes solve disk crossings on the step's dense output.  Parked
 // rays resume from their saved state, so a ray's arithmetic does not depend on
 // which rays share its warp.
-// Twelve warps: the pass kernels spill a little there, which measured faster than 8
-// warps without spills.  Sixteen serve the plain FP64 tracer over many rays: FP64
-// latency is what bounds it, and a third more warps hide more of it than the
-// spills cost (2048^2 34.0 / 31.9 ms; the FP64 pipe is busy 65 % of the time).
-// The far, near and critical passes lose by it (1279x717: 4.53 / 4.71, 0.89 / 1.19
-// and 1.73 / 2.01 ms): their warps run few rays or few lanes, and there a longer
-// attempt is a longer tail.
-template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, bool WIDE = false>
-__global__ void __launch_bounds__(BLOCK, (WIDE ? 512 : 384) / BLOCK) trace_kernel_t(TraceArgs args) {
+template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, int WARPS = 12>
+__global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(TraceArgs args) {
     __shared__ Cold<BLOCK> S;
     __shared__ KStore<ROLLED ? BLOCK : 1> K;
     const unsigned FULL = 0xffffffffu;
@@ -866,7 +867,13 @@ __global__ void __launch_bounds__(BLOCK, (WIDE ? 512 : 384) / BLOCK) trace_kerne
 template __global__ void trace_kernel_t<64, false, false>(TraceArgs);
 template __global__ void trace_kernel_t<128, false, false>(TraceArgs);
 template __global__ void trace_kernel_t<256, false, false>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, true>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 1, 8>(TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 0, 8>(TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1, 8>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 0, 8>(TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1, 8>(TraceArgs);
 template __global__ void trace_kernel_t<64, false, true>(TraceArgs);
 template __global__ void trace_kernel_t<128, false, true>(TraceArgs);
 template __global__ void trace_kernel_t<64, true, true>(TraceArgs);
@@ -914,24 +921,34 @@ const void* kernel_for(uint32_t block, bool mixed, bool rolled, int cont = 0) {
     return (cont == 1) ? kernel_for_t<1>(block, mixed, rolled) : kernel_for_t<0>(block, mixed, rolled);
 }
 
-// The plain FP64 tracer with 16 warps per SM.
-const void* wide_kernel() { return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, true>); }
+// The plain FP64 tracer with 16 warps per SM, and with 8.
+const void* wide_kernel() { return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16>); }
+const void* lean_kernel(bool cont) {
+    return cont ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 1, 8>)
+                : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8>);
+}
 
-// Rays per SM from which the plain FP64 tracer takes it.  More warps raise the rate
-// and lengthen one attempt, so the longest rays' tail has to be a small part of the
-// launch.  12 / 16 warps, three cameras (face-on, grazing, wide view): 1448^2
+// Rays per SM from which the plain FP64 tracer takes 16 warps.  More warps raise the
+// rate and lengthen one attempt, so the longest rays' tail has to be a small part of
+// the launch.  12 / 16 warps, three cameras (face-on, grazing, wide view): 1448^2
 // 17.2 / 16.2, 22.3 / 23.3, 12.9 / 12.4 ms; 1740^2 24.7 / 23.2, 32.8 / 34.3,
 // 18.4 / 17.5; 2048^2 34.0 / 31.9, 43.4 / 42.0, 25.3 / 24.0.  The line is at 3.6 M rays.
 constexpr uint64_t kWideRaysPerSm = 24576;
+// Rays per SM up to which it takes 8: the rays that 12 warps hold at once.  12 / 8
+// warps, the same cameras: 96^2 0.76 / 0.67, 1.43 / 1.36, 1.26 / 1.23 ms; 224^2 0.92 /
+// 0.74, 1.75 / 1.54, 1.87 / 1.69; past the line 288^2 0.97 / 1.04, 1.89 / 1.70, 1.98 / 1.93.
+constexpr uint64_t kLeanRaysPerSm = 384;
+// The same for the passes of the mixed tracer, in rays of the whole launch (each pass
+// runs a part of them): 213x119 1.00 / 0.81, 1.73 / 1.51, 2.29 / 1.99 ms; 512x288 1.39 /
+// 1.33, 2.50 / 2.25, 2.56 / 2.42; past the line 768x432 2.02 / 2.05, 3.17 / 3.30, 3.36 / 3.11.
+constexpr uint64_t kLeanMixedRaysPerSm = 1024;
 }  // namespace
 
-int trace_wide_occupancy() {
+// Loads the kernels that launch_trace may pick beside those of trace_occupancy.
+void preload_trace_shapes() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wide_kernel(), 128, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
+    for (const void* k : {wide_kernel(), lean_kernel(false)})
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, 0) != cudaSuccess) cudaGetLastError();
 }
 
 uint32_t kernel_block(uint32_t block, bool mixed, bool rolled) {
@@ -985,23 +1002,24 @@ template __global__ void finish_kernel_t<128>(TraceArgs);
 
 namespace {
 template <bool CONT>
-const void* pass_kernel_t(int pass, uint32_t block) {
-    if (pass == PASS_FAR)
-        return (block == 64) ? reinterpret_cast<const void*>(&trace_kernel_t<64, true, false, PASS_FAR, CONT>)
-                             : reinterpret_cast<const void*>(&trace_kernel_t<128, true, false, PASS_FAR, CONT>);
-    return (block == 64) ? reinterpret_cast<const void*>(&trace_kernel_t<64, false, false, PASS_NEAR, CONT>)
-                         : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_NEAR, CONT>);
+const void* pass_kernel_t(int pass, uint32_t block, bool lean) {
+    if (pass == PASS_FAR) {
+        if (block == 64) return reinterpret_cast<const void*>(&trace_kernel_t<64, true, false, PASS_FAR, CONT>);
+        return lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, true, false, PASS_FAR, CONT, 8>)
+                    : reinterpret_cast<const void*>(&trace_kernel_t<128, true, false, PASS_FAR, CONT>);
+    }
+    if (block == 64) return reinterpret_cast<const void*>(&trace_kernel_t<64, false, false, PASS_NEAR, CONT>);
+    return lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_NEAR, CONT, 8>)
+                : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_NEAR, CONT>);
 }
 
-const void* pass_kernel(int pass, uint32_t block, bool cont = false) {
-    return cont ? pass_kernel_t<true>(pass, block) : pass_kernel_t<false>(pass, block);
+const void* pass_kernel(int pass, uint32_t block, bool lean, bool cont = false) {
+    return cont ? pass_kernel_t<true>(pass, block, lean) : pass_kernel_t<false>(pass, block, lean);
 }
-}  // namespace
 
-int trace_pass_occupancy(int pass, uint32_t block) {
+int trace_pass_occupancy(int pass, uint32_t block, bool lean) {
     int n = 0;
-    block = (block == 64) ? 64u : 128u;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pass_kernel(pass, block), static_cast<int>(block), 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pass_kernel(pass, block, lean), static_cast<int>(block), 0) !=
         cudaSuccess) {
         cudaGetLastError();
         return 1;
@@ -1009,12 +1027,13 @@ int trace_pass_occupancy(int pass, uint32_t block) {
     return n;
 }
 
-void launch_trace_pass(const TraceArgs& args, int pass, uint32_t grid, uint32_t block, void* stream) {
+// One pass of the two-pass mixed tracer (PASS_FAR or PASS_NEAR).
+void launch_trace_pass(const TraceArgs& args, int pass, uint32_t grid, uint32_t block, bool lean, cudaStream_t stream) {
     void* params[] = {const_cast<TraceArgs*>(&args)};
-    block = (block == 64) ? 64u : 128u;
-    cudaLaunchKernel(pass_kernel(pass, block, args.cont.cross != nullptr), dim3(grid), dim3(block), params, 0,
-                     static_cast<cudaStream_t>(stream));
+    cudaLaunchKernel(pass_kernel(pass, block, lean, args.cont.cross != nullptr), dim3(grid), dim3(block), params, 0,
+                     stream);
 }
+}  // namespace
 
 // Rounds of the two-pass mixed tracer: far pass (FP32) then near pass (FP64),
 // the last near pass keeping every ray to its end.  A ray typically needs one
@@ -1040,7 +1059,7 @@ uint64_t two_pass_state_bytes(uint64_t n) {
 namespace {
 cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t begin, uint64_t count, char* qb,
                          uint32_t far_grid, uint32_t far_block, uint32_t near_grid, uint32_t finish_grid,
-                         int sm_count, uint32_t crit_ctas, bool crit_beside, cudaStream_t s) {
+                         int sm_count, uint32_t crit_ctas, bool crit_beside, bool lean, cudaStream_t s) {
     uint32_t* near_q = buf.queues + 4 * begin;
     uint32_t* far_q = near_q + count;
     uint32_t* crit_q = far_q + 2 * count;
@@ -1064,7 +1083,7 @@ cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t beg
         args.out_count = reinterpret_cast<uint32_t*>(qb + 8);
         args.crit_queue = (round == 0) ? crit_q : nullptr;
         args.crit_count = (round == 0) ? reinterpret_cast<uint32_t*>(qb + 32) : nullptr;
-        launch_trace_pass(args, PASS_FAR, far_grid, far_block, s);
+        launch_trace_pass(args, PASS_FAR, far_grid, far_block, lean, s);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if (round == 0) {
             // critical pass: the near-critical rays, FP64 from their pixels to their
@@ -1084,7 +1103,7 @@ cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t beg
                 if ((e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_fork), s)) != cudaSuccess) break;
                 if ((e = cudaStreamWaitEvent(cs, static_cast<cudaEvent_t>(buf.crit_fork), 0)) != cudaSuccess) break;
             }
-            launch_trace(c, sm_count, crit_ctas, kCriticalBlock, false, false, cs);
+            launch_trace(c, sm_count, crit_ctas, kCriticalBlock, false, false, cs, lean);
             if ((e = cudaGetLastError()) != cudaSuccess) break;
             if (crit_beside && (e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_join), cs)) != cudaSuccess) break;
         }
@@ -1098,7 +1117,7 @@ cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t beg
         args.in_count = reinterpret_cast<const uint32_t*>(qb + 8);
         args.out_queue = far_q;
         args.out_count = reinterpret_cast<uint32_t*>(qb + 12);
-        launch_trace_pass(args, PASS_NEAR, near_grid, 128, s);
+        launch_trace_pass(args, PASS_NEAR, near_grid, 128, lean, s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
@@ -1122,8 +1141,9 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
     bands = bands < 1 ? 1 : (bands > kMaxBands ? kMaxBands : bands);
     if (static_cast<uint64_t>(bands) > n) bands = static_cast<uint32_t>(n > 0 ? n : 1);
     far_block = (far_block == 64) ? 64u : 128u;
-    const int far_occ = trace_pass_occupancy(PASS_FAR, far_block);
-    const int near_occ = trace_pass_occupancy(PASS_NEAR, 128);
+    const bool lean = far_block == 128u && n <= kLeanMixedRaysPerSm * static_cast<uint64_t>(sm_count);
+    const int far_occ = trace_pass_occupancy(PASS_FAR, far_block, lean);
+    const int near_occ = trace_pass_occupancy(PASS_NEAR, 128, lean);
     const uint32_t far_grid = static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(far_occ > 1 ? far_occ : 1);
     const uint32_t near_grid = static_cast<uint32_t>(sm_count) * static_cast<uint32_t>(near_occ > 1 ? near_occ : 1);
     const uint32_t finish_grid = static_cast<uint32_t>(sm_count) * 8u;
@@ -1144,7 +1164,7 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
         cudaStream_t sb = (b & 1u) ? s2 : s;
         const bool crit_beside = bands == 1 && buf.crit_stream && buf.crit_fork && buf.crit_join;
         e = enqueue_band(base, buf, begin, count, buf.counters + kBandCounterBytes * b, far_grid, far_block, near_grid,
-                         finish_grid, sm_count, crit_ctas, crit_beside, sb);
+                         finish_grid, sm_count, crit_ctas, crit_beside, lean, sb);
         if (e == cudaSuccess && after_band && prev_stream)
             e = static_cast<cudaError_t>(after_band(hook_ctx, prev_begin, prev_count, prev_stream));
         prev_begin = begin;
@@ -1163,17 +1183,23 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
 }
 
 void launch_trace(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, uint32_t block, bool mixed, bool rolled,
-                  void* stream) {
+                  void* stream, bool lean) {
     void* params[] = {const_cast<TraceArgs*>(&args)};
     // hydro model 2: the FP64 straight-line tracer in 128-thread blocks
     const int cont = args.cont.vol ? 2 : (args.cont.cross ? 1 : 0);
     block = (cont == 2) ? 128u : kernel_block(block, mixed, rolled);
     const void* kernel = kernel_for(block, mixed, rolled, cont);
-    // only where the caller left the CTAs per SM at the occupancy maximum
-    if (!mixed && !rolled && cont == 0 && !args.in_queue && block == 128u && ctas_per_sm >= 3u &&
-        args.total_rays >= kWideRaysPerSm * static_cast<uint64_t>(sm_count)) {
-        kernel = wide_kernel();
-        ctas_per_sm = 4;
+    // 8 or 16 warps per SM only where the caller left the CTAs per SM at the occupancy
+    // maximum; the critical pass's rays are counted on the device, so its caller decides
+    if (!mixed && !rolled && cont != 2 && block == 128u && ctas_per_sm >= 3u) {
+        const uint64_t sm = static_cast<uint64_t>(sm_count);
+        if (lean || (!args.in_queue && args.total_rays <= kLeanRaysPerSm * sm)) {
+            kernel = lean_kernel(cont == 1);
+            ctas_per_sm = 2;
+        } else if (cont == 0 && !args.in_queue && args.total_rays >= kWideRaysPerSm * sm) {
+            kernel = wide_kernel();
+            ctas_per_sm = 4;
+        }
     }
     cudaLaunchKernel(kernel, dim3(static_cast<uint32_t>(sm_count) * ctas_per_sm), dim3(block), params, 0,
                      static_cast<cudaStream_t>(stream));

@@ -276,3 +276,26 @@ def test_sixteen_warp_tracer_gives_the_same_record(tracer, past):
         tracer.synchronize()
         for f in fields:
             assert torch.equal(part[f].view(torch.uint8), whole[f][r0 * width:(r0 + step) * width].view(torch.uint8)), f
+
+
+@pytest.mark.parametrize("precision,rays_per_sm", [(relsim.PRECISION_FP64, 384), (relsim.PRECISION_MIXED, 1024)])
+@pytest.mark.parametrize("past", [0, 1])
+def test_eight_warp_tracer_gives_the_same_record(tracer, precision, rays_per_sm, past):
+    """Up to 384 rays per SM (mixed: 1024) a launch takes the kernels' 8-warp forms, one row more
+    the 12-warp forms; both equal the same rows of an image past the line, bit for bit."""
+    import torch
+
+    tracer.set_launch_config()
+    width = rays_per_sm
+    rows = torch.cuda.get_device_properties(0).multi_processor_count
+    fields = ["status", "flags", "steps_accepted", "steps_rejected", "r", "theta", "phi", "r_hit", "g", "lambda"]
+    base = dict(width=width, height=3 * rows, incl_deg=65.0, r_obs=30.0, fov_deg=40.0, precision=precision)
+    ro, whole = relsim.device_ray_out(width * 3 * rows, fields)
+    tracer.dispatch_device(relsim.make_camera(**base), ro, None, width * 3 * rows)
+    tracer.synchronize()
+    n = width * (rows + past)
+    ro, part = relsim.device_ray_out(n, fields)
+    tracer.dispatch_device(relsim.make_camera(**base, row_offset=rows, row_count=rows + past), ro, None, n)
+    tracer.synchronize()
+    for f in fields:
+        assert torch.equal(part[f].view(torch.uint8), whole[f][rows * width:rows * width + n].view(torch.uint8)), f
