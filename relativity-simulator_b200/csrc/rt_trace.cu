@@ -219,6 +219,10 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
         (PASS == PASS_SINGLE) ? (args.in_queue != nullptr) : !(FAR_PASS && args.from_pixels != 0);
     const uint64_t total = from_queue ? static_cast<uint64_t>(*args.in_count) : args.total_rays;
 
+    // the rounds after a ray's last pass find their queues empty (5 of the 9 launches of
+    // an ordinary image): out at once, before the claims and counters (13 / 5 us each)
+    if (from_queue && total == 0) return;
+
     // hot lane state
     double y[6], k1[6];
     double r = 0.0, h = 0.0;
@@ -852,12 +856,12 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
         w_rhs += __shfl_down_sync(FULL, w_rhs, off);
         w_far += __shfl_down_sync(FULL, w_far, off);
     }
-    if (lane == 0) {
-        atomicAdd(args.stats + ST_RAYS, w_rays);
+    if (lane == 0 && w_rhs != 0) {
+        if (w_rays) atomicAdd(args.stats + ST_RAYS, w_rays);
         atomicAdd(args.stats + ST_ATTEMPTS, w_att);
         atomicAdd(args.stats + ST_ACCEPTED, w_acc);
         atomicAdd(args.stats + ST_RHS, w_rhs);
-        atomicAdd(args.stats + ST_FP64_ATTEMPTS, w_att - w_far);
+        if (w_att != w_far) atomicAdd(args.stats + ST_FP64_ATTEMPTS, w_att - w_far);
     }
 }
 
