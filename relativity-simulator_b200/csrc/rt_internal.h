@@ -132,6 +132,9 @@ struct ParkBuf {
 // near-zone pass; rays move between them through queues of launch indices.
 enum TracePass : int { PASS_SINGLE = 0, PASS_FAR = 1, PASS_NEAR = 2 };
 
+// Length classes of near-critical rays, in the upper bits of a queue entry.
+constexpr uint32_t kCritClasses = 32, kCritClassShift = 27;
+
 struct TraceArgs {
     const BundleDesc* bundles;
     uint32_t n_bundles;
@@ -154,6 +157,7 @@ struct TraceArgs {
     uint32_t* finish_count;
     uint32_t* crit_queue;       // first far pass: near-critical rays, for the critical pass
     uint32_t* crit_count;
+    uint64_t crit_classes;      // 1: crit_queue entries carry the ray's length class in their upper bits
     ParkBuf park;
     // translucent-disk continuation (single-camera launches with shading): the
     // crossings' outputs; cross null: off
@@ -300,7 +304,7 @@ struct TwoPassBuffers {
     void* crit_fork = nullptr;
     void* crit_join = nullptr;
 };
-constexpr uint32_t kBandCounterBytes = 64;
+constexpr uint32_t kBandCounterBytes = 320;
 constexpr uint32_t kMaxBands = 8;
 // Bytes of park.d, park.u and queues for n rays.
 uint64_t two_pass_state_bytes(uint64_t n);

@@ -395,6 +395,15 @@ __device__ __forceinline__ float critical_tol_scale(double db, double band) {
     return static_cast<float>(fmin(1.0, fmax(kCriticalTolScale, u * u)));
 }
 
+// Length class of a near-critical ray, the longest 0: half powers of two of |d_b| /
+// band, the closest to the curve first (its tolerance is the smallest and it orbits
+// the longest), and within one the rays that turn back before those that plunge.
+__device__ __forceinline__ uint32_t critical_class(double db, double band) {
+    const int k = static_cast<int>(-2.0f * __log2f(static_cast<float>(fabs(db) / band)));
+    const int near = static_cast<int>(kCritClasses / 2) - 1;
+    return 2u * static_cast<uint32_t>(near - (k < 0 ? 0 : (k > near ? near : k))) + (db > 0.0 ? 1u : 0u);
+}
+
 // Largest r_BL at which the FP32 stages are used (keeps r^4 and 1/r^4 in range).
 constexpr double kFp32MaxRadius = 1e6;
 

@@ -278,11 +278,12 @@ def test_sixteen_warp_tracer_gives_the_same_record(tracer, past):
             assert torch.equal(part[f].view(torch.uint8), whole[f][r0 * width:(r0 + step) * width].view(torch.uint8)), f
 
 
-@pytest.mark.parametrize("precision,rays_per_sm", [(relsim.PRECISION_FP64, 384), (relsim.PRECISION_MIXED, 1024)])
+@pytest.mark.parametrize("precision,rays_per_sm", [(relsim.PRECISION_FP64, 384), (relsim.PRECISION_MIXED, 1024), (relsim.PRECISION_MIXED, 768)])
 @pytest.mark.parametrize("past", [0, 1])
 def test_eight_warp_tracer_gives_the_same_record(tracer, precision, rays_per_sm, past):
     """Up to 384 rays per SM (mixed: 1024) a launch takes the kernels' 8-warp forms, one row more
-    the 12-warp forms; both equal the same rows of an image past the line, bit for bit."""
+    the 12-warp forms, and past 768 the near-critical rays are sorted; on each side of each line the
+    record equals the same rows of an image past all of them, bit for bit."""
     import torch
 
     tracer.set_launch_config()
