@@ -58,7 +58,7 @@ struct rt_handle {
     bool shade_on = false;               // rt_set_shading
     // translucent-disk continuation of a shaded dispatch: each ray's disk crossings
     // and how it ended, and what the launches pass the tracer
-    DevBuf cont_cross, cont_info, cont_body, cont_exit, cont_tail, cont_vol;
+    DevBuf cont_cross, cont_info, cont_body, cont_exit, cont_tail, cont_vol, cont_lz;
     DevBuf ms_shade;  // multi-source shading: one descriptor per source
     ContOut cur_cont{};
     rt_shading shading{};
@@ -300,22 +300,6 @@ struct BandCopyCtx;
 rt_status launch_banded_single(rt_handle* h, const rt_camera* cam, uint32_t col0, uint32_t ncols, uint32_t row0,
                                uint32_t nrows, uint64_t out_offset, const OutPtrs& out, BandCopyCtx& ctx);
 
-// The record fields the shading pass reads (status, phi, r_hit, g), taken from
-// the handle's scratch where the caller did not ask for them.
-rt_status add_shade_fields(rt_handle* h, rt_ray_out& dev, size_t n) {
-    void** dp = reinterpret_cast<void**>(&dev);
-    const int fields[4] = {0, 6, 7, 8};
-    const size_t elem[4] = {4, 8, 8, 8};
-    for (int k = 0; k < 4; ++k) {
-        const int f = fields[k];
-        if (dp[f]) continue;
-        const rt_status st = ensure(h, h->ray_fields[f], n * elem[k]);
-        if (st != RT_OK) return st;
-        dp[f] = h->ray_fields[f].ptr;
-    }
-    return RT_OK;
-}
-
 // The blackbody colour's table on the device: 57 KB, the same for every camera,
 // uploaded once and waited for, since later dispatches may use other streams.
 rt_status ensure_planck(rt_handle* h, cudaStream_t s) {
@@ -370,13 +354,15 @@ rt_status begin_continuation(rt_handle* h, size_t n, bool bodies = false, bool k
     if (st == RT_OK && bodies) st = ensure(h, h->cont_body, sizeof(uint32_t) * n);
     if (st == RT_OK && exit) st = ensure(h, h->cont_exit, sizeof(double) * 3 * n);
     if (st == RT_OK && tail) st = ensure(h, h->cont_tail, sizeof(double) * TL_COUNT * n);
+    if (st == RT_OK && kerr_schild) st = ensure(h, h->cont_lz, sizeof(double) * n);
     if (st != RT_OK) return st;
     h->cur_cont = ContOut{static_cast<double*>(h->cont_cross.ptr), static_cast<uint32_t*>(h->cont_info.ptr), n,
                           bodies ? static_cast<uint32_t*>(h->cont_body.ptr) : nullptr,
                           exit ? static_cast<double*>(h->cont_exit.ptr) : nullptr,
                           tail ? static_cast<double*>(h->cont_tail.ptr) : nullptr,
                           volume ? static_cast<double*>(h->cont_vol.ptr) : nullptr,
-                          volume ? static_cast<const ShadeDesc*>(h->shade_desc.ptr) : nullptr};
+                          volume ? static_cast<const ShadeDesc*>(h->shade_desc.ptr) : nullptr,
+                          kerr_schild ? static_cast<double*>(h->cont_lz.ptr) : nullptr};
     return RT_OK;
 }
 
@@ -407,8 +393,8 @@ rt_status shade_launch(rt_handle* h, const rt_camera* cam, const rt_ray_out& dev
                        cudaStream_t s, bool prepared = false) {
     rt_status st;
     if (!prepared && (st = shade_prepare(h, cam, s)) != RT_OK) return st;
-    launch_shade(static_cast<const ShadeDesc*>(h->shade_desc.ptr), dev.status, dev.r_hit, dev.phi, dev.g, h->cur_cont,
-                 pixels, n, s);
+    launch_shade(static_cast<const ShadeDesc*>(h->shade_desc.ptr), nullptr, nullptr, nullptr, nullptr, h->cur_cont, pixels,
+                 n, s);
     RT_CUDA(h, cudaGetLastError());
     return RT_OK;
 }
@@ -434,14 +420,11 @@ int band_copy_hook(void* vctx, uint64_t begin, uint64_t count, void* stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const uint64_t o = c.offset + begin;
     if (c.shade && c.dpix) {
-        launch_shade(static_cast<const ShadeDesc*>(c.h->shade_desc.ptr), c.dev.status + o, c.dev.r_hit + o,
-                     c.dev.phi + o, c.dev.g + o,
-                     c.cont.cross ? ContOut{c.cont.cross + o, c.cont.info + o, c.cont.stride,
-                                            c.cont.body ? c.cont.body + o : nullptr,
-                                            c.cont.exit ? c.cont.exit + o : nullptr,
-                                            c.cont.tail ? c.cont.tail + o * TL_COUNT : nullptr,
-                                            c.cont.vol ? c.cont.vol + o * VL_COUNT : nullptr, c.cont.shade}
-                                  : ContOut{},
+        launch_shade(static_cast<const ShadeDesc*>(c.h->shade_desc.ptr), nullptr, nullptr, nullptr, nullptr,
+                     ContOut{c.cont.cross + o, c.cont.info + o, c.cont.stride, c.cont.body ? c.cont.body + o : nullptr,
+                             c.cont.exit ? c.cont.exit + o : nullptr, c.cont.tail ? c.cont.tail + o * TL_COUNT : nullptr,
+                             c.cont.vol ? c.cont.vol + o * VL_COUNT : nullptr, c.cont.shade,
+                             c.cont.lz ? c.cont.lz + o : nullptr},
                      c.dpix + o, count, s);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return static_cast<int>(e);
@@ -498,7 +481,6 @@ rt_status dispatch_window(rt_handle* h, const rt_camera* cam, uint32_t col0, uin
     }
     const bool shade = h->shade_on && pixels;
     ContinuationScope cont_scope{h};
-    if (shade && (st = add_shade_fields(h, dev, n)) != RT_OK) return st;
     if (shade && (st = shade_prepare(h, cam, h->stream)) != RT_OK) return st;
     if (shade && (st = begin_continuation(h, n, false, !is_bl(cam), h->stream)) != RT_OK) return st;
     // bands of at most 2^24 rays; the cancel flag is polled between bands.  Each
@@ -881,6 +863,7 @@ void rt_destroy(rt_handle* h) {
     release(h->cont_exit);
     release(h->cont_tail);
     release(h->cont_vol);
+    release(h->cont_lz);
     release(h->park_d);
     release(h->park_u);
     release(h->pass_queues);
@@ -1122,7 +1105,6 @@ rt_status rt_dispatch_device(rt_handle* h, const rt_camera* cam, rt_pixel_out* p
     const bool shade = h->shade_on && pixels;
     rt_status st;
     ContinuationScope cont_scope{h};
-    if (shade && (st = add_shade_fields(h, dev, n)) != RT_OK) return st;
     if (is_bl(cam)) {
         // shaded: the shading constants go up before the trace, which follows each
         // ray through the translucent disk

@@ -83,7 +83,8 @@ enum : uint32_t {
 };
 struct ShadeDesc;
 struct ContOut {
-    double* cross;    // [3 * kMaxCrossings][stride]: r_k at [3k], phi_k at [3k + 1], g_k at [3k + 2]
+    double* cross;    // [3 * kMaxCrossings][stride]: r_k at [3k], phi_k at [3k + 1], g_k at [3k + 2]; with lz,
+                      // the Kerr-Schild point x_k, y_k, z_k
     uint32_t* info;   // [stride]
     uint64_t stride;
     uint32_t* body;   // multi-source: [stride], source of crossing k in bits 4k..4k+3 (else null)
@@ -93,6 +94,7 @@ struct ContOut {
     double* vol;      // hydro model 2 (Kerr-Schild FP64 tracer): [stride][VL_COUNT], the light the
                       // ray gathered in the Fishbone-Moncrief torus (else null)
     const ShadeDesc* shade;  // with vol: the torus and the disk profile (device)
+    double* lz;       // Kerr-Schild tracers: [stride], L_z of a ray that crossed (else null)
 };
 // The torus's light along a ray, gathered by the tracer step by step (every
 // field 0 before the ray's first emitting segment): radiance r, g, b, the

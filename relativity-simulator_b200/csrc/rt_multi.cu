@@ -152,8 +152,8 @@ __device__ __forceinline__ void ms_terms(const MsSource* __restrict__ const* sp,
         const double C = __dmul_rn(__dmul_rn(__dmul_rn(M, r2), inv_den), __dmul_rn(c, inv_den));
         const double D = __dmul_rn(__dmul_rn(-2.0, H), __dmul_rn(__dmul_rn(a2, x[2]), inv_den));
         const double tr = __dmul_rn(2.0, r);
-        const double U = __fma_rn(-tr, k[0], x[0]), V = __fma_rn(-tr, k[1], x[1]);
-        const double W = __fma_rn(U, px, __dmul_rn(V, py));
+        const double w0 = __fma_rn(-tr, k[0], x[0]), w1 = __fma_rn(-tr, k[1], x[1]);
+        const double W = __fma_rn(w0, px, __dmul_rn(w1, py));
         const double A = __fma_rn(inv_rpa, W, -__dmul_rn(__dmul_rn(inv_r, k[2]), pz));
         const double B0 = __dmul_rn(inv_rpa, __fma_rn(r, px, -__dmul_rn(a, py)));
         const double B1 = __dmul_rn(inv_rpa, __fma_rn(a, px, __dmul_rn(r, py)));

@@ -170,39 +170,41 @@ __device__ __noinline__ void finish_ray(const BundleDesc* __restrict__ Bp, ColdT
 #pragma unroll
         for (int i = 0; i < 6; ++i) y[i] = xch[12 + i];
     }
-    const double r = sqrt(bl_r2<double>(y[0], y[1], y[2], a * a));
-    const double rho = sqrt(fmax(r * r - y[2] * y[2], 0.0));
-    const double theta = atan2(rho, y[2]);
-    wind += branch_winding(y_prev_x, y_prev_y, y[0], y[1]);
-    const double phi = atan2(y[1], y[0]) - atan2(a, r) + kTwoPi * static_cast<double>(wind);
-    // invariants at the end
-    double kf[3], hf;
-    ks_field64(y, B.m, a, kf, hf);
-    const double kp = kf[0] * y[3] + kf[1] * y[4] + kf[2] * y[5];
-    const double pp = y[3] * y[3] + y[4] * y[4] + y[5] * y[5];
-    const double qa = 1.0 + 2.0 * hf, qb = 2.0 * hf * kp, qc = pp - 2.0 * hf * kp * kp;
-    const double energy = (-qb + sqrt(fmax(qb * qb + qa * qc, 0.0))) / qa;
-    const double lz = y[0] * y[4] - y[1] * y[3];
-    const double q = carter_q(y, a);
-
     const uint64_t o = B.out_offset + S.local[tid];
     const rt_ray_out& R = out.rays;
     if (R.status) R.status[o] = status;
     if (R.flags) R.flags[o] = flags;
     if (R.steps_accepted) R.steps_accepted[o] = acc;
     if (R.steps_rejected) R.steps_rejected[o] = rej;
-    if (R.r) R.r[o] = r;
-    if (R.theta) R.theta[o] = theta;
-    if (R.phi) R.phi[o] = phi;
     if (R.r_hit) R.r_hit[o] = r_hit;
     if (R.g) R.g[o] = g;
     if (R.lambda) R.lambda[o] = lambda;
     if (R.dH) R.dH[o] = S.dH[tid];
-    if (R.dE) R.dE[o] = energy - 1.0;
-    if (R.dLz) R.dLz[o] = lz - S.lz0[tid];
-    if (R.dQ) R.dQ[o] = q - S.q0[tid];
+    // fields that take work are formed only for callers that asked for them
+    if (R.r || R.theta || R.phi) {
+        const double r = sqrt(bl_r2<double>(y[0], y[1], y[2], a * a));
+        if (R.r) R.r[o] = r;
+        if (R.theta) R.theta[o] = atan2(sqrt(fmax(__dsub_rn(__dmul_rn(r, r), __dmul_rn(y[2], y[2])), 0.0)), y[2]);
+        if (R.phi) {
+            wind += branch_winding(y_prev_x, y_prev_y, y[0], y[1]);
+            R.phi[o] = atan2(y[1], y[0]) - atan2(a, r) + kTwoPi * static_cast<double>(wind);
+        }
+    }
+    const bool want_exit = R.exit_x || R.exit_y || R.exit_z;
+    double kf[3] = {0.0, 0.0, 0.0}, hf = 0.0, kp = 0.0;
+    if (R.dE || want_exit) {
+        ks_field64(y, B.m, a, kf, hf);
+        kp = kf[0] * y[3] + kf[1] * y[4] + kf[2] * y[5];
+    }
+    if (R.dE) {  // -p_t from the null condition at the end
+        const double pp = y[3] * y[3] + y[4] * y[4] + y[5] * y[5];
+        const double qa = 1.0 + 2.0 * hf, qb = 2.0 * hf * kp, qc = pp - 2.0 * hf * kp * kp;
+        R.dE[o] = (-qb + sqrt(fmax(qb * qb + qa * qc, 0.0))) / qa - 1.0;
+    }
+    if (R.dLz) R.dLz[o] = y[0] * y[4] - y[1] * y[3] - S.lz0[tid];
+    if (R.dQ) R.dQ[o] = carter_q(y, a) - S.q0[tid];
     if (R.body) R.body[o] = (status == RT_RAY_DISK || status == RT_RAY_CAPTURED) ? 0u : RT_BODY_NONE;
-    if (R.exit_x || R.exit_y || R.exit_z) {
+    if (want_exit) {
         // sky-lookup direction of an escaped ray: -dx/dlambda at the terminal
         // state, normalised (software_compute_engine.hpp:1771-1775); each
         // component is written only where the caller asked for it
@@ -319,16 +321,16 @@ __device__ __noinline__ double dense_disk_root(const double* __restrict__ y0, co
     return t;
 }
 
-// Record crossing k of a Kerr-Schild ray at the root point yr (winding
-// wind_root along the ray) for the translucent-disk continuation: r_BL, the
-// unwrapped azimuth and g, as the first hit's record has them.
+// Record crossing k of a Kerr-Schild ray at the root point yr for the
+// translucent-disk continuation: the point, and once the ray's L_z.  The shading
+// pass, whose lanes all work on crossings, forms r, the azimuth and g from them;
+// here the other lanes of the warp would wait for two atan2 and the redshift's roots.
 template <class ColdT>
 __device__ __forceinline__ void record_crossing(const TraceArgs& args, const BundleDesc* __restrict__ Bp, ColdT& S,
-                                                int j, uint32_t k, const double* __restrict__ yr, int wind_root) {
-    const double a = Bp->a;
-    const double r = sqrt(bl_r2<double>(yr[0], yr[1], yr[2], a * a));
-    const double phi = atan2(yr[1], yr[0]) - atan2(a, r) + kTwoPi * static_cast<double>(wind_root);
-    cont_record(args.cont, Bp->out_offset + S.local[j], k, r, phi, disk_redshift(Bp->m, a, r, S.lz0[j]));
+                                                int j, uint32_t k, const double* __restrict__ yr) {
+    const uint64_t o = Bp->out_offset + S.local[j];
+    cont_record(args.cont, o, k, yr[0], yr[1], yr[2]);
+    if (k == 0) args.cont.lz[o] = S.lz0[j];
 }
 
 // End of a Kerr-Schild ray's trace with the continuation on.  xch as end_ray

@@ -129,9 +129,17 @@ __global__ void __launch_bounds__(512) shade_kernel(const ShadeDesc* __restrict_
             }
             for (uint32_t k = 0; k < n_cross && thr > kMinThroughput; ++k) {
                 double sh[4];
-                const double gk = cont.cross[(3 * k + 2) * cont.stride + i];
-                disk_radiance(Dp[(bodies >> (4u * k)) & 15u], cont.cross[(3 * k) * cont.stride + i],
-                              cont.cross[(3 * k + 1) * cont.stride + i], gk, sh);
+                double rk = cont.cross[(3 * k) * cont.stride + i], phik = cont.cross[(3 * k + 1) * cont.stride + i],
+                       gk = cont.cross[(3 * k + 2) * cont.stride + i];
+                if (cont.lz) {
+                    // a Kerr-Schild point: r_BL, the azimuth (the pattern is periodic in it)
+                    // and the redshift of the circular orbit there
+                    const double a = D.disk_spin, x = rk, y = phik;
+                    rk = sqrt(bl_r2<double>(x, y, gk, a * a));
+                    phik = atan2(y, x) - atan2(a, rk);
+                    gk = disk_redshift(D.mass, a, rk, cont.lz[i]);
+                }
+                disk_radiance(Dp[(bodies >> (4u * k)) & 15u], rk, phik, gk, sh);
                 acc[0] += thr * sh[0];
                 acc[1] += thr * sh[1];
                 acc[2] += thr * sh[2];

@@ -325,11 +325,11 @@ __device__ __noinline__ void fm_segment(const ShadeDesc& D, const double* from, 
 // where it is found would run it one lane at a time while the warp waits).
 constexpr double kMinThroughput = 0.01;
 
-__device__ __forceinline__ void cont_record(const ContOut& C, uint64_t o, uint32_t k, double r, double phi,
-                                            double g) {
-    C.cross[(3 * k) * C.stride + o] = r;
-    C.cross[(3 * k + 1) * C.stride + o] = phi;
-    C.cross[(3 * k + 2) * C.stride + o] = g;
+__device__ __forceinline__ void cont_record(const ContOut& C, uint64_t o, uint32_t k, double c0, double c1,
+                                            double c2) {
+    C.cross[(3 * k) * C.stride + o] = c0;
+    C.cross[(3 * k + 1) * C.stride + o] = c1;
+    C.cross[(3 * k + 2) * C.stride + o] = c2;
 }
 
 // End of a ray's trace: crossings recorded, its class at the end (UNFINISHED

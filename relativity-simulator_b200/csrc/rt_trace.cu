@@ -629,8 +629,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                         }
                         mode = MODE_IDLE;
                         // translucent disk: record the crossing and go on through it
-                        record_crossing(args, Bp, S, tid, n_cross, y5,
-                                        wind + branch_winding(y[0], y[1], y5[0], y5[1]));
+                        record_crossing(args, Bp, S, tid, n_cross, y5);
                         ++n_cross;
                         if (n_cross < kMaxCrossings) {
                             S.lambda[tid] = lambda_step;
@@ -740,7 +739,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                                            disk_redshift(M, a, rr, S.lz0[tid]), args.out, xr);
                                 S.lambda[tid] = lambda_step;
                             }
-                            record_crossing(args, Bp, S, tid, n_cross, xr + 12, wroot);
+                            record_crossing(args, Bp, S, tid, n_cross, xr + 12);
                             ++n_cross;
                             if (n_cross >= kMaxCrossings) {
                                 end_continuation(args, Bp, S, tid, n_cross, RT_RAY_UNFINISHED, xr + 12);
