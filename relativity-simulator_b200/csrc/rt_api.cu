@@ -198,6 +198,10 @@ rt_status launch_two_pass(rt_handle* h, uint32_t n_bundles, uint64_t total, cons
     TraceArgs args{};
     args.bundles = static_cast<const BundleDesc*>(h->bundles.ptr);
     args.n_bundles = n_bundles;
+    if (n_bundles == 1 && !capturing) {
+        args.one = h->host_bundles[0];
+        args.has_one = 1;
+    }
     args.refill_threshold = c.refill_threshold;
     args.claim = 32u * c.rays_per_thread;
     args.total_rays = total;
@@ -235,6 +239,10 @@ rt_status launch(rt_handle* h, uint32_t n_bundles, uint64_t total, const OutPtrs
     TraceArgs args{};
     args.bundles = static_cast<const BundleDesc*>(h->bundles.ptr);
     args.n_bundles = n_bundles;
+    if (n_bundles == 1 && !capturing) {
+        args.one = h->host_bundles[0];
+        args.has_one = 1;
+    }
     args.refill_threshold = c.refill_threshold;
     args.claim = 32u * c.rays_per_thread;
     args.total_rays = total;
@@ -664,6 +672,8 @@ rt_status launch_banded_single(rt_handle* h, const rt_camera* cam, uint32_t col0
             TraceArgs args{};
             args.bundles = reinterpret_cast<const BundleDesc*>(dd);
             args.n_bundles = 1;
+            args.one = d;
+            args.has_one = 1;
             args.refill_threshold = c.refill_threshold;
             args.claim = 32u * c.rays_per_thread;
             args.total_rays = count;

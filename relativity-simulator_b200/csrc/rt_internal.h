@@ -142,7 +142,7 @@ struct TraceArgs {
     uint32_t n_bundles;
     uint32_t refill_threshold;
     uint32_t claim;             // rays a warp claims per global atomic
-    uint32_t pad;
+    uint32_t has_one;           // one bundle, in `one` (not in captured launches: replays change the table)
     uint64_t total_rays;
     unsigned long long* queue;  // [0]: next unclaimed ray (or queue entry)
     unsigned long long* stats;  // [ST_COUNT]
@@ -160,6 +160,7 @@ struct TraceArgs {
     uint32_t* crit_queue;       // first far pass: near-critical rays, for the critical pass
     uint32_t* crit_count;
     uint64_t crit_classes;      // 1: crit_queue entries carry the ray's length class in their upper bits
+    BundleDesc one;             // has_one: the launch's only bundle, read in place of bundles[0]
     ParkBuf park;
     // translucent-disk continuation (single-camera launches with shading): the
     // crossings' outputs; cross null: off

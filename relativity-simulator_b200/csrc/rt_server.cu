@@ -385,6 +385,10 @@ bool launch_epoch(rt_server* s, Slot& slot) {
     TraceArgs args{};
     args.bundles = slot.dev_table;
     args.n_bundles = nb;
+    if (nb == 1 && !multi && !bl) {
+        args.one = slot.host_table[0];
+        args.has_one = 1;
+    }
     args.refill_threshold = c.refill_threshold;
     args.claim = 32u * c.rays_per_thread;
     args.total_rays = total;

@@ -202,8 +202,15 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 // again.  Both passes solve disk crossings on the step's dense output.  Parked
 // rays resume from their saved state, so a ray's arithmetic does not depend on
 // which rays share its warp.
-template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, int WARPS = 12>
-__global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(TraceArgs args) {
+//
+// ONE: a launch of one camera, its descriptor among the kernel's parameters: the step
+// loop's dozen constants are operands from the constant bank instead of loads that
+// every attempt waits for and registers they sit in.  (Continued traces, CONT, are
+// always of one camera.)  Descriptor in memory / in the parameters: 2048^2 FP64 31.7 /
+// 30.6 ms, 2048^2 mixed 21.1 / 20.4 ms, 1279x717 mixed 6.2 / 5.9 ms.
+template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, int WARPS = 12,
+          bool ONE = (CONT != 0)>
+__global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(const __grid_constant__ TraceArgs args) {
     __shared__ Cold<BLOCK> S;
     __shared__ KStore<ROLLED ? BLOCK : 1> K;
     const unsigned FULL = 0xffffffffu;
@@ -216,6 +223,10 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
     static_assert(!NEAR_PASS || !MIXED, "the near pass runs FP64 stages");
     // rays of this launch: pixels (single kernel, first far pass) or queue entries
     // (later passes; the single kernel as the critical pass of a two-pass launch)
+    auto bundle = [&args](uint32_t i) -> const BundleDesc* {
+        if constexpr (ONE) return &args.one;
+        else return args.bundles + i;
+    };
     const bool from_queue =
         (PASS == PASS_SINGLE) ? (args.in_queue != nullptr) : !(FAR_PASS && args.from_pixels != 0);
     const uint64_t total = from_queue ? static_cast<uint64_t>(*args.in_count) : args.total_rays;
@@ -317,7 +328,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
             if (ended && (n_free == 32 || ((queue_open || chunk_next < chunk_end) &&
                                            n_free >= static_cast<int>(args.refill_threshold)))) {
                 if (mode == MODE_ENDED) {
-                    const BundleDesc* Be = args.bundles + bidx;
+                    const BundleDesc* Be = bundle(bidx);
                     const uint32_t cls = end_kind & 15u;
                     double target = 0.0, xch[24];
 #pragma unroll
@@ -380,11 +391,12 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                         if (from_queue) rix = args.in_queue[rid];
                     }
                     // bundle of this ray: last bundle whose ray_begin <= rix
-                    uint32_t lo = 0, hi = args.n_bundles;
+                    uint32_t lo = 0, hi = ONE ? 1u : args.n_bundles;
                     while (hi - lo > 1) {
                         const uint32_t mid = (lo + hi) >> 1;
                         if (args.bundles[mid].ray_begin <= rix) lo = mid; else hi = mid;
                     }
+                    const BundleDesc* Bc = bundle(lo);
                     bidx = lo;
                     ray = rix;
                     bool resumed = false;
@@ -392,7 +404,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                         if (from_queue) {
                             double xch[13];
                             uint32_t uch[PU_COUNT];
-                            r = resume_ray(args.bundles + lo, args.park, rix, rix - args.bundles[lo].ray_begin,
+                            r = resume_ray(Bc, args.park, rix, rix - Bc->ray_begin,
                                                   S, tid, xch, uch);
 #pragma unroll
                             for (int i = 0; i < 6; ++i) {
@@ -418,7 +430,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                     if (!resumed) {
                         double xch[12];
                         const InitResult ir =
-                            init_ray(args.bundles + lo, rix - args.bundles[lo].ray_begin, S, tid, xch);
+                            init_ray(Bc, rix - Bc->ray_begin, S, tid, xch);
 #pragma unroll
                         for (int i = 0; i < 6; ++i) {
                             y[i] = xch[i];
@@ -426,17 +438,16 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
                         }
                         r = ir.r;
                         can_early = ir.can_early;
-                        h = -args.bundles[lo].h0;
+                        h = -Bc->h0;
                         lnp = 0.0f;
                         has_hist = false;
                         acc = rej = flags = 0;
-                        wind = args.bundles[lo].wind0;
+                        wind = Bc->wind0;
                         k1_fp32 = false;
                         guard = 0;
                         n_cross = 0;
                         critical = false;
                         tol_sc = 1.0f;
-                        const BundleDesc* Bc = args.bundles + lo;
                         // mixed mode: the distance of the ray's constants from the critical
                         // curve decides whether it is near-critical (and the Carter early
                         // capture, from the same value); the critical pass grades its
@@ -475,7 +486,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
             far = true;  // near-zone rays were parked for the near pass
         } else if constexpr (MIXED) {
             const bool stepping = (mode == MODE_STEP || mode == MODE_REDO);
-            const BundleDesc* Bz = args.bundles + bidx;
+            const BundleDesc* Bz = bundle(bidx);
             const bool lane_far = stepping && !critical && r >= Bz->fp64_radius && r < kFp32MaxRadius;
             // every lane executes the ballot (no short-circuit around a full-mask sync)
             const unsigned near_lanes = __ballot_sync(FULL, stepping && !lane_far);
@@ -483,7 +494,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
         }
         if (mode == MODE_IDLE || mode == MODE_ENDED) continue;
 
-        const BundleDesc* Bp = args.bundles + bidx;
+        const BundleDesc* Bp = bundle(bidx);
         const double M = Bp->m, a = Bp->a;
         // backstop: a ray needs at most 62 iterations per attempt (attempt, <= 60
         // root iterations, redo); past that bound it is ended as unfinished
@@ -870,36 +881,41 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(Trac
 // unshaded launches (CONT = 0), shaded ones that follow rays through the
 // translucent disk (CONT = 1) and, for hydro model 2, the FP64 tracer that
 // gathers the Fishbone-Moncrief torus's light step by step (CONT = 2)
-template __global__ void trace_kernel_t<64, false, false>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false>(TraceArgs);
-template __global__ void trace_kernel_t<256, false, false>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 1, 8>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 0, 8>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1, 8>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 0, 8>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1, 8>(TraceArgs);
-template __global__ void trace_kernel_t<64, false, true>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, true>(TraceArgs);
-template __global__ void trace_kernel_t<64, true, true>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, true>(TraceArgs);
-template __global__ void trace_kernel_t<64, true, false, PASS_FAR>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, false, PASS_FAR>(TraceArgs);
-template __global__ void trace_kernel_t<64, false, false, PASS_NEAR>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_NEAR>(TraceArgs);
-template __global__ void trace_kernel_t<64, false, false, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<256, false, false, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<64, false, true, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, true, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<64, true, true, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, true, PASS_SINGLE, 1>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 2>(TraceArgs);
-template __global__ void trace_kernel_t<64, true, false, PASS_FAR, true>(TraceArgs);
-template __global__ void trace_kernel_t<128, true, false, PASS_FAR, true>(TraceArgs);
-template __global__ void trace_kernel_t<64, false, false, PASS_NEAR, true>(TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, true>(TraceArgs);
+template __global__ void trace_kernel_t<64, false, false>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<256, false, false>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 1, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 0, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 0, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 12, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 0, 8, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 0, 12, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 0, 8, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 0, 12, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, false, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, true, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, true>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, true, false, PASS_FAR>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, false, false, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<256, false, false, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, false, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 2>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<64, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1>(const __grid_constant__ TraceArgs);
 
 namespace {
 // Mixed precision always uses the rolled FP64 step (its FP64 steps are a
@@ -927,11 +943,13 @@ const void* kernel_for(uint32_t block, bool mixed, bool rolled, int cont = 0) {
     return (cont == 1) ? kernel_for_t<1>(block, mixed, rolled) : kernel_for_t<0>(block, mixed, rolled);
 }
 
-// The plain FP64 tracer with 16 warps per SM, and with 8.
-const void* wide_kernel() { return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, 16>); }
-const void* lean_kernel(bool cont) {
-    return cont ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 1, 8>)
-                : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, 8>);
+// The plain FP64 tracer in 128-thread blocks with 8, 12 or 16 warps per SM.
+template <int WARPS>
+const void* plain_kernel_t(bool cont, bool one) {
+    if constexpr (WARPS < 16)
+        if (cont) return reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 1, WARPS>);
+    return one ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, WARPS, true>)
+               : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 0, WARPS, false>);
 }
 
 // Rays per SM from which the plain FP64 tracer takes 16 warps.  More warps raise the
@@ -953,7 +971,7 @@ constexpr uint64_t kLeanMixedRaysPerSm = 1024;
 // Loads the kernels that launch_trace may pick beside those of trace_occupancy.
 void preload_trace_shapes() {
     int n = 0;
-    for (const void* k : {wide_kernel(), lean_kernel(false)})
+    for (const void* k : {plain_kernel_t<8>(false, false), plain_kernel_t<16>(false, false)})
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, 0) != cudaSuccess) cudaGetLastError();
 }
 
@@ -1007,25 +1025,26 @@ __global__ void __launch_bounds__(BLOCK) finish_kernel_t(TraceArgs args) {
 template __global__ void finish_kernel_t<128>(TraceArgs);
 
 namespace {
-template <bool CONT>
-const void* pass_kernel_t(int pass, uint32_t block, bool lean) {
-    if (pass == PASS_FAR) {
-        if (block == 64) return reinterpret_cast<const void*>(&trace_kernel_t<64, true, false, PASS_FAR, CONT>);
-        return lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, true, false, PASS_FAR, CONT, 8>)
-                    : reinterpret_cast<const void*>(&trace_kernel_t<128, true, false, PASS_FAR, CONT>);
-    }
-    if (block == 64) return reinterpret_cast<const void*>(&trace_kernel_t<64, false, false, PASS_NEAR, CONT>);
-    return lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_NEAR, CONT, 8>)
-                : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_NEAR, CONT>);
+template <bool MIXED, int PASS, int WARPS>
+const void* pass_kernel_t(bool cont, bool one) {
+    if (cont) return reinterpret_cast<const void*>(&trace_kernel_t<128, MIXED, false, PASS, 1, WARPS>);
+    return one ? reinterpret_cast<const void*>(&trace_kernel_t<128, MIXED, false, PASS, 0, WARPS, true>)
+               : reinterpret_cast<const void*>(&trace_kernel_t<128, MIXED, false, PASS, 0, WARPS, false>);
 }
 
-const void* pass_kernel(int pass, uint32_t block, bool lean, bool cont = false) {
-    return cont ? pass_kernel_t<true>(pass, block, lean) : pass_kernel_t<false>(pass, block, lean);
+const void* pass_kernel(int pass, uint32_t block, bool lean, bool cont, bool one) {
+    if (pass == PASS_FAR) {
+        if (block == 64)
+            return cont ? reinterpret_cast<const void*>(&trace_kernel_t<64, true, false, PASS_FAR, 1>)
+                        : reinterpret_cast<const void*>(&trace_kernel_t<64, true, false, PASS_FAR, 0>);
+        return lean ? pass_kernel_t<true, PASS_FAR, 8>(cont, one) : pass_kernel_t<true, PASS_FAR, 12>(cont, one);
+    }
+    return lean ? pass_kernel_t<false, PASS_NEAR, 8>(cont, one) : pass_kernel_t<false, PASS_NEAR, 12>(cont, one);
 }
 
 int trace_pass_occupancy(int pass, uint32_t block, bool lean) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pass_kernel(pass, block, lean), static_cast<int>(block), 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pass_kernel(pass, block, lean, false, false), static_cast<int>(block), 0) !=
         cudaSuccess) {
         cudaGetLastError();
         return 1;
@@ -1036,8 +1055,8 @@ int trace_pass_occupancy(int pass, uint32_t block, bool lean) {
 // One pass of the two-pass mixed tracer (PASS_FAR or PASS_NEAR).
 void launch_trace_pass(const TraceArgs& args, int pass, uint32_t grid, uint32_t block, bool lean, cudaStream_t stream) {
     void* params[] = {const_cast<TraceArgs*>(&args)};
-    cudaLaunchKernel(pass_kernel(pass, block, lean, args.cont.cross != nullptr), dim3(grid), dim3(block), params, 0,
-                     stream);
+    cudaLaunchKernel(pass_kernel(pass, block, lean, args.cont.cross != nullptr, args.has_one != 0u), dim3(grid),
+                     dim3(block), params, 0, stream);
 }
 }  // namespace
 
@@ -1276,13 +1295,15 @@ void launch_trace(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, uin
     const void* kernel = kernel_for(block, mixed, rolled, cont);
     // 8 or 16 warps per SM only where the caller left the CTAs per SM at the occupancy
     // maximum; the critical pass's rays are counted on the device, so its caller decides
-    if (!mixed && !rolled && cont != 2 && block == 128u && ctas_per_sm >= 3u) {
+    if (!mixed && !rolled && cont != 2 && block == 128u) {
         const uint64_t sm = static_cast<uint64_t>(sm_count);
-        if (lean || (!args.in_queue && args.total_rays <= kLeanRaysPerSm * sm)) {
-            kernel = lean_kernel(cont == 1);
+        const bool one = args.has_one != 0u, shaped = ctas_per_sm >= 3u;
+        kernel = plain_kernel_t<12>(cont == 1, one);
+        if (shaped && (lean || (!args.in_queue && args.total_rays <= kLeanRaysPerSm * sm))) {
+            kernel = plain_kernel_t<8>(cont == 1, one);
             ctas_per_sm = 2;
-        } else if (cont == 0 && !args.in_queue && args.total_rays >= kWideRaysPerSm * sm) {
-            kernel = wide_kernel();
+        } else if (shaped && cont == 0 && !args.in_queue && args.total_rays >= kWideRaysPerSm * sm) {
+            kernel = plain_kernel_t<16>(false, one);
             ctas_per_sm = 4;
         }
     }
