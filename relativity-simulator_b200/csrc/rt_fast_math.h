@@ -44,6 +44,12 @@ RT_FM_FN double refine_sqrt(double v, double y) {
     return fma(fma(-g, g, v), 0.5 * y, g);
 }
 
+// 1 / sqrt(v) by the same third-order step; within an ulp, not correctly rounded.
+RT_FM_FN double refine_rsqrt(double v, double y) {
+    const double e = fma(-v * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ double fast_rcp(double v) {
     double y;
@@ -55,6 +61,12 @@ __device__ __forceinline__ double fast_sqrt(double v) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
     return refine_sqrt(v, y);
+}
+
+__device__ __forceinline__ double fast_rsqrt(double v) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    return refine_rsqrt(v, y);
 }
 #endif
 

@@ -9,6 +9,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "rt_fast_math.h"
+
 #ifdef __CUDACC__
 #define RT_FM_HD __host__ __device__ inline
 #else
@@ -61,8 +63,11 @@ RT_FM_HD double potential(const Torus& t, double r, double theta) { return poten
 // imposed): false outside the torus (no such orbit, or an enthalpy h = exp(W_in - W)
 // of 1 + 1e-9 or less, :152-159), else h and the four-velocity's u^t and u^phi
 // (:210-224: u_t = -e^W, u_phi = -l u_t, raised with the Boyer-Lindquist Kerr inverse
-// metric, metrics/kerr.hpp:151-177).  W = log(X) / 2, so e^W = sqrt(X) and no
-// logarithm or exponential is taken; e_in = exp(W_in).
+// metric, metrics/kerr.hpp:151-177).  With W = log(X) / 2, X = rho^2 Delta sin^2 / D,
+// no logarithm or exponential is taken: h = e_in / sqrt(X), e_in = exp(W_in), and
+// e^W / (rho^2 Delta) = sin^2 / (sqrt(X) D) leaves 1 / D and 1 / sqrt(X) as the only
+// divisions.  On the device these are the straight-line forms (rt_fast_math.h): D and
+// X of a sampled point are far from the ends of the range, and a NaN is outside.
 RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_in, double& h, double& ut, double& uphi) {
     if (r <= t.rh * 1.0001) return false;
     const double s2 = fmx(s2_in, 1e-30);
@@ -73,13 +78,18 @@ RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_
     const double ds = delta - a2 * s2;
     const double denom = sigma * s2 - 2.0 * mra * t.l * s2 - t.l * t.l * ds;
     if (denom <= 0.0 || delta <= 0.0) return false;
-    const double rd = rho2 * delta;
-    const double ew = sqrt(fmx((rd * s2) / denom, 1e-30));
-    h = e_in / ew;
+#ifdef __CUDA_ARCH__
+    const double inv_d = fast_rcp(denom);
+    const double inv_ew = fast_rsqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30));
+#else
+    const double inv_d = 1.0 / denom;
+    const double inv_ew = 1.0 / sqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30));
+#endif
+    h = e_in * inv_ew;
     if (!(h > 1.0 + 1e-9)) return false;
-    const double q = ew / rd;
-    ut = q * (sigma - mra * t.l);
-    uphi = q * (mra + t.l * ds / s2);
+    const double q = inv_ew * inv_d;
+    ut = q * (sigma - mra * t.l) * s2;
+    uphi = q * (mra * s2 + t.l * ds);
     return true;
 }
 

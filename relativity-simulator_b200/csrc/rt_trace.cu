@@ -207,7 +207,8 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 // loop's dozen constants are operands from the constant bank instead of loads that
 // every attempt waits for and registers they sit in.  (Continued traces, CONT, are
 // always of one camera.)  Descriptor in memory / in the parameters: 2048^2 FP64 31.7 /
-// 30.6 ms, 2048^2 mixed 21.1 / 20.4 ms, 1279x717 mixed 6.2 / 5.9 ms.
+// 31.5 ms, 2048^2 mixed 21.1 / 20.1 ms, 1279x717 mixed 6.2 / 5.85 ms, the 1536^2 frame
+// with the sky 30.9 / 28.8 ms.
 template <int BLOCK, bool MIXED, bool ROLLED, int PASS = PASS_SINGLE, int CONT = 0, int WARPS = 12,
           bool ONE = (CONT != 0)>
 __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(const __grid_constant__ TraceArgs args) {
