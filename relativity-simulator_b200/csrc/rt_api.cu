@@ -59,6 +59,8 @@ struct rt_handle {
     // translucent-disk continuation of a shaded dispatch: each ray's disk crossings
     // and how it ended, and what the launches pass the tracer
     DevBuf cont_cross, cont_info, cont_body, cont_exit, cont_tail, cont_vol, cont_lz;
+    DevBuf path_pages, path_rays, path_cursor;  // torus-shaded traces: the steps' points (PathOut)
+    double torus_skip = 0.0;                    // PathOut::skip of the dispatch
     DevBuf ms_shade;  // multi-source shading: one descriptor per source
     ContOut cur_cont{};
     rt_shading shading{};
@@ -228,6 +230,32 @@ rt_status launch_two_pass(rt_handle* h, uint32_t n_bundles, uint64_t total, cons
     return RT_OK;
 }
 
+// A torus-shaded Kerr-Schild trace in parts whose steps' points fit the page pool: 64
+// points (1.5 KB) a page, five pages a ray at rtol 1e-10 (an edge-on frame of a hole of
+// spin 0.998 uses three), more at a tighter tolerance or step cap, at most 4 GB.  False:
+// the pool could not be had, or the parts would be so small that each is bound by its
+// longest ray (10 ms; a part of 2^17 rays traces as long).
+constexpr uint64_t kMaxPathPages = 2'600'000, kMinPathPart = 1u << 17;
+bool reserve_path(rt_handle* h, uint64_t total, PathOut& path, uint64_t& part) {
+    const BundleDesc& b = h->host_bundles[0];
+    const double scale = std::max(1.0, std::pow(1e-10 / std::max(b.rtol, 1e-16), 0.2)) * std::max(1.0, 0.1 / b.cap_c);
+    const uint64_t per_ray = static_cast<uint64_t>(std::ceil(5.0 * std::min(scale, 1e3)));
+    part = std::max<uint64_t>(1, std::min<uint64_t>(total, kMaxPathPages / per_ray));
+    if (part < std::min(total, kMinPathPart)) return false;
+    const uint64_t pages = std::min<uint64_t>(part * per_ray, kMaxPathPages);
+    if (ensure(h, h->path_pages, sizeof(double) * kPathPageDoubles * pages) != RT_OK ||
+        ensure(h, h->path_rays, sizeof(uint32_t) * 4 * total) != RT_OK ||
+        ensure(h, h->path_cursor, kPathCursorBytes) != RT_OK) {
+        h->error.clear();  // the tracer that gathers as it goes needs no pool
+        return false;
+    }
+    uint32_t* rays = static_cast<uint32_t*>(h->path_rays.ptr);
+    path = PathOut{static_cast<double*>(h->path_pages.ptr), rays, rays + total,
+                   static_cast<uint32_t*>(h->path_cursor.ptr), rays + 2 * total, rays + 3 * total,
+                   static_cast<uint32_t>(pages), 0u, h->torus_skip};
+    return true;
+}
+
 // Launch the tracer over `n` bundles already in h->bundles (device).  The
 // timing events bracket the launch unless it is being captured into a graph
 // (an event recorded on a capturing stream only orders the capture; the graph
@@ -252,9 +280,21 @@ rt_status launch(rt_handle* h, uint32_t n_bundles, uint64_t total, const OutPtrs
     args.cont = h->cur_cont;
     RT_CUDA(h, cudaMemsetAsync(h->queue.ptr, 0, sizeof(unsigned long long), s));
     RT_CUDA(h, cudaMemsetAsync(h->stats.ptr, 0, sizeof(unsigned long long) * ST_COUNT, s));
+    uint64_t part = 0;
+    const bool sampled = args.cont.vol && args.has_one && !c.fp64_rolled && total <= 0xffffffffull &&
+                         reserve_path(h, total, args.path, part);
     if (!capturing) RT_CUDA(h, cudaEventRecord(h->ev0, s));
-    launch_trace(args, h->sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, s);
-    RT_CUDA(h, cudaGetLastError());
+    if (sampled) {
+        for (uint64_t b = 0; b < total; b += part) {
+            args.ray_base = b;
+            args.total_rays = std::min(part, total - b);
+            RT_CUDA(h, static_cast<cudaError_t>(enqueue_torus(args, h->sm_count, c.ctas_per_sm,
+                                                              static_cast<char*>(h->queue.ptr), s)));
+        }
+    } else {
+        launch_trace(args, h->sm_count, c.ctas_per_sm, c.block_size, mixed, c.fp64_rolled != 0, s);
+        RT_CUDA(h, cudaGetLastError());
+    }
     if (!capturing) {
         RT_CUDA(h, cudaEventRecord(h->ev1, s));
         h->timed = true;
@@ -330,6 +370,8 @@ rt_status shade_prepare(rt_handle* h, const rt_camera* cam, cudaStream_t s) {
     if (!build_shade_desc(*cam, h->shading, d)) return fail(h, RT_ERR_INVALID_ARG, "unsupported shading settings");
     rt_status st;
     if ((st = ensure_planck(h, s)) != RT_OK) return st;
+    // a chord between two points within the inner bound has no sample outside it
+    h->torus_skip = d.fm_valid ? d.fm_inner * (1.0 - 1e-9) : 1e300;
     d.planck = static_cast<const double*>(h->planck.ptr);
     if ((st = ensure(h, h->shade_desc, sizeof(ShadeDesc))) != RT_OK) return st;
     // pageable descriptor: the copy is staged before the call returns
@@ -503,7 +545,8 @@ rt_status dispatch_window(rt_handle* h, const rt_camera* cam, uint32_t col0, uin
         BandCopyCtx ctx{h, rays, dev, pixels, dpix, offset, shade, 0, h->cur_cont};
         const bool two_pass = !is_bl(cam) && uses_two_pass(effective_cfg(h, cam->precision_mode == RT_PRECISION_MIXED),
                                                           cam->precision_mode == RT_PRECISION_MIXED, launch_rays);
-        if (!two_pass && launch_rays >= kBandedMinRays && rows >= kCopyBands) {
+        const bool torus = !is_bl(cam) && h->cur_cont.vol;  // traced in parts of its own (reserve_path)
+        if (!two_pass && !torus && launch_rays >= kBandedMinRays && rows >= kCopyBands) {
             if ((st = launch_banded_single(h, cam, col0, ncols, row0 + r, rows, offset, OutPtrs{dpix, dev}, ctx)) !=
                 RT_OK)
                 return st;
@@ -874,6 +917,9 @@ void rt_destroy(rt_handle* h) {
     release(h->cont_tail);
     release(h->cont_vol);
     release(h->cont_lz);
+    release(h->path_pages);
+    release(h->path_rays);
+    release(h->path_cursor);
     release(h->park_d);
     release(h->park_u);
     release(h->pass_queues);

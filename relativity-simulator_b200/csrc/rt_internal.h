@@ -134,6 +134,25 @@ struct ParkBuf {
 // near-zone pass; rays move between them through queues of launch indices.
 enum TracePass : int { PASS_SINGLE = 0, PASS_FAR = 1, PASS_NEAR = 2 };
 
+// Points of the accepted steps of a torus-shaded trace, for the sampling pass: per ray
+// a chain of pages, each kPathPoints Kerr-Schild points and the index of the next page.
+// Steps inside the torus's inner bound are left out; a point whose x is NaN stands for
+// them, and the chain goes on with the start of the next step.
+constexpr uint32_t kPathPoints = 64, kPathPageDoubles = 3 * kPathPoints + 1, kPathOverflow = 0xffffffffu;
+constexpr size_t kPathCursorBytes = 5 * sizeof(uint32_t);
+struct PathOut {
+    double* pages;       // [capacity][kPathPageDoubles]
+    uint32_t* first;     // per output element: the ray's first page
+    uint32_t* points;    // per output element: points stored; kPathOverflow: the pages ran out
+    uint32_t* cursor;    // [0] next free page, [1] rays in the overflow queue, [2] and [3] plunging and
+                         // other rays placed in `order`, [4] rays in it
+    uint32_t* overflow;  // launch indices of rays whose pages ran out
+    uint32_t* order;     // launch indices, the rays that plunge into the hole first
+    uint32_t capacity;   // pages
+    uint32_t pad;
+    double skip;         // a step with both ends within this radius crosses no part of the torus
+};
+
 // Length classes of near-critical rays, in the upper bits of a queue entry.
 constexpr uint32_t kCritClasses = 32, kCritClassShift = 27;
 
@@ -160,6 +179,7 @@ struct TraceArgs {
     uint32_t* crit_queue;       // first far pass: near-critical rays, for the critical pass
     uint32_t* crit_count;
     uint64_t crit_classes;      // 1: crit_queue entries carry the ray's length class in their upper bits
+    PathOut path;               // torus-shaded traces that leave the torus to the sampling pass (else null)
     BundleDesc one;             // has_one: the launch's only bundle, read in place of bundles[0]
     ParkBuf park;
     // translucent-disk continuation (single-camera launches with shading): the
@@ -330,6 +350,11 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
                      BandHook after_band = nullptr, void* hook_ctx = nullptr);
 int trace_occupancy(uint32_t block, bool mixed, bool rolled);
 void preload_trace_shapes();
+// Torus-shaded rays [args.ray_base, + args.total_rays) of one camera: the trace storing
+// its steps' points, the sampling pass over them, then the rays whose pages ran out,
+// traced again with the torus sampled step by step.  claims: two zeroed-here counters
+// 64 bytes apart.
+int enqueue_torus(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, char* claims, void* stream);
 uint32_t kernel_block(uint32_t block, bool mixed, bool rolled);
 // Launch shape with defaults filled in and limits applied for one precision.
 rt_launch_config resolve_launch_config(rt_launch_config c, bool mixed);

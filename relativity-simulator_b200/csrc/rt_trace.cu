@@ -185,6 +185,45 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 
 }  // namespace
 
+// Store the end of a ray's accepted step (after a gap its start too) in its chain of
+// pages (PathOut); the page is S.side, the count S.rit (both idle: a torus-shaded trace
+// has no disk roots).  False: no free page; the ray is in the overflow queue and its
+// steps are off the counters.
+constexpr int kPathGap = 1 << 30;  // in S.rit: steps were left out since the last point
+template <class ColdT>
+__device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, int tid, uint64_t ray, uint64_t o,
+                                               uint32_t acc, uint32_t rej, const double* x) {
+    const PathOut& P = args.path;
+    uint32_t k = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
+    double* page = P.pages + static_cast<uint64_t>(S.side[tid]) * kPathPageDoubles;
+    for (int i = (S.rit[tid] & kPathGap) ? 0 : 2; i < 3; ++i, ++k) {  // gap, start, end
+        const uint32_t slot = k % kPathPoints;
+        if (slot == 0) {
+            const uint32_t next = atomicAdd(P.cursor, 1u);
+            if (next >= P.capacity) {
+                P.points[o] = kPathOverflow;
+                P.overflow[atomicAdd(P.cursor + 1, 1u)] = static_cast<uint32_t>(ray);
+                const unsigned long long att = static_cast<unsigned long long>(acc) + rej;
+                atomicAdd(args.stats + ST_ATTEMPTS, 0ull - att);
+                atomicAdd(args.stats + ST_FP64_ATTEMPTS, 0ull - att);
+                atomicAdd(args.stats + ST_ACCEPTED, 0ull - acc);
+                atomicAdd(args.stats + ST_RHS, 0ull - (6 * att + 1));
+                return false;
+            }
+            if (k == 0) P.first[o] = next;
+            else page[3 * kPathPoints] = static_cast<double>(next);
+            S.side[tid] = static_cast<int>(next);
+            page = P.pages + static_cast<uint64_t>(next) * kPathPageDoubles;
+        }
+        double* at = page + 3 * slot;
+        at[0] = (i == 0) ? __longlong_as_double(0x7ff8000000000000ll) : x[3 * (i - 1)];
+        at[1] = x[i == 0 ? 1 : 3 * (i - 1) + 1];
+        at[2] = x[i == 0 ? 2 : 3 * (i - 1) + 2];
+    }
+    S.rit[tid] = static_cast<int>(k);
+    return true;
+}
+
 // WARPS resident warps per SM set the registers per thread: 8 warps at up to 255
 // registers, 12 at 168, 16 at 128.  Fewer warps spill less and an attempt takes less
 // time; more warps hide more of the FP64 latency that bounds the step loop.
@@ -350,6 +389,11 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                                    disk_redshift(Be->m, Be->a, rr, S.lz0[tid]), args.out, xch);
                     } else {
                         end_ray<(CONT != 0)>(args, Be, S, tid, n_cross, cls, flags, acc, rej, wind, target, h, xch);
+                        if constexpr (CONT == 3) {
+                            const uint64_t o = Be->out_offset + S.local[tid];
+                            args.path.points[o] = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
+                            args.cont.lz[o] = S.lz0[tid];
+                        }
                     }
                     mode = MODE_IDLE;
                 }
@@ -444,6 +488,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                         has_hist = false;
                         acc = rej = flags = 0;
                         wind = Bc->wind0;
+                        if constexpr (CONT == 3) S.rit[tid] = S.side[tid] = 0;  // points stored, page
                         k1_fp32 = false;
                         guard = 0;
                         n_cross = 0;
@@ -453,7 +498,8 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                         // curve decides whether it is near-critical (and the Carter early
                         // capture, from the same value); the critical pass grades its
                         // tolerance with it
-                        if ((MIXED && Bc->critical_band > 0.0f) || (PASS == PASS_SINGLE && !MIXED && from_queue)) {
+                        if ((MIXED && Bc->critical_band > 0.0f) ||
+                            (PASS == PASS_SINGLE && !MIXED && CONT < 2 && from_queue)) {
                             const double db = shadow_distance(Bc->m, Bc->a, 0.0, Bc->rh, S.lz0[tid], S.q0[tid]);
                             if (can_early < 0) can_early = db > kEarlyCaptureMargin;
                             const double band = static_cast<double>(Bc->critical_band) * Bc->m;
@@ -462,7 +508,8 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                             if (critical && FAR_PASS) n_cross = critical_class(db, band);
                         }
                         mode = MODE_STEP;
-                        if (!(PASS == PASS_SINGLE && from_queue)) ++n_rays;  // counted by the far pass
+                        // a queue of rays left by a pass that has counted them
+                        if (!(PASS == PASS_SINGLE && from_queue) || CONT == 3) ++n_rays;
                         ++n_rhs;
                     }
                 }
@@ -832,6 +879,18 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                 }
             }
         }
+        if constexpr (CONT == 3) {
+            // hydro model 2: the step's end, for the sampling pass
+            if (fmax(r, r5) < args.path.skip) {
+                S.rit[tid] |= kPathGap;
+            } else {
+                const double ends[6] = {y[0], y[1], y[2], y5[0], y5[1], y5[2]};
+                if (!store_path_points(args, S, tid, ray, Bp->out_offset + S.local[tid], acc, rej, ends)) {
+                    mode = MODE_IDLE;  // out of pages: traced again from the start
+                    continue;
+                }
+            }
+        }
         if constexpr (CONT == 2) {
             // hydro model 2: the step's chord through the Fishbone-Moncrief torus
             // (software_compute_engine.hpp:1725-1731)
@@ -879,9 +938,16 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
     }
 }
 
+// The trace of a torus-shaded frame is bound by its longest rays' chains of steps (3,700
+// where the mean is 320), so the lean form: 640x360 17.0 ms at 8 warps per SM, 18.0 at
+// 12; 1920x1080 83.6 / 81.2.
+constexpr int kTorusWarps = 8;
+constexpr uint32_t kSampleBlock = 64;
+
 // unshaded launches (CONT = 0), shaded ones that follow rays through the
 // translucent disk (CONT = 1) and, for hydro model 2, the FP64 tracer that
-// gathers the Fishbone-Moncrief torus's light step by step (CONT = 2)
+// gathers the Fishbone-Moncrief torus's light step by step (CONT = 2) or stores the
+// steps' points for the sampling pass (CONT = 3)
 template __global__ void trace_kernel_t<64, false, false>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, false, false>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<256, false, false>(const __grid_constant__ TraceArgs);
@@ -914,6 +980,7 @@ template __global__ void trace_kernel_t<128, false, true, PASS_SINGLE, 1>(const 
 template __global__ void trace_kernel_t<64, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 2>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 3, kTorusWarps>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<64, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1>(const __grid_constant__ TraceArgs);
@@ -1310,6 +1377,113 @@ void launch_trace(const TraceArgs& args, int sm_count, uint32_t ctas_per_sm, uin
     }
     cudaLaunchKernel(kernel, dim3(static_cast<uint32_t>(sm_count) * ctas_per_sm), dim3(block), params, 0,
                      static_cast<cudaStream_t>(stream));
+}
+
+// The order in which a torus-shaded trace takes its rays: those inside the critical
+// curve first.  They plunge, and their steps shrink with the distance to the horizon
+// (about 1,750 a ray against 180 for one that turns back), so that a warp of them begun
+// late runs on alone; begun first, and with their like in a warp, the short rays fill in.
+__global__ void __launch_bounds__(128) torus_order_kernel(const __grid_constant__ TraceArgs args) {
+    __shared__ Cold<128> S;
+    const BundleDesc& B = args.one;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * 128 + tid;
+    const bool live = i < args.total_rays;
+    bool plunges = false;
+    if (live) {
+        double xch[12];
+        init_ray(&B, args.ray_base + i, S, tid, xch);
+        plunges = shadow_distance(B.m, B.a, 0.0, B.rh, S.lz0[tid], S.q0[tid]) > 0.0;
+    }
+    const unsigned first = __ballot_sync(~0u, live && plunges), rest = __ballot_sync(~0u, live && !plunges);
+    uint32_t at = 0;
+    if (lane < 2) {
+        const uint32_t n = static_cast<uint32_t>(__popc(lane == 0 ? first : rest));
+        if (n) at = atomicAdd(args.path.cursor + 2 + lane, n);
+    }
+    const uint32_t at_first = __shfl_sync(~0u, at, 0), at_rest = __shfl_sync(~0u, at, 1);
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t total = static_cast<uint32_t>(args.total_rays);
+    if (live) {
+        const uint32_t to = plunges ? at_first + __popc(first & below) : total - 1u - (at_rest + __popc(rest & below));
+        args.path.order[to] = static_cast<uint32_t>(args.ray_base + i);
+    }
+    if (i == 0) args.path.cursor[4] = total;
+}
+
+// The sampling pass of a torus-shaded trace: one thread per ray walks its chain of
+// points and gathers the light of each chord (fm_chord), in the order of the steps.
+// Gathering inside the step loop ran two large pieces of code in turn on every warp,
+// each evicting the other from the instruction cache (no_instruction 3.5 of 9.6 cycles
+// per issue, FP64 pipe 26 %).  Measured, 640x360, gathering as it goes / in this pass:
+// 32.7 / 17.0 ms (trace 12.5, this pass 4.5, bound by the few rays that run along the
+// equatorial plane), 1920x1080 159 / 84, 64x36 14.6 / 10.1.
+__global__ void __launch_bounds__(kSampleBlock) torus_sample_kernel(const __grid_constant__ TraceArgs args) {
+    const BundleDesc& B = args.one;
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kSampleBlock + threadIdx.x;
+    if (i >= args.total_rays) return;
+    const uint64_t o = B.out_offset + args.path.order[i];
+    const uint32_t points = args.path.points[o];
+    if (points == kPathOverflow || points == 0) return;
+    double x[3], from[3], V[VL_COUNT] = {};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[c] = B.x0[c];
+    bl_cartesian(x, B.a, from);
+    const double lz = args.cont.lz[o];
+    const double* page = args.path.pages + static_cast<uint64_t>(args.path.first[o]) * kPathPageDoubles;
+    bool gap = false;
+    for (uint32_t k = 0, slot = 0; k < points; ++k, ++slot) {
+        if (slot == kPathPoints) {
+            page = args.path.pages + static_cast<uint64_t>(page[3 * kPathPoints]) * kPathPageDoubles;
+            slot = 0;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = page[3 * slot + c];
+        if (x[0] != x[0]) {
+            gap = true;
+            continue;
+        }
+        double to[3];
+        bl_cartesian(x, B.a, to);
+        if (!gap) {
+            fm_chord(*args.cont.shade, from, to, lz, V);
+            if (V[VL_HIT] != 0.0 && !(V[VL_THR] > kMinThroughputVol)) break;
+        }
+        gap = false;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) from[c] = to[c];
+    }
+    double* out = args.cont.vol + o * VL_COUNT;
+#pragma unroll
+    for (int f = 0; f < VL_COUNT; ++f) out[f] = V[f];
+}
+
+int enqueue_torus(const TraceArgs& base, int sm_count, uint32_t ctas_per_sm, char* claims, void* stream) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    TraceArgs args = base;
+    cudaError_t e = cudaMemsetAsync(claims, 0, 72, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(args.path.cursor, 0, kPathCursorBytes, s);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    torus_order_kernel<<<static_cast<uint32_t>((args.total_rays + 127) / 128), 128, 0, s>>>(args);
+    if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
+    args.queue = reinterpret_cast<unsigned long long*>(claims);
+    args.in_queue = args.path.order;
+    args.in_count = args.path.cursor + 4;
+    void* params[] = {&args};
+    cudaLaunchKernel(reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, kTorusWarps>),
+                     dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, kTorusWarps / 4u)), dim3(128), params,
+                     0, s);
+    if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
+    torus_sample_kernel<<<static_cast<uint32_t>((args.total_rays + kSampleBlock - 1) / kSampleBlock), kSampleBlock, 0,
+                          s>>>(args);
+    if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
+    // the rays whose pages ran out
+    args.queue = reinterpret_cast<unsigned long long*>(claims + 64);
+    args.in_queue = args.path.overflow;
+    args.in_count = args.path.cursor + 1;
+    cudaLaunchKernel(reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 2>),
+                     dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, 3u)), dim3(128), params, 0, s);
+    return static_cast<int>(cudaGetLastError());
 }
 
 rt_launch_config resolve_launch_config(rt_launch_config c, bool mixed) {

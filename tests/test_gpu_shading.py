@@ -533,3 +533,46 @@ def test_headline_image_with_the_sky_matches_oracle_sample(tracer, sky_sampler):
     _sky_check(got, want, "headline 2048^2 sample", MIXED_CONT_BAR, 1e-2)
     sky_seen = (cont["fate"] == O.ESCAPED)
     assert sky_seen.mean() > 0.5
+
+
+TORUS = dict(spin=0.9, r_obs=50.0, incl_deg=75.0, fov_deg=40.0)
+
+
+def _torus_frame(tracer, cam, tile=False):
+    sh = relsim.shading(hydro_model=2, tonemapping_mode=1, torus_inner_radius=6.0, torus_center_radius=10.0)
+    return _shaded(tracer, sh, lambda: tracer.dispatch(cam, fields=["status", "steps_accepted", "steps_rejected"],
+                                                       pixels=True, tile=tile))
+
+
+@pytest.mark.parametrize("width,height", [(1, 1), (33, 5), (64, 36)])
+def test_torus_rays_that_run_out_of_pages(tracer, width, height):
+    """A far escape radius gives most rays more steps than the pool of step
+    points holds, so they are traced again with the torus gathered step by
+    step.  No step beyond the torus adds light and the steps up to there do not
+    depend on the escape radius: the same light, to float rounding, as the
+    frame whose points all fit; and the launch counts each ray's steps once."""
+    near = _torus_frame(tracer, relsim.make_camera(width=width, height=height, **TORUS))
+    far = _torus_frame(tracer, relsim.make_camera(width=width, height=height, escape_radius=1e13, **TORUS))
+    st = tracer.stats()
+    np.testing.assert_array_equal(near["status"], far["status"])
+    np.testing.assert_allclose(_rgb(far["pixels"]), _rgb(near["pixels"]), rtol=0, atol=1e-6)
+    assert st.rays == width * height
+    assert st.accepted == far["steps_accepted"].astype(np.int64).sum()
+    assert st.attempts == st.accepted + far["steps_rejected"].astype(np.int64).sum()
+    if width * height > 1000:
+        assert far["steps_accepted"].mean() > 5 * 64 + 32, "the pool of five pages a ray should run out"
+
+
+def test_torus_frame_in_parts(tracer):
+    """A frame of more rays than one pool of step points serves is traced in
+    parts; its rows across the parts' border are those of a small frame's own
+    launch."""
+    kw = dict(width=1024, height=560, **TORUS)  # 573,440 rays; a part holds 520,000
+    frame = _torus_frame(tracer, relsim.make_camera(**kw))
+    cam = relsim.make_camera(**kw)
+    cam.tile_origin_x, cam.tile_origin_y, cam.tile_extent_x, cam.tile_extent_y = 0, 500, 1024, 16
+    rows = _torus_frame(tracer, cam, tile=True)
+    n = slice(500 * 1024, 516 * 1024)
+    for f in ("status", "steps_accepted", "steps_rejected"):
+        np.testing.assert_array_equal(frame[f][n], rows[f])
+    np.testing.assert_array_equal(_rgb(frame["pixels"][n]), _rgb(rows["pixels"]))
