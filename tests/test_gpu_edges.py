@@ -164,3 +164,18 @@ def test_attempts_outside_the_fast_range(tracer, precision):
         w = x @ x - 0.25
         r = np.sqrt(0.5 * (w + np.sqrt(w * w + x[2] ** 2)))
         assert abs(out["r"][i] / m / r - 1.0) < 1e-9, (i, out["r"][i] / m, r)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (61, 67), (256, 256)])
+def test_small_readback_matches_the_fields_own_copies(tracer, w, h):
+    """Outputs of up to 4 MB come back in one copy: each field asked for alone
+    (always that way here), all of them with the pixels (a copy per field at
+    256^2) and the pixels alone hold the same bytes."""
+    tracer.set_launch_config()
+    cam = config_cam("c2", width=w, height=h)
+    both = tracer.dispatch(cam)
+    for name in both:
+        pix = name == "pixels"
+        alone = tracer.dispatch(cam, fields=[] if pix else [name], pixels=pix)
+        assert list(alone) == [name]
+        assert alone[name].tobytes() == both[name].tobytes(), name
