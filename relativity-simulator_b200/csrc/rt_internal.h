@@ -142,8 +142,8 @@ constexpr uint32_t kPathPoints = 64, kPathPageDoubles = 3 * kPathPoints + 1, kPa
 constexpr size_t kPathCursorBytes = 5 * sizeof(uint32_t);
 struct PathOut {
     double* pages;       // [capacity][kPathPageDoubles]
-    uint32_t* first;     // per output element: the ray's first page
-    uint32_t* points;    // per output element: points stored; kPathOverflow: the pages ran out
+    uint32_t* first;     // per ray of the launch: its first page
+    uint32_t* points;    // per ray of the launch: points stored; kPathOverflow: the pages ran out
     uint32_t* cursor;    // [0] next free page, [1] rays in the overflow queue, [2] and [3] plunging and
                          // other rays placed in `order`, [4] rays in it
     uint32_t* overflow;  // launch indices of rays whose pages ran out

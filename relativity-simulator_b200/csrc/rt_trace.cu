@@ -191,9 +191,10 @@ __device__ __noinline__ void fp64_stages_special(double* __restrict__ io, double
 // steps are off the counters.
 constexpr int kPathGap = 1 << 30;  // in S.rit: steps were left out since the last point
 template <class ColdT>
-__device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, int tid, uint64_t ray, uint64_t o,
+__device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, int tid, uint64_t ray,
                                                uint32_t acc, uint32_t rej, const double* x) {
     const PathOut& P = args.path;
+    const uint64_t local = S.local[tid];
     uint32_t k = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
     double* page = P.pages + static_cast<uint64_t>(S.side[tid]) * kPathPageDoubles;
     for (int i = (S.rit[tid] & kPathGap) ? 0 : 2; i < 3; ++i, ++k) {  // gap, start, end
@@ -201,7 +202,7 @@ __device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, 
         if (slot == 0) {
             const uint32_t next = atomicAdd(P.cursor, 1u);
             if (next >= P.capacity) {
-                P.points[o] = kPathOverflow;
+                P.points[local] = kPathOverflow;
                 P.overflow[atomicAdd(P.cursor + 1, 1u)] = static_cast<uint32_t>(ray);
                 const unsigned long long att = static_cast<unsigned long long>(acc) + rej;
                 atomicAdd(args.stats + ST_ATTEMPTS, 0ull - att);
@@ -210,7 +211,7 @@ __device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, 
                 atomicAdd(args.stats + ST_RHS, 0ull - (6 * att + 1));
                 return false;
             }
-            if (k == 0) P.first[o] = next;
+            if (k == 0) P.first[local] = next;
             else page[3 * kPathPoints] = static_cast<double>(next);
             S.side[tid] = static_cast<int>(next);
             page = P.pages + static_cast<uint64_t>(next) * kPathPageDoubles;
@@ -390,9 +391,9 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                     } else {
                         end_ray<(CONT != 0)>(args, Be, S, tid, n_cross, cls, flags, acc, rej, wind, target, h, xch);
                         if constexpr (CONT == 3) {
-                            const uint64_t o = Be->out_offset + S.local[tid];
-                            args.path.points[o] = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
-                            args.cont.lz[o] = S.lz0[tid];
+                            const uint64_t local = S.local[tid];
+                            args.path.points[local] = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
+                            args.cont.lz[Be->out_offset + local] = S.lz0[tid];
                         }
                     }
                     mode = MODE_IDLE;
@@ -885,7 +886,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                 S.rit[tid] |= kPathGap;
             } else {
                 const double ends[6] = {y[0], y[1], y[2], y5[0], y5[1], y5[2]};
-                if (!store_path_points(args, S, tid, ray, Bp->out_offset + S.local[tid], acc, rej, ends)) {
+                if (!store_path_points(args, S, tid, ray, acc, rej, ends)) {
                     mode = MODE_IDLE;  // out of pages: traced again from the start
                     continue;
                 }
@@ -1422,15 +1423,16 @@ __global__ void __launch_bounds__(kSampleBlock) torus_sample_kernel(const __grid
     const BundleDesc& B = args.one;
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kSampleBlock + threadIdx.x;
     if (i >= args.total_rays) return;
-    const uint64_t o = B.out_offset + args.path.order[i];
-    const uint32_t points = args.path.points[o];
+    const uint32_t local = args.path.order[i];
+    const uint64_t o = B.out_offset + local;
+    const uint32_t points = args.path.points[local];
     if (points == kPathOverflow || points == 0) return;
     double x[3], from[3], V[VL_COUNT] = {};
 #pragma unroll
     for (int c = 0; c < 3; ++c) x[c] = B.x0[c];
     bl_cartesian(x, B.a, from);
     const double lz = args.cont.lz[o];
-    const double* page = args.path.pages + static_cast<uint64_t>(args.path.first[o]) * kPathPageDoubles;
+    const double* page = args.path.pages + static_cast<uint64_t>(args.path.first[local]) * kPathPageDoubles;
     bool gap = false;
     for (uint32_t k = 0, slot = 0; k < points; ++k, ++slot) {
         if (slot == kPathPoints) {

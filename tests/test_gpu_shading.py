@@ -576,3 +576,15 @@ def test_torus_frame_in_parts(tracer):
     for f in ("status", "steps_accepted", "steps_rejected"):
         np.testing.assert_array_equal(frame[f][n], rows[f])
     np.testing.assert_array_equal(_rgb(frame["pixels"][n]), _rgb(rows["pixels"]))
+
+
+def test_torus_frame_in_bands(tracer):
+    """A window of more than 2^24 rays is dispatched in bands, whose outputs
+    begin where the last band's ended: the last row, a band of its own, is that
+    of a one-row dispatch."""
+    kw = dict(width=16384, height=1025, **TORUS)
+    frame = _torus_frame(tracer, relsim.make_camera(**kw))
+    row = _torus_frame(tracer, relsim.make_camera(row_offset=1024, row_count=1, **kw))
+    for f in ("status", "steps_accepted"):
+        np.testing.assert_array_equal(frame[f][-16384:], row[f])
+    np.testing.assert_array_equal(_rgb(frame["pixels"][-16384:]), _rgb(row["pixels"]))
