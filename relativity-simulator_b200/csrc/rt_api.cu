@@ -237,7 +237,7 @@ rt_status launch_two_pass(rt_handle* h, uint32_t n_bundles, uint64_t total, cons
 // points (1.5 KB) a page, five pages a ray at rtol 1e-10 (an edge-on frame of a hole of
 // spin 0.998 uses three), more at a tighter tolerance or step cap, at most 4 GB.  False:
 // the pool could not be had, or the parts would be so small that each is bound by its
-// longest ray (10 ms; a part of 2^17 rays traces as long).
+// longest ray (10 ms at spin 0.998; a part of 2^17 rays traces as long).
 constexpr uint64_t kMaxPathPages = 2'600'000, kMinPathPart = 1u << 17;
 bool reserve_path(rt_handle* h, uint64_t total, PathOut& path, uint64_t& part) {
     const BundleDesc& b = h->host_bundles[0];

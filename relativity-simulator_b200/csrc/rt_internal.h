@@ -138,14 +138,17 @@ enum TracePass : int { PASS_SINGLE = 0, PASS_FAR = 1, PASS_NEAR = 2 };
 // a chain of pages, each kPathPoints Kerr-Schild points and the index of the next page.
 // Steps inside the torus's inner bound are left out; a point whose x is NaN stands for
 // them, and the chain goes on with the start of the next step.
-constexpr uint32_t kPathPoints = 64, kPathPageDoubles = 3 * kPathPoints + 1, kPathOverflow = 0xffffffffu;
-constexpr size_t kPathCursorBytes = 5 * sizeof(uint32_t);
+constexpr uint32_t kPathPoints = 64, kPathPageDoubles = 3 * kPathPoints + 1, kPathOpen = 0xffffffffu;
+// Counters of a torus-shaded trace: the next free page, rays in the overflow queue,
+// plunging and other rays placed in the order (two in a row), rays in it, rays of it the
+// trace's idle warps have come to, and those warps.
+enum PathCursor : int { PC_PAGE = 0, PC_OVERFLOW, PC_PLUNGING, PC_OTHER, PC_TOTAL, PC_SAMPLED, PC_IDLE_WARPS, PC_COUNT };
+constexpr size_t kPathCursorBytes = PC_COUNT * sizeof(uint32_t);
 struct PathOut {
     double* pages;       // [capacity][kPathPageDoubles]
     uint32_t* first;     // per ray of the launch: its first page
-    uint32_t* points;    // per ray of the launch: points stored; kPathOverflow: the pages ran out
-    uint32_t* cursor;    // [0] next free page, [1] rays in the overflow queue, [2] and [3] plunging and
-                         // other rays placed in `order`, [4] rays in it
+    uint32_t* points;    // per ray of the launch: points stored; kPathOpen: not ended, or the pages ran out
+    uint32_t* cursor;    // PathCursor
     uint32_t* overflow;  // launch indices of rays whose pages ran out
     uint32_t* order;     // launch indices, the rays that plunge into the hole first
     uint32_t capacity;   // pages

@@ -224,6 +224,8 @@ constexpr double kMinThroughputVol = 0.01;  // the reference's loop condition (t
 // A ray gathers nothing once its throughput is 0.01 or less (the reference's
 // loop ends there).
 //
+// fm_chord is one chord's light by itself, fm_add its share of the ray's.
+//
 // What bounds it is FP64 arithmetic per sample.  A sample as the reference writes it
 // takes acos, two sin and cos, two log and two exp of the potential, two pow and the
 // 33-node colour, about 3,000 FP64 instructions.  Here sin^2 and cos^2 come from the
@@ -231,23 +233,26 @@ constexpr double kMinThroughputVol = 0.01;  // the reference's loop condition (t
 // the two positive bases exp(y log x): about 350, and the divisions and roots that
 // are left are the straight-line forms.
 // Measured, a 640x360 frame with the torus: 68.1 ms before, 32.7 gathered as the
-// tracer goes, 17.0 in a pass of its own (torus_sample_kernel).
-__device__ __forceinline__ void fm_chord(const ShadeDesc& D, const double* from, const double* to, double l_over_e,
-                                         double* V) {
-    if (!D.fm_valid) return;
-    const bool seen = V[VL_HIT] != 0.0;
-    if (seen && !(V[VL_THR] > kMinThroughputVol)) return;
+// tracer goes, 13.6 from the steps' stored points (sample_paths).
+struct ChordLight {
+    double rad[3], opacity, z;
+};
+
+// The chord's own light; false: none (an opacity of 1e-6 or less).
+__device__ __forceinline__ bool fm_chord(const ShadeDesc& D, const double* from, const double* to, double l_over_e,
+                                         ChordLight& out) {
+    if (!D.fm_valid) return false;
     const double dx = to[0] - from[0], dy = to[1] - from[1], dz = to[2] - from[2];
     const double len2 = dx * dx + dy * dy + dz * dz;
-    if (len2 < 1e-24) return;
+    if (len2 < 1e-24) return false;
     const double len = sqrt(len2);
     const double b = (from[0] * dx + from[1] * dy + from[2] * dz) / len2;
     const double c = (from[0] * from[0] + from[1] * from[1] + from[2] * from[2] - D.fm_outer * D.fm_outer) / len2;
     const double disc = b * b - c;
-    if (disc <= 0.0) return;
+    if (disc <= 0.0) return false;
     const double root = sqrt(disc);
     const double t0 = cd(-b - root, 0.0, 1.0), t1 = cd(-b + root, 0.0, 1.0);
-    if (t1 <= t0) return;
+    if (t1 <= t0) return false;
     const double clipped = len * (t1 - t0);
     const double m = D.fm_m;
     int count = static_cast<int>(ceil(clipped * D.fm_density / m));
@@ -304,21 +309,32 @@ __device__ __forceinline__ void fm_chord(const ShadeDesc& D, const double* from,
         trans *= st;
         if (trans < 0.002) break;
     }
-    const double opacity = 1.0 - trans;
-    if (opacity <= 1e-6) return;
-    const double thr = seen ? V[VL_THR] : 1.0;
-    V[VL_R] += thr * rad[0];
-    V[VL_G] += thr * rad[1];
-    V[VL_B] += thr * rad[2];
-    V[VL_THR] = thr * (1.0 - opacity);
-    V[VL_Z] = (wsum > 1e-30) ? (zsum / wsum) : 1.0;
+    out.opacity = 1.0 - trans;
+    if (out.opacity <= 1e-6) return false;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out.rad[c] = rad[c];
+    out.z = (wsum > 1e-30) ? (zsum / wsum) : 1.0;
+    return true;
+}
+
+// Whether a ray's throughput still lets it gather.
+__device__ __forceinline__ bool fm_open(const double* V) { return V[VL_HIT] == 0.0 || V[VL_THR] > kMinThroughputVol; }
+
+__device__ __forceinline__ void fm_add(const ChordLight& c, double* V) {
+    const double thr = (V[VL_HIT] != 0.0) ? V[VL_THR] : 1.0;
+    V[VL_R] += thr * c.rad[0];
+    V[VL_G] += thr * c.rad[1];
+    V[VL_B] += thr * c.rad[2];
+    V[VL_THR] = thr * (1.0 - c.opacity);
+    V[VL_Z] = c.z;
     V[VL_HIT] = 1.0;
 }
 
 // The chord within a tracer's step loop (the tracers that gather as they go).
 __device__ __noinline__ void fm_segment(const ShadeDesc& D, const double* from, const double* to, double l_over_e,
                                         double* V) {
-    fm_chord(D, from, to, l_over_e, V);
+    ChordLight c;
+    if (fm_open(V) && fm_chord(D, from, to, l_over_e, c)) fm_add(c, V);
 }
 
 // ---- translucent-disk continuation ----

@@ -200,10 +200,9 @@ __device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, 
     for (int i = (S.rit[tid] & kPathGap) ? 0 : 2; i < 3; ++i, ++k) {  // gap, start, end
         const uint32_t slot = k % kPathPoints;
         if (slot == 0) {
-            const uint32_t next = atomicAdd(P.cursor, 1u);
+            const uint32_t next = atomicAdd(P.cursor + PC_PAGE, 1u);
             if (next >= P.capacity) {
-                P.points[local] = kPathOverflow;
-                P.overflow[atomicAdd(P.cursor + 1, 1u)] = static_cast<uint32_t>(ray);
+                P.overflow[atomicAdd(P.cursor + PC_OVERFLOW, 1u)] = static_cast<uint32_t>(ray);
                 const unsigned long long att = static_cast<unsigned long long>(acc) + rej;
                 atomicAdd(args.stats + ST_ATTEMPTS, 0ull - att);
                 atomicAdd(args.stats + ST_FP64_ATTEMPTS, 0ull - att);
@@ -223,6 +222,105 @@ __device__ __noinline__ bool store_path_points(const TraceArgs& args, ColdT& S, 
     }
     S.rit[tid] = static_cast<int>(k);
     return true;
+}
+
+// The light of four rays of a torus-shaded trace by one warp (local: this lane's ray,
+// the same in the eight lanes of its group; points 0: none).  A group walks its ray's
+// chain eight points at a time, one chord to a lane (fm_chord), and adds the chords'
+// light in the order of the steps.  Gathering inside the step loop ran two large pieces
+// of code in turn on every warp, each evicting the other from the instruction cache
+// (no_instruction 3.5 of 9.6 cycles per issue, FP64 pipe 26 %); one lane to a ray left
+// the pass to the few rays along the equatorial plane (4.5 ms at 640x360, the SMs idle
+// for two thirds of it).  Measured, gathering as it goes / a pass after the trace, one
+// lane to a ray / eight lanes, idle warps of the trace first: 64x36 14.6 / 10.1 / 3.0 ms,
+// 640x360 32.7 / 17.3 / 13.6, 1920x1080 159 / 76 / 67.  Sixteen lanes: the same, 77.
+constexpr int kPathLanes = 8;
+__device__ __forceinline__ void sample_paths(const TraceArgs& args, uint32_t local, uint32_t points) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const BundleDesc& B = args.one;
+    const int sub = threadIdx.x % kPathLanes;
+    const uint64_t o = B.out_offset + local;
+    double x[3], last[3], V[VL_COUNT] = {}, lz = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[c] = B.x0[c];
+    bl_cartesian(x, B.a, last);  // the end of the group's last chord
+    const double* page = args.path.pages;
+    if (points) {
+        lz = args.cont.lz[o];
+        page += static_cast<uint64_t>(args.path.first[local]) * kPathPageDoubles;
+    }
+    bool open = points != 0;
+    for (uint32_t k = 0; __any_sync(FULL, open); k += kPathLanes) {
+        const uint32_t slot = k % kPathPoints;
+        double to[3], from[3];
+        bool live = open && k + sub < points;
+        if (open && slot == 0 && k)
+            page = args.path.pages + static_cast<uint64_t>(page[3 * kPathPoints]) * kPathPageDoubles;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = live ? page[3 * (slot + sub) + c] : 1.0;
+        bl_cartesian(x, B.a, to);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double before = __shfl_up_sync(FULL, to[c], 1, kPathLanes);
+            from[c] = sub ? before : last[c];
+            last[c] = __shfl_sync(FULL, to[c], kPathLanes - 1, kPathLanes);
+        }
+        live = live && to[0] == to[0] && from[0] == from[0];  // not beside a gap
+        ChordLight light;
+        const bool lit = live && fm_chord(*args.cont.shade, from, to, lz, light);
+        const unsigned any = __ballot_sync(FULL, lit);
+        unsigned mine = (any >> (threadIdx.x % 32 - sub)) & ((1u << kPathLanes) - 1u);
+        while (__any_sync(FULL, mine != 0u)) {
+            const int j = mine ? __ffs(mine) - 1 : 0;
+            ChordLight c;
+#pragma unroll
+            for (int f = 0; f < 3; ++f) c.rad[f] = __shfl_sync(FULL, light.rad[f], j, kPathLanes);
+            c.opacity = __shfl_sync(FULL, light.opacity, j, kPathLanes);
+            c.z = __shfl_sync(FULL, light.z, j, kPathLanes);
+            if (mine && open) {
+                fm_add(c, V);
+                open = fm_open(V);
+            }
+            mine &= mine - 1u;
+        }
+        open = open && k + kPathLanes < points;
+    }
+    if (points && sub < VL_COUNT) {
+        double v = V[0];
+#pragma unroll
+        for (int f = 1; f < VL_COUNT; ++f) v = (sub == f) ? V[f] : v;
+        args.cont.vol[o * VL_COUNT + sub] = v;
+    }
+}
+
+// A warp of a torus-shaded trace that finds no more rays: while others still trace, it
+// samples the rays that have ended, four of the launch's order at a time.  Nothing is
+// waited for: a ray that has not ended when its turn comes is left to the sampling pass,
+// and so is all the rest once the last warp's rays have ended.
+__device__ __noinline__ void sample_ended_paths(const TraceArgs& args) {
+    const PathOut& P = args.path;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = static_cast<uint32_t>(args.total_rays), warps = gridDim.x * (blockDim.x / 32u);
+    if (lane == 0) atomicAdd(P.cursor + PC_IDLE_WARPS, 1u);
+    for (;;) {
+        uint32_t at = total;
+        if (lane == 0 && *static_cast<volatile uint32_t*>(P.cursor + PC_IDLE_WARPS) < warps)
+            at = atomicAdd(P.cursor + PC_SAMPLED, 32u / kPathLanes);
+        at = __shfl_sync(~0u, at, 0);
+        if (at >= total) return;
+        const uint32_t i = at + lane / kPathLanes;
+        uint32_t local = 0, points = 0;
+        if (i < total) {
+            local = P.order[i];
+            if (lane % kPathLanes == 0) points = *static_cast<volatile uint32_t*>(P.points + local);
+        }
+        points = __shfl_sync(~0u, points, 0, kPathLanes);
+        if (points == kPathOpen) points = 0;
+        __threadfence();  // the chain was stored before its length
+        sample_paths(args, local, points);
+        if (points && lane % kPathLanes == 0) P.points[local] = 0;  // gathered
+        __syncwarp();
+    }
 }
 
 // WARPS resident warps per SM set the registers per thread: 8 warps at up to 255
@@ -392,8 +490,10 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                         end_ray<(CONT != 0)>(args, Be, S, tid, n_cross, cls, flags, acc, rej, wind, target, h, xch);
                         if constexpr (CONT == 3) {
                             const uint64_t local = S.local[tid];
-                            args.path.points[local] = static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
                             args.cont.lz[Be->out_offset + local] = S.lz0[tid];
+                            __threadfence();  // the chain before its length
+                            *static_cast<volatile uint32_t*>(args.path.points + local) =
+                                static_cast<uint32_t>(S.rit[tid] & ~kPathGap);
                         }
                     }
                     mode = MODE_IDLE;
@@ -937,12 +1037,14 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
         atomicAdd(args.stats + ST_RHS, w_rhs);
         if (w_att != w_far) atomicAdd(args.stats + ST_FP64_ATTEMPTS, w_att - w_far);
     }
+    if constexpr (CONT == 3) sample_ended_paths(args);
 }
 
-// The trace of a torus-shaded frame is bound by its longest rays' chains of steps (3,700
-// where the mean is 320), so the lean form: 640x360 17.0 ms at 8 warps per SM, 18.0 at
-// 12; 1920x1080 83.6 / 81.2.
-constexpr int kTorusWarps = 8;
+// The trace of a small torus-shaded frame is bound by its longest rays' chains of steps
+// (3,700 where the mean is 320): 8 warps per SM, whose steps take less time.  A large one
+// is bound by throughput: 12.  Measured at 8 / 12: 64x36 3.0 / 3.2 ms, 213x119 4.2 / 4.5,
+// 640x360 at spin 0.998 13.6 / 14.6 and at 0.9 9.9 / 9.0, 1920x1080 72.2 / 67.2.
+constexpr uint64_t kTorusLeanRaysPerSm = 2048;
 constexpr uint32_t kSampleBlock = 64;
 
 // unshaded launches (CONT = 0), shaded ones that follow rays through the
@@ -981,7 +1083,8 @@ template __global__ void trace_kernel_t<128, false, true, PASS_SINGLE, 1>(const 
 template __global__ void trace_kernel_t<64, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, true, true, PASS_SINGLE, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 2>(const __grid_constant__ TraceArgs);
-template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 3, kTorusWarps>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 3, 8>(const __grid_constant__ TraceArgs);
+template __global__ void trace_kernel_t<128, false, false, PASS_SINGLE, 3, 12>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<64, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, true, false, PASS_FAR, 1>(const __grid_constant__ TraceArgs);
 template __global__ void trace_kernel_t<128, false, false, PASS_NEAR, 1>(const __grid_constant__ TraceArgs);
@@ -1400,7 +1503,7 @@ __global__ void __launch_bounds__(128) torus_order_kernel(const __grid_constant_
     uint32_t at = 0;
     if (lane < 2) {
         const uint32_t n = static_cast<uint32_t>(__popc(lane == 0 ? first : rest));
-        if (n) at = atomicAdd(args.path.cursor + 2 + lane, n);
+        if (n) at = atomicAdd(args.path.cursor + PC_PLUNGING + lane, n);
     }
     const uint32_t at_first = __shfl_sync(~0u, at, 0), at_rest = __shfl_sync(~0u, at, 1);
     const unsigned below = (1u << lane) - 1u;
@@ -1409,55 +1512,19 @@ __global__ void __launch_bounds__(128) torus_order_kernel(const __grid_constant_
         const uint32_t to = plunges ? at_first + __popc(first & below) : total - 1u - (at_rest + __popc(rest & below));
         args.path.order[to] = static_cast<uint32_t>(args.ray_base + i);
     }
-    if (i == 0) args.path.cursor[4] = total;
+    if (i == 0) args.path.cursor[PC_TOTAL] = total;
 }
 
-// The sampling pass of a torus-shaded trace: one thread per ray walks its chain of
-// points and gathers the light of each chord (fm_chord), in the order of the steps.
-// Gathering inside the step loop ran two large pieces of code in turn on every warp,
-// each evicting the other from the instruction cache (no_instruction 3.5 of 9.6 cycles
-// per issue, FP64 pipe 26 %).  Measured, 640x360, gathering as it goes / in this pass:
-// 32.7 / 17.0 ms (trace 12.5, this pass 4.5, bound by the few rays that run along the
-// equatorial plane), 1920x1080 159 / 84, 64x36 14.6 / 10.1.
+// The sampling pass of a torus-shaded trace: what the trace's idle warps left of it.
 __global__ void __launch_bounds__(kSampleBlock) torus_sample_kernel(const __grid_constant__ TraceArgs args) {
-    const BundleDesc& B = args.one;
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kSampleBlock + threadIdx.x;
-    if (i >= args.total_rays) return;
-    const uint32_t local = args.path.order[i];
-    const uint64_t o = B.out_offset + local;
-    const uint32_t points = args.path.points[local];
-    if (points == kPathOverflow || points == 0) return;
-    double x[3], from[3], V[VL_COUNT] = {};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) x[c] = B.x0[c];
-    bl_cartesian(x, B.a, from);
-    const double lz = args.cont.lz[o];
-    const double* page = args.path.pages + static_cast<uint64_t>(args.path.first[local]) * kPathPageDoubles;
-    bool gap = false;
-    for (uint32_t k = 0, slot = 0; k < points; ++k, ++slot) {
-        if (slot == kPathPoints) {
-            page = args.path.pages + static_cast<uint64_t>(page[3 * kPathPoints]) * kPathPageDoubles;
-            slot = 0;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) x[c] = page[3 * slot + c];
-        if (x[0] != x[0]) {
-            gap = true;
-            continue;
-        }
-        double to[3];
-        bl_cartesian(x, B.a, to);
-        if (!gap) {
-            fm_chord(*args.cont.shade, from, to, lz, V);
-            if (V[VL_HIT] != 0.0 && !(V[VL_THR] > kMinThroughputVol)) break;
-        }
-        gap = false;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) from[c] = to[c];
+    const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * kSampleBlock + threadIdx.x) / kPathLanes;
+    uint32_t local = 0, points = 0;
+    if (i < args.total_rays) {
+        local = args.path.order[i];
+        points = args.path.points[local];
+        if (points == kPathOpen) points = 0;
     }
-    double* out = args.cont.vol + o * VL_COUNT;
-#pragma unroll
-    for (int f = 0; f < VL_COUNT; ++f) out[f] = V[f];
+    if (__any_sync(0xffffffffu, points != 0)) sample_paths(args, local, points);
 }
 
 int enqueue_torus(const TraceArgs& base, int sm_count, uint32_t ctas_per_sm, char* claims, void* stream) {
@@ -1465,24 +1532,28 @@ int enqueue_torus(const TraceArgs& base, int sm_count, uint32_t ctas_per_sm, cha
     TraceArgs args = base;
     cudaError_t e = cudaMemsetAsync(claims, 0, 72, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(args.path.cursor, 0, kPathCursorBytes, s);
+    if (e == cudaSuccess)  // no ray has ended
+        e = cudaMemsetAsync(args.path.points + args.ray_base, 0xff, sizeof(uint32_t) * args.total_rays, s);
     if (e != cudaSuccess) return static_cast<int>(e);
     torus_order_kernel<<<static_cast<uint32_t>((args.total_rays + 127) / 128), 128, 0, s>>>(args);
     if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
     args.queue = reinterpret_cast<unsigned long long*>(claims);
     args.in_queue = args.path.order;
-    args.in_count = args.path.cursor + 4;
+    args.in_count = args.path.cursor + PC_TOTAL;
     void* params[] = {&args};
-    cudaLaunchKernel(reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, kTorusWarps>),
-                     dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, kTorusWarps / 4u)), dim3(128), params,
-                     0, s);
+    const bool lean = args.total_rays <= kTorusLeanRaysPerSm * static_cast<uint64_t>(sm_count);
+    cudaLaunchKernel(lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, 8>)
+                          : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, 12>),
+                     dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, lean ? 2u : 3u)), dim3(128), params, 0,
+                     s);
     if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
-    torus_sample_kernel<<<static_cast<uint32_t>((args.total_rays + kSampleBlock - 1) / kSampleBlock), kSampleBlock, 0,
+    torus_sample_kernel<<<static_cast<uint32_t>((args.total_rays * kPathLanes + kSampleBlock - 1) / kSampleBlock), kSampleBlock, 0,
                           s>>>(args);
     if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
     // the rays whose pages ran out
     args.queue = reinterpret_cast<unsigned long long*>(claims + 64);
     args.in_queue = args.path.overflow;
-    args.in_count = args.path.cursor + 1;
+    args.in_count = args.path.cursor + PC_OVERFLOW;
     cudaLaunchKernel(reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 2>),
                      dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, 3u)), dim3(128), params, 0, s);
     return static_cast<int>(cudaGetLastError());
