@@ -705,6 +705,8 @@ rt_status bl_launch(rt_handle* h, const rt_camera* cam, uint32_t col0, uint32_t 
     BlArgs args{};
     args.bundles = static_cast<const BlDesc*>(h->bl_desc.ptr);
     args.n_bundles = 1;
+    args.one = d;
+    args.has_one = 1;
     args.fast_range = (d.flags & BF_FAST_RANGE) ? 1u : 0u;
     args.refill_threshold = c.refill_threshold;
     args.claim = 32u * c.rays_per_thread;
@@ -760,6 +762,8 @@ rt_status launch_banded_single(rt_handle* h, const rt_camera* cam, uint32_t col0
             BlArgs args{};
             args.bundles = reinterpret_cast<const BlDesc*>(dd);
             args.n_bundles = 1;
+            args.one = d;
+            args.has_one = 1;
             args.fast_range = (d.flags & BF_FAST_RANGE) ? 1u : 0u;
             args.refill_threshold = c.refill_threshold;
             args.claim = 32u * c.rays_per_thread;

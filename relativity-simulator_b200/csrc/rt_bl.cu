@@ -441,8 +441,11 @@ __device__ __noinline__ void bl_finish(const BlDesc* __restrict__ Bp, BlCold<BLO
 // FAST: the straight-line reciprocal of the step's right-hand sides, the same values
 // without a special-case test and branch in each (1024^2 Kerr-Newman image 22.7 / 22.0
 // ms); every camera of the launch has BF_FAST_RANGE.
-template <int BLOCK, bool VOL, bool FAST>
-__global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs args) {
+// ONE: one camera, its constants read as kernel parameters (BlArgs::one) instead of
+// loads each step waits for (1024^2 Kerr-Newman image 22.05 / 21.44 ms).
+template <int BLOCK, bool VOL, bool FAST, bool ONE>
+__global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(const __grid_constant__ BlArgs args) {
+    const auto bundle = [&](uint32_t i) -> const BlDesc* { return ONE ? &args.one : args.bundles + i; };
     __shared__ BlCold<BLOCK> S;
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x;
@@ -482,7 +485,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
             if (ended && (n_free == 32 || ((queue_open || chunk_next < chunk_end) &&
                                            n_free >= static_cast<int>(args.refill_threshold)))) {
                 if (mode == BL_ENDED) {
-                    const BlDesc* Bp = args.bundles + bidx;
+                    const BlDesc* Bp = bundle(bidx);
                     const BlDesc& B = *Bp;
                     const uint32_t cls = end_kind & 15u, todo = end_kind & ~15u;
                     double yt[NB], r_hit = NAN, g = 1.0;
@@ -564,13 +567,13 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
                 if (rank < avail) rid = chunk_next + rank;
                 else if (got2) rid = base2 + (rank - avail);
                 if (rid < args.total_rays) {
-                    uint32_t lo = 0, hi = args.n_bundles;
+                    uint32_t lo = 0, hi = ONE ? 1u : args.n_bundles;
                     while (hi - lo > 1) {
                         const uint32_t mid = (lo + hi) >> 1;
                         if (args.bundles[mid].ray_begin <= rid) lo = mid; else hi = mid;
                     }
                     bidx = lo;
-                    const BlDesc* Bp = args.bundles + lo;
+                    const BlDesc* Bp = bundle(lo);
                     bl_init_ray<BLOCK>(Bp, rid - Bp->ray_begin, S, tid, y);
                     bl_rhs(Bp->m, Bp->a, Bp->q2, y, k1);
                     h = -Bp->h0;
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
         }
         if (mode == BL_IDLE || mode == BL_ENDED) continue;
 
-        const BlDesc* Bp = args.bundles + bidx;
+        const BlDesc* Bp = bundle(bidx);
         const BlDesc& B = *Bp;
         // termination before the attempt; a backstop on loop iterations per ray
         uint32_t term = 0;
@@ -785,16 +788,18 @@ __global__ void __launch_bounds__(BLOCK, 384 / BLOCK) bl_trace_kernel(BlArgs arg
     }
 }
 
-template __global__ void bl_trace_kernel<128, false, false>(BlArgs);
-template __global__ void bl_trace_kernel<128, false, true>(BlArgs);
-template __global__ void bl_trace_kernel<128, true, false>(BlArgs);
-template __global__ void bl_trace_kernel<128, true, true>(BlArgs);
+template __global__ void bl_trace_kernel<128, false, false, false>(const __grid_constant__ BlArgs);
+template __global__ void bl_trace_kernel<128, false, true, false>(const __grid_constant__ BlArgs);
+template __global__ void bl_trace_kernel<128, false, true, true>(const __grid_constant__ BlArgs);
+template __global__ void bl_trace_kernel<128, true, false, false>(const __grid_constant__ BlArgs);
+template __global__ void bl_trace_kernel<128, true, true, false>(const __grid_constant__ BlArgs);
+template __global__ void bl_trace_kernel<128, true, true, true>(const __grid_constant__ BlArgs);
 
 }  // namespace
 
 uint32_t bl_trace_grid(int sm_count) {
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bl_trace_kernel<128, false, true>, 128, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bl_trace_kernel<128, false, true, true>, 128, 0) != cudaSuccess) {
         cudaGetLastError();
         occ = 1;
     }
@@ -803,13 +808,14 @@ uint32_t bl_trace_grid(int sm_count) {
 
 void launch_bl_trace(const BlArgs& args, uint32_t grid, void* stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (args.cont.vol) {
-        if (args.fast_range) bl_trace_kernel<128, true, true><<<grid, 128, 0, s>>>(args);
-        else bl_trace_kernel<128, true, false><<<grid, 128, 0, s>>>(args);
-    } else {
-        if (args.fast_range) bl_trace_kernel<128, false, true><<<grid, 128, 0, s>>>(args);
-        else bl_trace_kernel<128, false, false><<<grid, 128, 0, s>>>(args);
-    }
+    const bool one = args.fast_range && args.has_one;
+    const auto kernel = args.cont.vol ? (one                 ? bl_trace_kernel<128, true, true, true>
+                                         : args.fast_range ? bl_trace_kernel<128, true, true, false>
+                                                           : bl_trace_kernel<128, true, false, false>)
+                                      : (one                 ? bl_trace_kernel<128, false, true, true>
+                                         : args.fast_range ? bl_trace_kernel<128, false, true, false>
+                                                           : bl_trace_kernel<128, false, false, false>);
+    kernel<<<grid, 128, 0, s>>>(args);
 }
 
 }  // namespace relsim

@@ -261,6 +261,8 @@ struct BlArgs {
     // translucent-disk continuation (shaded dispatches): the crossings' outputs;
     // cross null: off
     ContOut cont;
+    uint32_t has_one, pad;
+    BlDesc one;             // has_one: the launch's only bundle
 };
 
 // Per-camera constants of the pixel shading pass (rt_shade.cu): the resolved

@@ -423,6 +423,10 @@ bool launch_epoch(rt_server* s, Slot& slot) {
         BlArgs ba{};
         ba.bundles = slot.dev_bl;
         ba.n_bundles = nb;
+        if (nb == 1) {
+            ba.one = slot.host_bl[0];
+            ba.has_one = 1;
+        }
         ba.fast_range = 1u;
         for (uint32_t b = 0; b < nb; ++b)
             if (!(slot.host_bl[b].flags & BF_FAST_RANGE)) ba.fast_range = 0u;
