@@ -60,9 +60,10 @@ H2D_BYTES_PER_IMAGE = 464  # one bundle descriptor (per-camera constants) per im
 # stage sums and error norm for the reference's 8-component state
 BL_FLOP_PER_ATTEMPT = 3542.0
 # kernels one device-resident trace of the image launches: the two-pass mixed
-# tracer runs 4 rounds of a far and a near pass and one finish pass (the
+# tracer lists its rays, sorts the near-critical ones (two kernels), runs the
+# critical pass, 4 rounds of a far and a near pass and one finish pass (the
 # library's round count); the single-kernel tracers launch once
-MIXED_TWO_PASS_LAUNCHES = 2 * 4 + 1
+MIXED_TWO_PASS_LAUNCHES = 1 + 2 + 1 + 2 * 4 + 1
 BL_CAMERA = dict(spin=0.9, charge=0.3, r_obs=50.0, incl_deg=75.0, fov_deg=30.0)
 BL_H2D_BYTES_PER_IMAGE = 352  # the Boyer-Lindquist camera descriptor (sizeof BlDesc)
 SHADE_H2D_BYTES = 3248  # the shading pass's per-camera constants with the sky profile and torus (sizeof ShadeDesc)

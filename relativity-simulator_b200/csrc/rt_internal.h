@@ -156,6 +156,9 @@ struct PathOut {
     double skip;         // a step with both ends within this radius crosses no part of the torus
 };
 
+// In the first far pass's list, the place of a near-critical ray.
+constexpr uint32_t kListHole = 0xffffffffu;
+
 // Length classes of near-critical rays, in the upper bits of a queue entry.
 constexpr uint32_t kCritClasses = 32, kCritClassShift = 27;
 
@@ -170,8 +173,8 @@ struct TraceArgs {
     unsigned long long* stats;  // [ST_COUNT]
     OutPtrs out;
     // two-pass mixed tracer (zero for PASS_SINGLE launches)
-    uint64_t ray_base;          // far pass from pixels: launch index of this band's first ray
-    uint32_t from_pixels;       // far pass: rays start at their pixels
+    uint64_t ray_base;          // launch index of this band's or part's first ray
+    uint32_t from_pixels;       // far pass: rays of in_queue start at their pixels
     uint32_t allow_exit;        // near pass: rays leaving the near zone go back to the far pass
     const uint32_t* in_queue;   // launch indices of the rays to resume
     const uint32_t* in_count;
@@ -179,9 +182,6 @@ struct TraceArgs {
     uint32_t* out_count;
     uint32_t* finish_queue;     // disk hits parked with their root point for the finish pass
     uint32_t* finish_count;
-    uint32_t* crit_queue;       // first far pass: near-critical rays, for the critical pass
-    uint32_t* crit_count;
-    uint64_t crit_classes;      // 1: crit_queue entries carry the ray's length class in their upper bits
     PathOut path;               // torus-shaded traces that leave the torus to the sampling pass (else null)
     BundleDesc one;             // has_one: the launch's only bundle, read in place of bundles[0]
     ParkBuf park;
@@ -326,7 +326,7 @@ struct TwoPassBuffers {
     ParkBuf park;       // parked state, n slots
     uint32_t* queues;   // 4n entries: per band near, far, finish and near-critical queues
     char* counters;     // kBandCounterBytes per band (up to kMaxBands): claim counters and queue counts
-    // one band: the critical pass runs on this stream beside the near pass
+    // one band: the critical pass runs on this stream beside the other passes
     // (forked and joined with the two events); null: after it, on the band's
     void* crit_stream = nullptr;
     void* crit_fork = nullptr;

@@ -31,7 +31,6 @@ enum LaneMode : int {
     MODE_REDO = 3,
     MODE_PARK = 4,     // two-pass: to the other pass, state parked
     MODE_FINISHQ = 5,  // two-pass: a disk hit, root point parked for the finish pass
-    MODE_CRITQ = 6,    // far pass: a near-critical ray, to the critical pass (no state)
     MODE_ENDED = 7     // the ray has ended; its record is written when the warp refills
 };
 // end_kind: the record needs the last step's end (y5, k7), or the disk root in its place

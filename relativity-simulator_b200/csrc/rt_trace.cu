@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
     constexpr bool NEAR_PASS = (PASS == PASS_NEAR);
     static_assert(!FAR_PASS || MIXED, "the far pass runs the FP32 stages");
     static_assert(!NEAR_PASS || !MIXED, "the near pass runs FP64 stages");
-    // rays of this launch: pixels (single kernel, first far pass) or queue entries
+    // rays of this launch: pixels (single kernel; the first far pass, but for the holes
+    // of its list) or queue entries
     // (later passes; the single kernel as the critical pass of a two-pass launch)
     auto bundle = [&args](uint32_t i) -> const BundleDesc* {
         if constexpr (ONE) return &args.one;
@@ -442,22 +443,6 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                     mode = MODE_IDLE;
                 }
             }
-            if constexpr (FAR_PASS) {
-                // near-critical rays to the critical pass, before their first step
-                const unsigned cmask = __ballot_sync(FULL, mode == MODE_CRITQ);
-                if (cmask) {
-                    const int leader = __ffs(cmask) - 1;
-                    uint32_t cbase = 0;
-                    if (lane == leader) cbase = atomicAdd(args.crit_count, static_cast<uint32_t>(__popc(cmask)));
-                    cbase = __shfl_sync(FULL, cbase, leader);
-                    if (mode == MODE_CRITQ) {
-                        // n_cross holds the ray's length class until its first crossing
-                        args.crit_queue[cbase + static_cast<uint32_t>(__popc(cmask & lt_mask))] =
-                            static_cast<uint32_t>(ray) | (args.crit_classes ? n_cross << kCritClassShift : 0u);
-                        mode = MODE_IDLE;
-                    }
-                }
-            }
         }
         {
             // ---- the ends waiting in this warp, all together, when it can refill or
@@ -529,13 +514,9 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                 uint64_t rid = ~0ull;
                 if (rank < avail) rid = chunk_next + rank;
                 else if (got2) rid = base2 + (rank - avail);
-                if (rid < total) {
-                    uint64_t rix = rid;
-                    if constexpr (PASS != PASS_SINGLE) {
-                        rix = from_queue ? static_cast<uint64_t>(args.in_queue[rid]) : args.ray_base + rid;
-                    } else {
-                        if (from_queue) rix = args.in_queue[rid];
-                    }
+                uint64_t rix = rid;
+                if (rid < total && (PASS != PASS_SINGLE || from_queue)) rix = args.in_queue[rid];
+                if (rid < total && !(FAR_PASS && rix == kListHole)) {
                     // bundle of this ray: last bundle whose ray_begin <= rix
                     uint32_t lo = 0, hi = ONE ? 1u : args.n_bundles;
                     while (hi - lo > 1) {
@@ -595,22 +576,22 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                         n_cross = 0;
                         critical = false;
                         tol_sc = 1.0f;
-                        // mixed mode: the distance of the ray's constants from the critical
-                        // curve decides whether it is near-critical (and the Carter early
-                        // capture, from the same value); the critical pass grades its
-                        // tolerance with it
-                        if ((MIXED && Bc->critical_band > 0.0f) ||
+                        // the distance of the ray's constants from the critical curve: the
+                        // critical pass grades its tolerance with it; in the single mixed
+                        // kernel it decides whether the ray is near-critical (the two-pass
+                        // tracer's list is sorted out before); the Carter early capture
+                        // takes the same value
+                        if ((MIXED && !FAR_PASS && Bc->critical_band > 0.0f) ||
                             (PASS == PASS_SINGLE && !MIXED && CONT < 2 && from_queue)) {
                             const double db = shadow_distance(Bc->m, Bc->a, 0.0, Bc->rh, S.lz0[tid], S.q0[tid]);
                             if (can_early < 0) can_early = db > kEarlyCaptureMargin;
                             const double band = static_cast<double>(Bc->critical_band) * Bc->m;
                             critical = fabs(db) < band;
-                            if (critical && PASS == PASS_SINGLE) tol_sc = critical_tol_scale(db, band);
-                            if (critical && FAR_PASS) n_cross = critical_class(db, band);
+                            if (critical) tol_sc = critical_tol_scale(db, band);
+                            if (!MIXED) ++n_rhs;  // the list's
                         }
                         mode = MODE_STEP;
-                        // a queue of rays left by a pass that has counted them
-                        if (!(PASS == PASS_SINGLE && from_queue) || CONT == 3) ++n_rays;
+                        if (!(CONT == 2 && from_queue)) ++n_rays;  // else counted by the trace that ran out of pages
                         ++n_rhs;
                     }
                 }
@@ -678,8 +659,8 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                 continue;
             }
             if constexpr (FAR_PASS) {
-                if (critical || r < Bp->fp64_radius || r >= kFp32MaxRadius) {  // into the FP64 zone
-                    mode = critical ? MODE_CRITQ : MODE_PARK;
+                if (r < Bp->fp64_radius || r >= kFp32MaxRadius) {  // into the FP64 zone
+                    mode = MODE_PARK;
                     continue;
                 }
             }
@@ -1232,8 +1213,48 @@ void launch_trace_pass(const TraceArgs& args, int pass, uint32_t grid, uint32_t 
 }
 }  // namespace
 
-// The near-critical queue, sorted by length class.  The far pass lists the rays in the
-// order it meets them; across the critical curve neighbours differ several times over
+// The rays of a two-pass launch's band sorted out before its passes: the near-critical
+// ones to the critical pass's list (with the length class when that list is sorted
+// below), and a list for the first far pass that has a hole in place of each of them,
+// so that its warps keep their neighbours (closed up, in the order of the blocks, the
+// far pass is 2 % faster and the near pass after it 18 % slower).  The critical pass then
+// runs beside the far pass, and a ray is on exactly one list.  Measured, the far pass
+// sorting its rays out as it meets them and the critical pass after it / this: 213x119
+// 1.75 / 1.54 ms, 2048^2 20.1 / 19.2, a table of 40 cameras 35.5 / 34.1, a burst of
+// server requests 19.3 / 17.9.
+__global__ void __launch_bounds__(128) band_list_kernel(const __grid_constant__ TraceArgs args, uint32_t* far_list,
+                                                        uint32_t* crit_list, uint32_t* crit_count, bool classes) {
+    __shared__ Cold<128> S;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * 128 + tid, rix = args.ray_base + i;
+    bool critical = false;
+    uint32_t cls = 0;
+    if (i < args.total_rays) {
+        uint32_t lo = 0, hi = args.has_one ? 1u : args.n_bundles;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (args.bundles[mid].ray_begin <= rix) lo = mid; else hi = mid;
+        }
+        const BundleDesc* B = args.has_one ? &args.one : args.bundles + lo;
+        if (B->critical_band > 0.0f) {
+            double xch[12];
+            init_ray(B, rix - B->ray_begin, S, tid, xch);
+            const double db = shadow_distance(B->m, B->a, 0.0, B->rh, S.lz0[tid], S.q0[tid]);
+            const double band = static_cast<double>(B->critical_band) * B->m;
+            critical = fabs(db) < band;
+            if (critical && classes) cls = critical_class(db, band);
+        }
+        far_list[i] = critical ? kListHole : static_cast<uint32_t>(rix);
+    }
+    const unsigned crit = __ballot_sync(~0u, critical);
+    uint32_t at = 0;
+    if (lane == 0 && crit) at = atomicAdd(crit_count, static_cast<uint32_t>(__popc(crit)));
+    at = __shfl_sync(~0u, at, 0);
+    if (critical) crit_list[at + __popc(crit & ((1u << lane) - 1u))] = static_cast<uint32_t>(rix) | (cls << kCritClassShift);
+}
+
+// The near-critical list, sorted by length class.  It holds the rays in about the order
+// of the launch; across the critical curve neighbours differ several times over
 // in attempts (the tolerance is graded by |d_b|, and the orbits near the photon sphere
 // add to it), so a warp of neighbours runs at 17 to 21 of 32 lanes.  A counting sort
 // into 32 classes (two small launches) puts rays of like length in a warp and the
@@ -1315,29 +1336,79 @@ uint64_t two_pass_state_bytes(uint64_t n) {
 // Per-band queue counters (kBandCounterBytes): [0] far-pass claim (u64), [8]
 // near queue count (u32), [12] far queue count (u32), [16] near-pass claim
 // (u64), zeroed pairwise before each pass; [24] finish queue count (u32), [32]
-// near-critical queue count (u32), [40] the critical pass's claim (u64) and [64] the
+// near-critical list's count (u32), [40] the critical pass's claim (u64) and [64] the
 // near-critical classes' histogram and cursors (kCritClasses u32 each), zeroed once.
 namespace {
-cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t launch_rays, uint64_t begin,
-                         uint64_t count, char* qb,
-                         uint32_t far_grid, uint32_t far_block, uint32_t near_grid, uint32_t finish_grid,
-                         int sm_count, uint32_t crit_ctas, bool crit_beside, bool lean, cudaStream_t s) {
-    uint32_t* near_q = buf.queues + 4 * begin;
-    uint32_t* far_q = near_q + count;
-    uint32_t* crit_q = far_q + 2 * count;
+// A band's part of the launch's scratch.
+struct Band {
+    uint32_t *near_q, *far_q, *finish_q, *crit_q;
+    char* counters;
+    uint64_t begin, count;
+};
+
+// The band's rays sorted out (band_list_kernel): the far list in the far queue, which the
+// near pass fills later; the critical list, before it is sorted, in the near queue, which
+// the far pass fills.
+cudaError_t enqueue_lists(TraceArgs args, const Band& band, bool sorted, int sm_count, cudaStream_t s) {
+    args.total_rays = band.count;
+    args.ray_base = band.begin;
+    char* qb = band.counters;
+    cudaError_t e = cudaMemsetAsync(qb, 0, kBandCounterBytes, s);
+    if (e != cudaSuccess) return e;
+    uint32_t* n_crit = reinterpret_cast<uint32_t*>(qb + 32);
+    uint32_t* crit_list = sorted ? band.near_q : band.crit_q;
+    band_list_kernel<<<static_cast<uint32_t>((band.count + 127) / 128), 128, 0, s>>>(
+        args, band.far_q, crit_list, n_crit, sorted);
+    if ((e = cudaGetLastError()) != cudaSuccess || !sorted) return e;
+    uint32_t* hist = reinterpret_cast<uint32_t*>(qb + 64);
+    const uint32_t blocks =
+        static_cast<uint32_t>(std::min<uint64_t>((band.count + kCritBlock - 1) / kCritBlock, 2u * sm_count));
+    crit_count_kernel<<<blocks, kCritBlock, 0, s>>>(crit_list, n_crit, hist);
+    crit_scatter_kernel<<<blocks, kCritBlock, 0, s>>>(crit_list, n_crit, hist, hist + kCritClasses, band.crit_q);
+    return cudaGetLastError();
+}
+
+cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, const Band& band, uint32_t far_grid,
+                         uint32_t far_block, uint32_t near_grid, uint32_t finish_grid, int sm_count, uint32_t crit_ctas,
+                         bool crit_beside, bool crit_first, bool lean, cudaStream_t s) {
+    char* qb = band.counters;
+    uint32_t *near_q = band.near_q, *far_q = band.far_q;
     args.park = buf.park;
-    args.total_rays = count;
-    args.ray_base = begin;
-    args.finish_queue = far_q + count;
+    args.total_rays = band.count;
+    args.ray_base = band.begin;
+    args.finish_queue = band.finish_q;
     args.finish_count = reinterpret_cast<uint32_t*>(qb + 24);
     const uint32_t far_refill = args.refill_threshold;
-    // a class needs the index's upper bits
-    const bool sorted = launch_rays <= (1ull << kCritClassShift) &&
-                        launch_rays > kCritSortRaysPerSm * static_cast<uint64_t>(sm_count);
-    cudaError_t e = cudaMemsetAsync(qb + 24, 0, kBandCounterBytes - 24, s);
+    cudaError_t e = cudaSuccess;
+    // critical pass: the near-critical rays, FP64 from their pixels to their end at
+    // their graded tolerance (the single FP64 kernel over a queue); on its own stream it
+    // runs beside the other passes, each filling the SMs the other's tail leaves idle.
+    // In a band of several, whose gaps another band's passes fill, it comes after the
+    // far pass (the 1536^2 frame 29.6 / 30.2 ms before it)
+    const TraceArgs base = args;
+    const auto critical_pass = [&]() -> cudaError_t {
+        TraceArgs c = base;
+        c.queue = reinterpret_cast<unsigned long long*>(qb + 40);
+        c.refill_threshold = 32;
+        c.in_queue = band.crit_q;
+        c.in_count = reinterpret_cast<const uint32_t*>(qb + 32);
+        c.finish_queue = nullptr;
+        c.finish_count = nullptr;
+        cudaStream_t cs = s;
+        cudaError_t ce = cudaSuccess;
+        if (crit_beside) {
+            cs = static_cast<cudaStream_t>(buf.crit_stream);
+            if ((ce = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_fork), s)) != cudaSuccess) return ce;
+            if ((ce = cudaStreamWaitEvent(cs, static_cast<cudaEvent_t>(buf.crit_fork), 0)) != cudaSuccess) return ce;
+        }
+        launch_trace(c, sm_count, crit_ctas, kCriticalBlock, false, false, cs, lean);
+        if ((ce = cudaGetLastError()) != cudaSuccess) return ce;
+        return crit_beside ? cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_join), cs) : cudaSuccess;
+    };
+    if (crit_first && (e = critical_pass()) != cudaSuccess) return e;
     for (int round = 0; e == cudaSuccess && round < kMixedRounds; ++round) {
-        // far pass: pixels (first round) or the far queue -> near queue
-        if ((e = cudaMemsetAsync(qb, 0, 12, s)) != cudaSuccess) break;
+        // far pass: the far list (first round) or the far queue -> near queue
+        if (round > 0 && (e = cudaMemsetAsync(qb, 0, 12, s)) != cudaSuccess) break;
         args.queue = reinterpret_cast<unsigned long long*>(qb);
         args.refill_threshold = far_refill;
         args.from_pixels = (round == 0) ? 1u : 0u;
@@ -1346,43 +1417,9 @@ cudaError_t enqueue_band(TraceArgs args, const TwoPassBuffers& buf, uint64_t lau
         args.in_count = reinterpret_cast<const uint32_t*>(qb + 12);
         args.out_queue = near_q;
         args.out_count = reinterpret_cast<uint32_t*>(qb + 8);
-        // the near pass fills the far queue later: until then its memory takes the
-        // unsorted near-critical list
-        args.crit_classes = sorted ? 1u : 0u;
-        args.crit_queue = (round == 0) ? (sorted ? far_q : crit_q) : nullptr;
-        args.crit_count = (round == 0) ? reinterpret_cast<uint32_t*>(qb + 32) : nullptr;
         launch_trace_pass(args, PASS_FAR, far_grid, far_block, lean, s);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if (round == 0 && sorted) {
-            uint32_t* hist = reinterpret_cast<uint32_t*>(qb + 64);
-            const uint32_t* n_crit = reinterpret_cast<const uint32_t*>(qb + 32);
-            const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + kCritBlock - 1) / kCritBlock, 2u * sm_count));
-            crit_count_kernel<<<blocks, kCritBlock, 0, s>>>(far_q, n_crit, hist);
-            crit_scatter_kernel<<<blocks, kCritBlock, 0, s>>>(far_q, n_crit, hist, hist + kCritClasses, crit_q);
-            if ((e = cudaGetLastError()) != cudaSuccess) break;
-        }
-        if (round == 0) {
-            // critical pass: the near-critical rays, FP64 from their pixels to their
-            // end at their graded tolerance (the single FP64 kernel over a queue);
-            // on its own stream it runs beside the near passes, each filling the
-            // SMs the other's tail leaves idle
-            TraceArgs c = args;
-            c.queue = reinterpret_cast<unsigned long long*>(qb + 40);
-            c.refill_threshold = 32;
-            c.in_queue = crit_q;
-            c.in_count = reinterpret_cast<const uint32_t*>(qb + 32);
-            c.out_queue = c.finish_queue = c.crit_queue = nullptr;
-            c.out_count = c.finish_count = c.crit_count = nullptr;
-            cudaStream_t cs = s;
-            if (crit_beside) {
-                cs = static_cast<cudaStream_t>(buf.crit_stream);
-                if ((e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_fork), s)) != cudaSuccess) break;
-                if ((e = cudaStreamWaitEvent(cs, static_cast<cudaEvent_t>(buf.crit_fork), 0)) != cudaSuccess) break;
-            }
-            launch_trace(c, sm_count, crit_ctas, kCriticalBlock, false, false, cs, lean);
-            if ((e = cudaGetLastError()) != cudaSuccess) break;
-            if (crit_beside && (e = cudaEventRecord(static_cast<cudaEvent_t>(buf.crit_join), cs)) != cudaSuccess) break;
-        }
+        if (round == 0 && !crit_first && (e = critical_pass()) != cudaSuccess) break;
         // near pass: near queue -> far queue (the last one keeps its rays)
         if ((e = cudaMemsetAsync(qb + 12, 0, 12, s)) != cudaSuccess) break;
         args.queue = reinterpret_cast<unsigned long long*>(qb + 16);
@@ -1426,30 +1463,43 @@ int enqueue_two_pass(const TraceArgs& base, const TwoPassBuffers& buf, int sm_co
     const int crit_occ = trace_occupancy(kCriticalBlock, false, false);
     const uint32_t crit_ctas = static_cast<uint32_t>(crit_occ > 1 ? crit_occ : 1);
     cudaError_t e = cudaSuccess;
+    // bands of whole warps' worth of rays (multiples of 32); every band's lists first,
+    // while the SMs are free
+    const uint64_t per = ((n + bands - 1) / bands + 31) / 32 * 32;
+    // a class needs the index's upper bits
+    const bool sorted = n <= (1ull << kCritClassShift) && n > kCritSortRaysPerSm * static_cast<uint64_t>(sm_count);
+    Band part[kMaxBands];
+    uint32_t n_parts = 0;
+    for (uint64_t begin = 0; begin < n; begin += per, ++n_parts) {
+        Band& p = part[n_parts];
+        p.begin = begin;
+        p.count = std::min(per, n - begin);
+        p.near_q = buf.queues + 4 * begin;
+        p.far_q = p.near_q + p.count;
+        p.finish_q = p.far_q + p.count;
+        p.crit_q = p.finish_q + p.count;
+        p.counters = buf.counters + kBandCounterBytes * n_parts;
+        if ((e = enqueue_lists(base, p, sorted, sm_count, s)) != cudaSuccess) return static_cast<int>(e);
+    }
     if (bands > 1) {
         if ((e = cudaEventRecord(static_cast<cudaEvent_t>(fork), s)) != cudaSuccess) return static_cast<int>(e);
         if ((e = cudaStreamWaitEvent(s2, static_cast<cudaEvent_t>(fork), 0)) != cudaSuccess) return static_cast<int>(e);
     }
-    // bands of whole warps' worth of rays (multiples of 32); a band's hook is
-    // enqueued after the next band's trace, so its work overlaps that trace
-    const uint64_t per = ((n + bands - 1) / bands + 31) / 32 * 32;
-    uint64_t begin = 0, prev_begin = 0, prev_count = 0;
+    // a band's hook is enqueued after the next band's trace, so its work overlaps that trace
+    const Band* prev = nullptr;
     cudaStream_t prev_stream = nullptr;
-    for (uint32_t b = 0; b < bands && begin < n && e == cudaSuccess; ++b) {
-        const uint64_t count = (n - begin < per) ? n - begin : per;
+    const bool crit_beside = bands == 1 && buf.crit_stream && buf.crit_fork && buf.crit_join;
+    for (uint32_t b = 0; b < n_parts && e == cudaSuccess; ++b) {
         cudaStream_t sb = (b & 1u) ? s2 : s;
-        const bool crit_beside = bands == 1 && buf.crit_stream && buf.crit_fork && buf.crit_join;
-        e = enqueue_band(base, buf, n, begin, count, buf.counters + kBandCounterBytes * b, far_grid, far_block, near_grid,
-                         finish_grid, sm_count, crit_ctas, crit_beside, lean, sb);
-        if (e == cudaSuccess && after_band && prev_stream)
-            e = static_cast<cudaError_t>(after_band(hook_ctx, prev_begin, prev_count, prev_stream));
-        prev_begin = begin;
-        prev_count = count;
+        e = enqueue_band(base, buf, part[b], far_grid, far_block, near_grid, finish_grid, sm_count, crit_ctas, crit_beside,
+                         bands == 1, lean, sb);
+        if (e == cudaSuccess && after_band && prev)
+            e = static_cast<cudaError_t>(after_band(hook_ctx, prev->begin, prev->count, prev_stream));
+        prev = &part[b];
         prev_stream = sb;
-        begin += count;
     }
-    if (e == cudaSuccess && after_band && prev_stream)
-        e = static_cast<cudaError_t>(after_band(hook_ctx, prev_begin, prev_count, prev_stream));
+    if (e == cudaSuccess && after_band && prev)
+        e = static_cast<cudaError_t>(after_band(hook_ctx, prev->begin, prev->count, prev_stream));
     if (e != cudaSuccess) return static_cast<int>(e);
     if (bands > 1) {
         if ((e = cudaEventRecord(static_cast<cudaEvent_t>(join), s2)) != cudaSuccess) return static_cast<int>(e);
