@@ -317,6 +317,7 @@ __device__ __noinline__ void sample_ended_paths(const TraceArgs& args) {
         points = __shfl_sync(~0u, points, 0, kPathLanes);
         if (points == kPathOpen) points = 0;
         __threadfence();  // the chain was stored before its length
+        __syncwarp();     // and the group's other lanes read it after the one that saw that
         sample_paths(args, local, points);
         if (points && lane % kPathLanes == 0) P.points[local] = 0;  // gathered
         __syncwarp();
