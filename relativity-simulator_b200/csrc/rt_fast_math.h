@@ -1,19 +1,26 @@
 // rt_fast_math.h -- FP64 reciprocal and square root for the step loops, host/device.
 //
-// The compiler's 1.0 / v and sqrt(v) each end in a test for special arguments and
-// a branch to a slow path: about six instructions of their own, and a fence for
-// the scheduler in the middle of a dependency chain.  The tracers' arguments
-// (r^2 and r^6 of a point) are far from the ends of the range, so these forms
-// leave the special cases out.  Both refine a hardware seed (about 20 bits) by
-// Newton's iteration and end with Markstein's fused correction (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34, 1990), after which the result is the correctly rounded one
-// and so the one that 1.0 / v and sqrt(v) give.  Measured in the FP64 tracer with
-// the compiler's forms / these: 2048^2 37.0 / 34.1 ms, 512^2 2.60 / 2.41 ms.
+// The tracers' arguments (r^2 and r^6 of a point) are far from the ends of the range,
+// so these forms leave special arguments out and are one straight line of fused
+// operations.  Measured in the FP64 tracer with 1.0 / v and sqrt(v) / with these:
+// 2048^2 37.0 / 34.1 ms, 512^2 2.60 / 2.41 ms.
 //
-// Outside [2^-900, 2^1020] a result may be wrong; for zero, subnormal, negative and
-// infinite arguments and NaN it is NaN (the seed is infinite, zero or NaN, and the
-// corrections multiply infinity by zero).
+// Both start from the hardware's approximation (PTX rcp.approx.ftz.f64 and
+// rsqrt.approx.ftz.f64, about 20 bits).  The reciprocal takes Newton-Raphson steps,
+// the root the coupled iteration of R. E. Goldschmidt ("Applications of division by
+// convergence", M.Sc. thesis, MIT 1964) in the fused form of P. Markstein ("Software
+// division and square root using Goldschmidt's algorithms", 6th Conference on Real
+// Numbers and Computers, 2004).  The last step of each is Markstein's correction by a
+// fused residual ("Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990), which rounds correctly: the results are those
+// of 1.0 / v and sqrt(v), but for a reciprocal whose argument has a significand of all
+// ones, which is one ulp low.
+//
+// That holds for arguments in [2^-900, 2^1020].  For zero, subnormal, negative (the
+// root) and infinite arguments and NaN the result is NaN: the seed is infinite, zero or
+// NaN, and the steps multiply infinity by zero or subtract infinities.  Other arguments
+// have no such mark: below 2^-900 a root may be an ulp off, and from 2^1022 on the
+// reciprocal's seed is flushed to zero and the result is 0.
 #pragma once
 
 #include <cmath>
@@ -26,28 +33,29 @@
 
 namespace relsim {
 
-// 1 / v from a seed y of at least 18 bits: e is the seed's relative error; the
-// cubic step leaves about e^3, the last line rounds correctly.
+// 1 / v from a seed y of at least 18 bits.  With e = 1 - v y, 1 / v = y / (1 - e) =
+// y (1 + e + ...), so y + y e leaves a relative error of e^2: 2^-36 and 2^-72 after two
+// steps.  The second result is then within an ulp, which the third step rounds correctly.
 RT_FM_FN double refine_rcp(double v, double y) {
-    double e = fma(-v, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
-    e = fma(-v, y, 1.0);
-    return fma(y, e, y);
+    y = fma(y, fma(-v, y, 1.0), y);
+    y = fma(y, fma(-v, y, 1.0), y);
+    return fma(y, fma(-v, y, 1.0), y);
 }
 
-// sqrt(v) from a seed y of 1 / sqrt(v) of at least 18 bits: third-order Newton step
-// of the reciprocal root (1 + e/2 + 3 e^2/8), then g = v y and its residual.
+// sqrt(v) from a seed y of 1 / sqrt(v) of at least 18 bits.  g = v y goes to sqrt(v) and
+// h = y / 2 to 1 / (2 sqrt(v)): with r = 1/2 - g h, where 2 g h = 1 - 2 r, both are short
+// of their limits by the factor (1 - 2 r)^(1/2) = 1 - r - ..., so g + g r and h + h r
+// leave an error of the order of r^2: 2^-35 and 2^-69.  The correction adds the residual
+// v - g^2 divided by 2 g.
 RT_FM_FN double refine_sqrt(double v, double y) {
-    const double e = fma(-v * y, y, 1.0);
-    y = fma(y * e, fma(0.375, e, 0.5), y);
-    const double g = v * y;
-    return fma(fma(-g, g, v), 0.5 * y, g);
-}
-
-// 1 / sqrt(v) by the same third-order step; within an ulp, not correctly rounded.
-RT_FM_FN double refine_rsqrt(double v, double y) {
-    const double e = fma(-v * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    double g = v * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, v), h, g);
 }
 
 #ifdef __CUDACC__
@@ -61,12 +69,6 @@ __device__ __forceinline__ double fast_sqrt(double v) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
     return refine_sqrt(v, y);
-}
-
-__device__ __forceinline__ double fast_rsqrt(double v) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-    return refine_rsqrt(v, y);
 }
 #endif
 

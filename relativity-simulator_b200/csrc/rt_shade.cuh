@@ -274,9 +274,9 @@ __device__ __forceinline__ bool fm_chord(const ShadeDesc& D, const double* from,
         const double px = from[0] + t * dx, py = from[1] + t * dy, pz = from[2] + t * dz;
         const double rho2 = px * px + py * py, z2 = pz * pz, r2 = rho2 + z2;
         if (r2 < inner2 || r2 > outer2) continue;
-        const double inv_r = fast_rsqrt(r2), inv_r2 = inv_r * inv_r;
+        const double inv_r2 = fast_rcp(r2);
         double h, ut, uphi;
-        if (!torus::fluid(T, e_in, r2 * inv_r, z2 * inv_r2, rho2 * inv_r2, h, ut, uphi)) continue;
+        if (!torus::fluid(T, e_in, fast_sqrt(r2), z2 * inv_r2, rho2 * inv_r2, h, ut, uphi)) continue;
         const double ratio = cd((h - 1.0) * inv_span, 0.0, 1.0);
         const double tau = tau_step * exp(D.fm_exponent * log(ratio));
         if (tau < 1e-12) continue;

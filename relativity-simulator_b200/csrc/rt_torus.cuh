@@ -80,7 +80,7 @@ RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_
     if (denom <= 0.0 || delta <= 0.0) return false;
 #ifdef __CUDA_ARCH__
     const double inv_d = fast_rcp(denom);
-    const double inv_ew = fast_rsqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30));
+    const double inv_ew = fast_rcp(fast_sqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30)));
 #else
     const double inv_d = 1.0 / denom;
     const double inv_ew = 1.0 / sqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30));
