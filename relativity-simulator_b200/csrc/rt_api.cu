@@ -321,17 +321,26 @@ rt_status scratch_rays(rt_handle* h, const rt_ray_out* host, size_t n, rt_ray_ou
     return RT_OK;
 }
 
+// Bands of a host dispatch on the two-pass tracer: each band's copies overlap
+// the next band's trace (1 M rays and up).  Four: with every ray followed
+// through the disk and the sky shaded, each band's pass tails cost more than
+// the longer exposed copy of the last band (measured at 2048^2: 2 / 4 / 8 / 16
+// bands 75.7 / 75.2 / 80.9 / 81.3 ms an image).
+constexpr uint32_t kCopyBands = 4;
+constexpr uint64_t kBandedMinRays = uint64_t{1} << 20;
+
 // Outputs of a small host dispatch side by side in one device buffer, read back in one
 // copy to pinned memory: a copy per field into the caller's pageable arrays waits for the
 // device and stages each time.  Measured, the call less its kernel, a copy per field /
 // one copy: six fields of a 64x64 tile 110 / 49 us, of 192^2 rays 213 / 172; all fields
 // and pixels of 64^2 rays 310 / 92, of 192^2 (4.7 MB) 675 / 535.  From 6 MB on both take
-// as long (first touches of the caller's arrays).
+// as long (first touches of the caller's arrays).  A dispatch of kBandedMinRays and more
+// copies band by band and is never staged.
 constexpr size_t kStagedBytes = size_t{4} << 20;
 rt_status stage_outputs(rt_handle* h, const rt_ray_out* rays, const rt_pixel_out* pixels, size_t n, rt_ray_out& dev,
                         rt_pixel_out*& dpix, size_t& bytes) {
     constexpr size_t kAlign = 256;
-    if (n > kStagedBytes) return RT_OK;
+    if (n >= kBandedMinRays) return RT_OK;
     void* const* hp = reinterpret_cast<void* const*>(rays);
     size_t total = pixels ? (n * sizeof(rt_pixel_out) + kAlign - 1) / kAlign * kAlign : 0;
     const size_t first_field = total;
@@ -549,14 +558,6 @@ int band_copy_hook(void* vctx, uint64_t begin, uint64_t count, void* stream) {
     }
     return static_cast<int>(cudaSuccess);
 }
-
-// Bands of a host dispatch on the two-pass tracer: each band's copies overlap
-// the next band's trace (1 M rays and up).  Four: with every ray followed
-// through the disk and the sky shaded, each band's pass tails cost more than
-// the longer exposed copy of the last band (measured at 2048^2: 2 / 4 / 8 / 16
-// bands 75.7 / 75.2 / 80.9 / 81.3 ms an image).
-constexpr uint32_t kCopyBands = 4;
-constexpr uint64_t kBandedMinRays = uint64_t{1} << 20;
 
 // One host-buffer dispatch over a window (dispatch_and_readback semantics).
 rt_status dispatch_window(rt_handle* h, const rt_camera* cam, uint32_t col0, uint32_t ncols, uint32_t row0,
