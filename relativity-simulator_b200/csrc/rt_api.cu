@@ -21,6 +21,7 @@
 #include "relsim_cuda.h"
 #include "rt_internal.h"
 #include "rt_planck.h"
+#include "rt_stage.h"
 
 namespace relsim {
 double measure_fma_peak(bool fp64, int sm_count, cudaStream_t stream, float* ms_out);
@@ -321,54 +322,29 @@ rt_status scratch_rays(rt_handle* h, const rt_ray_out* host, size_t n, rt_ray_ou
     return RT_OK;
 }
 
-// Bands of a host dispatch on the two-pass tracer: each band's copies overlap
-// the next band's trace (1 M rays and up).  Four: with every ray followed
-// through the disk and the sky shaded, each band's pass tails cost more than
-// the longer exposed copy of the last band (measured at 2048^2: 2 / 4 / 8 / 16
-// bands 75.7 / 75.2 / 80.9 / 81.3 ms an image).
-constexpr uint32_t kCopyBands = 4;
-constexpr uint64_t kBandedMinRays = uint64_t{1} << 20;
-
-// Outputs of a small host dispatch side by side in one device buffer, read back in one
-// copy to pinned memory: a copy per field into the caller's pageable arrays waits for the
-// device and stages each time.  Measured, the call less its kernel, a copy per field /
-// one copy: six fields of a 64x64 tile 110 / 49 us, of 192^2 rays 213 / 172; all fields
-// and pixels of 64^2 rays 310 / 92, of 192^2 (4.7 MB) 675 / 535.  From 6 MB on both take
-// as long (first touches of the caller's arrays).  A dispatch of kBandedMinRays and more
-// copies band by band and is never staged.
-constexpr size_t kStagedBytes = size_t{4} << 20;
-rt_status stage_outputs(rt_handle* h, const rt_ray_out* rays, const rt_pixel_out* pixels, size_t n, rt_ray_out& dev,
-                        rt_pixel_out*& dpix, size_t& bytes) {
-    constexpr size_t kAlign = 256;
-    if (n >= kBandedMinRays) return RT_OK;
-    void* const* hp = reinterpret_cast<void* const*>(rays);
-    size_t total = pixels ? (n * sizeof(rt_pixel_out) + kAlign - 1) / kAlign * kAlign : 0;
-    const size_t first_field = total;
-    for (int f = 0; rays && f < kRayFields; ++f)
-        if (hp[f]) total += (n * kRayFieldBytes[f] + kAlign - 1) / kAlign * kAlign;
-    if (total == 0 || total > kStagedBytes) return RT_OK;
-    const rt_status st = ensure(h, h->stage, total);
-    if (st != RT_OK) return st;
-    if (h->stage_host_bytes < total) {
+// The handle's buffers of a staged dispatch (stage_outputs); both go with the handle.
+struct StageMemory {
+    rt_handle* h;
+    char* device(size_t bytes) const {
+        if (ensure(h, h->stage, bytes) == RT_OK) return static_cast<char*>(h->stage.ptr);
+        h->error.clear();
+        return nullptr;
+    }
+    bool pinned(size_t bytes) const {
+        if (h->stage_host_bytes >= bytes) return true;
         if (h->stage_host) cudaFreeHost(h->stage_host);
         h->stage_host = nullptr;
         h->stage_host_bytes = 0;
-        const size_t grow = std::max(size_t{1} << 18, std::min(2 * total, kStagedBytes));
-        RT_CUDA(h, cudaMallocHost(&h->stage_host, grow));
+        const size_t grow = std::max(size_t{1} << 18, std::min(2 * bytes, kStagedBytes));
+        if (cudaMallocHost(&h->stage_host, grow) != cudaSuccess) {
+            cudaGetLastError();
+            h->stage_host = nullptr;
+            return false;
+        }
         h->stage_host_bytes = grow;
+        return true;
     }
-    char* base = static_cast<char*>(h->stage.ptr);
-    if (pixels) dpix = reinterpret_cast<rt_pixel_out*>(base);
-    void** dp = reinterpret_cast<void**>(&dev);
-    size_t at = first_field;
-    for (int f = 0; rays && f < kRayFields; ++f) {
-        if (!hp[f]) continue;
-        dp[f] = base + at;
-        at += (n * kRayFieldBytes[f] + kAlign - 1) / kAlign * kAlign;
-    }
-    bytes = total;
-    return RT_OK;
-}
+};
 
 rt_status copy_back(rt_handle* h, const rt_ray_out* host, const rt_ray_out& dev, rt_pixel_out* hpix,
                     const rt_pixel_out* dpix, size_t n, cudaStream_t s) {
@@ -559,6 +535,13 @@ int band_copy_hook(void* vctx, uint64_t begin, uint64_t count, void* stream) {
     return static_cast<int>(cudaSuccess);
 }
 
+// Bands of a host dispatch on the two-pass tracer: each band's copies overlap
+// the next band's trace (1 M rays and up).  Four: with every ray followed
+// through the disk and the sky shaded, each band's pass tails cost more than
+// the longer exposed copy of the last band (measured at 2048^2: 2 / 4 / 8 / 16
+// bands 75.7 / 75.2 / 80.9 / 81.3 ms an image).
+constexpr uint32_t kCopyBands = 4;
+
 // One host-buffer dispatch over a window (dispatch_and_readback semantics).
 rt_status dispatch_window(rt_handle* h, const rt_camera* cam, uint32_t col0, uint32_t ncols, uint32_t row0,
                           uint32_t nrows, rt_pixel_out* pixels, const rt_ray_out* rays, size_t capacity,
@@ -571,8 +554,8 @@ rt_status dispatch_window(rt_handle* h, const rt_camera* cam, uint32_t col0, uin
     if ((st = ensure(h, h->bundles, sizeof(BundleDesc))) != RT_OK) return st;
     rt_ray_out dev{};
     rt_pixel_out* dpix = nullptr;
-    size_t staged = 0;  // bytes read back in one copy
-    if ((st = stage_outputs(h, rays, pixels, n, dev, dpix, staged)) != RT_OK) return st;
+    StageMemory stage{h};
+    const size_t staged = stage_outputs(stage, rays, pixels != nullptr, n, dev, dpix);  // bytes read back in one copy
     if (!staged) {
         if ((st = scratch_rays(h, rays, n, dev)) != RT_OK) return st;
         if (pixels) {
