@@ -379,7 +379,7 @@ struct BandCopyCtx;
 rt_status launch_banded_single(rt_handle* h, const rt_camera* cam, uint32_t col0, uint32_t ncols, uint32_t row0,
                                uint32_t nrows, uint64_t out_offset, const OutPtrs& out, BandCopyCtx& ctx);
 
-// The blackbody colour's table on the device: 57 KB, the same for every camera,
+// The blackbody colour's table on the device: 59 KB, the same for every camera,
 // uploaded once and waited for, since later dispatches may use other streams.
 rt_status ensure_planck(rt_handle* h, cudaStream_t s) {
     if (h->planck.ptr) return RT_OK;

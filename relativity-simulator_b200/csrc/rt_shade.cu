@@ -31,7 +31,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <vector>
 
 #include "rt_device.cuh"
 #include "rt_internal.h"
@@ -248,14 +247,15 @@ static void spectral_table(double* lambda_um, double (*weight)[3]) {
 }
 
 const double* planck_table_host() {
-    static const std::vector<double> table = [] {
-        double lambda_um[33], weight[33][3];
-        spectral_table(lambda_um, weight);
-        std::vector<double> t(kPlanckTableDoubles);
-        planck_table_fill(lambda_um, weight, t.data());
-        return t;
-    }();
-    return table.data();
+    static const struct Table {
+        double v[kPlanckTableDoubles];
+        Table() {
+            double lambda_um[33], weight[33][3];
+            spectral_table(lambda_um, weight);
+            planck_table_fill(lambda_um, weight, v);
+        }
+    } table;
+    return table.v;
 }
 
 bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d) {
