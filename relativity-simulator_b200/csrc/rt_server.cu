@@ -34,6 +34,7 @@
 
 #include "relsim_cuda.h"
 #include "rt_internal.h"
+#include "rt_planck.h"
 
 using namespace relsim;
 
@@ -190,6 +191,7 @@ struct rt_server {
     bool shade_on = false;
     rt_shading shading{};
     ShadeDesc* dev_shade = nullptr;  // ring of per-request shading constants, used in copy-stream order
+    double* dev_planck = nullptr;    // the blackbody colour's table
     uint32_t shade_next = 0;
 };
 
@@ -252,6 +254,7 @@ bool start_copy(rt_server* s, Request* r) {
     if (s->shade_on && r->n_sources == 0 && r->host_pixels) {
         ShadeDesc d;
         if (build_shade_desc(r->cam, s->shading, d)) {
+            d.planck = s->dev_planck;
             ShadeDesc* slot = s->dev_shade + (s->shade_next++ % kShadeSlots);
             // pageable descriptor: the copy is staged before the call returns; the ring slot
             // is next written kShadeSlots requests later, after this kernel in stream order
@@ -669,6 +672,7 @@ void rt_server_destroy(rt_server* s) {
     }
     if (s->arena) cudaFree(s->arena);
     if (s->dev_shade) cudaFree(s->dev_shade);
+    if (s->dev_planck) cudaFree(s->dev_planck);
     delete s;
 }
 
@@ -793,10 +797,18 @@ rt_status rt_server_set_shading(rt_server* s, const rt_shading* sh) {
         (s->cfg.record_mask & kShadeMask) != kShadeMask)
         return RT_ERR_INVALID_ARG;
     if (!s->dev_shade) {
+        // both or neither; the table goes up on the stream that the requests are shaded on
         cudaSetDevice(s->device);
-        if (cudaMalloc(&s->dev_shade, sizeof(ShadeDesc) * kShadeSlots) != cudaSuccess) {
+        constexpr size_t table = sizeof(double) * kPlanckTableDoubles;
+        if (cudaMalloc(&s->dev_shade, sizeof(ShadeDesc) * kShadeSlots) != cudaSuccess ||
+            cudaMalloc(&s->dev_planck, table) != cudaSuccess ||
+            cudaMemcpyAsync(s->dev_planck, planck_table_host(), table, cudaMemcpyHostToDevice, s->copy_stream) !=
+                cudaSuccess) {
             cudaGetLastError();
+            cudaFree(s->dev_shade);
+            cudaFree(s->dev_planck);
             s->dev_shade = nullptr;
+            s->dev_planck = nullptr;
             return RT_ERR_OOM;
         }
     }
