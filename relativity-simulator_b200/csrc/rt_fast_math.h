@@ -58,18 +58,25 @@ RT_FM_FN double refine_sqrt(double v, double y) {
     return fma(fma(-g, g, v), h, g);
 }
 
-#ifdef __CUDACC__
-__device__ __forceinline__ double fast_rcp(double v) {
+// On the host, which has no such seeds, the operations themselves.
+RT_FM_FN double fast_rcp(double v) {
+#ifdef __CUDA_ARCH__
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
     return refine_rcp(v, y);
+#else
+    return 1.0 / v;
+#endif
 }
 
-__device__ __forceinline__ double fast_sqrt(double v) {
+RT_FM_FN double fast_sqrt(double v) {
+#ifdef __CUDA_ARCH__
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
     return refine_sqrt(v, y);
-}
+#else
+    return std::sqrt(v);
 #endif
+}
 
 }  // namespace relsim

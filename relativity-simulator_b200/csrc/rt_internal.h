@@ -285,6 +285,7 @@ struct alignas(16) ShadeDesc {
     // exponent 1 / (gamma - 1), kappa (optical depth per M at peak enthalpy) and
     // samples per M of chord
     double fm_m, fm_a, fm_rh, fm_l, fm_w_in, fm_h_max, fm_inner, fm_outer, fm_exponent, fm_kappa, fm_density;
+    double fm_e_in, fm_e_in_lo;  // e^W_in in two parts (torus::EdgeFactor)
     const double* planck;  // device: the blackbody colour's table (rt_planck.h); null: not at hand
 };
 

@@ -106,11 +106,7 @@ inline void planck_table_fill(const double* lambda_um, const double (*w)[3], dou
 // XYZ from the table for kPlanckMinT <= t (clamped to 400,000 K above).
 RT_PL_HD inline void planck_lookup(const double* __restrict__ table, double temperature_k, double* xyz) {
     const double t = 400000.0 < temperature_k ? 400000.0 : temperature_k;
-#ifdef __CUDA_ARCH__
     const double s = fast_rcp(t);
-#else
-    const double s = 1.0 / t;
-#endif
     const double at = s * kPlanckPerS;  // exact, and so is the place within the piece
     int p = static_cast<int>(at);
     p = p < 0 ? 0 : (p > kPlanckPieces - 1 ? kPlanckPieces - 1 : p);

@@ -331,18 +331,8 @@ bool build_shade_desc(const rt_camera& cam, const rt_shading& s, ShadeDesc& d) {
     if (s.hydro_model == 2u) {
         const torus::TorusContext c = torus::make_torus(d.mass, a, static_cast<double>(s.torus_inner_radius),
                                                         static_cast<double>(s.torus_center_radius));
-        d.fm_valid = c.valid ? 1u : 0u;
-        d.fm_m = c.t.m;
-        d.fm_a = c.t.a;
-        d.fm_rh = c.t.rh;
-        d.fm_l = c.t.l;
-        d.fm_w_in = c.t.w_in;
-        d.fm_h_max = c.h_max;
-        d.fm_inner = c.inner_bound;
-        d.fm_outer = c.outer_bound;
-        d.fm_exponent = 1.0 / mxd(static_cast<double>(s.adiabatic_index) - 1.0, 1e-3);
-        d.fm_kappa = static_cast<double>(s.optical_depth_scale) * mxd(static_cast<double>(P[DP_OPACITY_SCALE]), 0.0);
-        d.fm_density = mxd(static_cast<double>(s.sampling_density), 0.1);
+        set_torus(d, c, static_cast<double>(s.adiabatic_index), static_cast<double>(s.optical_depth_scale),
+                  static_cast<double>(s.sampling_density));
     }
     return true;
 }

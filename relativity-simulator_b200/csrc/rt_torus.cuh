@@ -59,16 +59,30 @@ RT_FM_HD double potential(double m, double a, double rh, double l, double r, dou
 }
 RT_FM_HD double potential(const Torus& t, double r, double theta) { return potential(t.m, t.a, t.rh, t.l, r, theta); }
 
+// e^W_in in two parts, the second what the first rounds off.
+struct EdgeFactor {
+    double hi, lo;
+};
+inline EdgeFactor edge_factor(double w_in) {
+    const long double e = std::exp(static_cast<long double>(w_in));
+    const double hi = static_cast<double>(e);
+    return {hi, static_cast<double>(e - hi)};
+}
+
 // The fluid at radius r with c2 = cos^2 theta and s2 = sin^2 theta (s2 >= 1e-30 is
 // imposed): false outside the torus (no such orbit, or an enthalpy h = exp(W_in - W)
-// of 1 + 1e-9 or less, :152-159), else h and the four-velocity's u^t and u^phi
-// (:210-224: u_t = -e^W, u_phi = -l u_t, raised with the Boyer-Lindquist Kerr inverse
-// metric, metrics/kerr.hpp:151-177).  With W = log(X) / 2, X = rho^2 Delta sin^2 / D,
-// no logarithm or exponential is taken: h = e_in / sqrt(X), e_in = exp(W_in), and
-// e^W / (rho^2 Delta) = sin^2 / (sqrt(X) D) leaves 1 / D and 1 / sqrt(X) as the only
-// divisions.  On the device these are the straight-line forms (rt_fast_math.h): D and
-// X of a sampled point are far from the ends of the range, and a NaN is outside.
-RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_in, double& h, double& ut, double& uphi) {
+// of 1 + 1e-9 or less, :152-159), else h - 1 and the four-velocity, u^t = ut / per and
+// u^phi = uphi / per (:210-224: u_t = -e^W, u_phi = -l u_t, raised with the
+// Boyer-Lindquist Kerr inverse metric, metrics/kerr.hpp:151-177).  With W = -log(Z) / 2,
+// Z = D / (rho^2 Delta sin^2), no logarithm or exponential is taken: h = e^W_in sqrt(Z)
+// and per = rho^2 Delta sin^2 sqrt(Z).  h is near 1 and the light goes with powers of
+// h - 1, so that difference is formed without rounding h: the roundings of the root (its
+// residual Z - sqrt(Z)^2 is exact) and of e^W_in are taken back out.  Mean error of h - 1
+// as the reference writes it / so: spin 0 7.3e-17 / 5.8e-17, spin 0.998 8.5e-17 / 7.3e-17.
+// D and Z of a sampled point are far from the ends of the range of the straight-line
+// forms (rt_fast_math.h), and a NaN is outside.
+RT_FM_HD bool fluid(const Torus& t, const EdgeFactor& e_in, double r, double c2, double s2_in, double& h_above_1,
+                    double& per, double& ut, double& uphi) {
     if (r <= t.rh * 1.0001) return false;
     const double s2 = fmx(s2_in, 1e-30);
     const double r2 = r * r, a2 = t.a * t.a, mra = 2.0 * t.m * r * t.a;
@@ -78,36 +92,35 @@ RT_FM_HD bool fluid(const Torus& t, double e_in, double r, double c2, double s2_
     const double ds = delta - a2 * s2;
     const double denom = sigma * s2 - 2.0 * mra * t.l * s2 - t.l * t.l * ds;
     if (denom <= 0.0 || delta <= 0.0) return false;
-#ifdef __CUDA_ARCH__
-    const double inv_d = fast_rcp(denom);
-    const double inv_ew = fast_rcp(fast_sqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30)));
-#else
-    const double inv_d = 1.0 / denom;
-    const double inv_ew = 1.0 / sqrt(fmx((rho2 * delta * s2) * inv_d, 1e-30));
-#endif
-    h = e_in * inv_ew;
-    if (!(h > 1.0 + 1e-9)) return false;
-    const double q = inv_ew * inv_d;
-    ut = q * (sigma - mra * t.l) * s2;
-    uphi = q * (mra * s2 + t.l * ds);
+    const double p = rho2 * delta * s2;
+    const double ratio = denom * fast_rcp(p), z = (1e30 < ratio) ? 1e30 : ratio;
+    const double root = fast_sqrt(z);
+    const double rest = fma(-root, root, z) * static_cast<double>(0.5f / static_cast<float>(root));
+    h_above_1 = fma(e_in.hi, root, -1.0) + fma(e_in.hi, rest, e_in.lo * root);
+    if (!(h_above_1 > 1e-9)) return false;
+    per = p * root;
+    ut = (sigma - mra * t.l) * s2;
+    uphi = mra * s2 + t.l * ds;
     return true;
 }
 
 // Specific enthalpy at (r, theta), 1 outside the torus.
-RT_FM_HD double enthalpy(const Torus& t, double r, double theta) {
+inline double enthalpy(const Torus& t, double r, double theta) {
     const double st = sin(theta), ct = cos(theta);
-    double h, ut, uphi;
-    return fluid(t, exp(t.w_in), r, ct * ct, st * st, h, ut, uphi) ? h : 1.0;
+    double h_above_1, per, ut, uphi;
+    return fluid(t, edge_factor(t.w_in), r, ct * ct, st * st, h_above_1, per, ut, uphi) ? 1.0 + h_above_1 : 1.0;
 }
 
 // The fluid's u^t and u^phi at (r, theta); at rest (1, 0) outside the torus.
-RT_FM_HD void four_velocity(const Torus& t, double r, double theta, double& ut, double& uphi) {
+inline void four_velocity(const Torus& t, double r, double theta, double& ut, double& uphi) {
     const double st = sin(theta), ct = cos(theta);
-    double h;
-    if (!fluid(t, exp(t.w_in), r, ct * ct, st * st, h, ut, uphi)) {
-        ut = 1.0;
+    double h_above_1, per;
+    if (!fluid(t, edge_factor(t.w_in), r, ct * ct, st * st, h_above_1, per, ut, uphi)) {
+        per = ut = 1.0;
         uphi = 0.0;
     }
+    ut /= per;
+    uphi /= per;
 }
 
 // The torus of a hole (mass, spin clamped as the shading context does) with its
