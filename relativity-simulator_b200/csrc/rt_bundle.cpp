@@ -131,7 +131,7 @@ void build_bundle(const rt_camera& cam, uint32_t col0, uint32_t ncols, uint32_t 
                       : (cam.mixed_critical_band > 0.0) ? static_cast<float>(cam.mixed_critical_band)
                                                         : kDefaultCriticalBand;
     b.flags = (disk ? BF_DISK : 0u) | (cam.early_capture ? BF_EARLY_CAPTURE : 0u) |
-              (cam.precision_mode == RT_PRECISION_MIXED ? BF_MIXED : 0u);
+              (cam.precision_mode == RT_PRECISION_MIXED ? BF_MIXED : 0u) | (m <= kFastMaxMass ? BF_FAST_RANGE : 0u);
 }
 
 double kn_horizon(double m, double a, double q) {
@@ -233,6 +233,7 @@ uint32_t build_ms_sources(const rt_camera& cam, const rt_source* src, uint32_t n
     const double rh = m + std::sqrt(maxd(m * m - a * a, 0.0));
     MsSource p{};
     p.m = m;
+    p.m_fast = (m <= kFastMaxMass) ? m : NAN;
     p.a = a;
     p.axis[2] = 1.0;
     p.fx[0] = 1.0;
@@ -271,6 +272,7 @@ uint32_t build_ms_sources(const rt_camera& cam, const rt_source* src, uint32_t n
             q.fy[k] = fy[k];
         }
         q.m = mb;
+        q.m_fast = (mb <= kFastMaxMass) ? mb : NAN;
         q.a = ab;
         q.rh = rhb;
         q.req = std::sqrt(rhb * rhb + ab * ab);

@@ -83,10 +83,11 @@ __device__ __forceinline__ T bl_r2(T x, T y, T z, T a2) {
 // With GRAV = true the position part returns only the gravitational term
 // -2 H s k (the mixed-precision step keeps the free-streaming p in FP64).
 // With FAST = true (FP64) the square root and the reciprocal are the straight-line
-// forms of rt_fast_math.h: the same values where their arguments lie between
-// 2^-900 and 2^1020, and all six outputs NaN where one does not (sv, a factor of
-// every gravitational term, takes k and with it r, 1/r and 1/(r^2 + a^2)).  A
-// caller looks for that NaN and evaluates again with FAST = false.
+// forms of rt_fast_math.h: the same values while the reciprocal's argument, about r^6,
+// is below 2^1020, and all six outputs NaN where an argument has no finite seed (sv, a
+// factor of every gravitational term, takes k and with it r, 1/r and 1/(r^2 + a^2)).  A
+// caller looks for that NaN and evaluates again with FAST = false.  It does so too for
+// holes whose field still counts where the reciprocal gives 0 instead (kFastMaxMass).
 template <typename T, bool GRAV = false, bool FAST = false>
 __device__ __forceinline__ T ks_rhs(const T* __restrict__ y, T M, T a, T* __restrict__ dy, T& hf, T& s) {
     const T x = y[0], yy = y[1], z = y[2], px = y[3], py = y[4], pz = y[5];

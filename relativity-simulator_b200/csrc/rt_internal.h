@@ -20,8 +20,8 @@ enum : uint32_t {
     BF_DISK = 1u << 0,          // thin disk present
     BF_EARLY_CAPTURE = 1u << 1, // Carter early capture allowed
     BF_MIXED = 1u << 2,         // mixed-precision stages
-    BF_FAST_RANGE = 1u << 3     // Boyer-Lindquist: the stages' reciprocal stays far from the ends of the
-                                // range (the straight-line form of rt_fast_math.h gives the same values)
+    BF_FAST_RANGE = 1u << 3     // the stages' straight-line reciprocal (rt_fast_math.h) gives the ordinary
+                                // one's values; Kerr-Schild: or a NaN
 };
 
 // Mixed mode: the near-critical band (M, distance of a ray's constants from
@@ -29,6 +29,13 @@ enum : uint32_t {
 // traced in FP64 from their first step, at a tolerance graded with their
 // distance from the curve.
 constexpr float kDefaultCriticalBand = 1.0f;
+
+// Mass up to which a hole's FP64 Kerr-Schild stages take the straight-line reciprocal
+// (rt_fast_math.h).  Its argument is about r^6, and from 2^1022 on (r = 1.2e51) it gives 0
+// instead of NaN: a hole's field, M / r, would drop out unnoticed.  Up to this mass the
+// field is below 1e-18 there, which is nothing beside the momentum.  The attempts of a
+// heavier hole's rays are all made again with the ordinary operations.
+constexpr double kFastMaxMass = 1e33;
 
 // Per-camera constants, precomputed once on the host in FP64 (the same
 // operations the reference performs per pixel that do not depend on the pixel:
@@ -195,12 +202,12 @@ struct TraceArgs {
 // (software_compute_engine.hpp:2738-2798) builds it.
 constexpr uint32_t kMaxSources = 16;
 struct alignas(16) MsSource {
-    double pos[3], m;
+    double pos[3], m_fast;  // the mass for the straight-line stages: NaN above kFastMaxMass
     double axis[3], a;
     double fx[3], rh;
     double fy[3], req;
     double disk_in, disk_out;  // disk_in < 0: no disk
-    double pad0, pad1;
+    double m, pad0;
 };
 
 // Per-camera constants of a multi-source bundle.

@@ -129,7 +129,7 @@ __device__ __forceinline__ void ms_terms(const MsSource* __restrict__ const* sp,
         const MsSource& s = *sp[u];
         const double* x = X[u];
         const double px = P[u][0], py = P[u][1], pz = P[u][2];
-        const double M = s.m, a = s.a;
+        const double M = FAST ? s.m_fast : s.m, a = s.a;
         const double a2 = __dmul_rn(a, a), z2 = __dmul_rn(x[2], x[2]);
         const double r2 = R2[u], inv_r = IR[u];
         const double r = __dmul_rn(r2, inv_r);
@@ -198,7 +198,7 @@ __device__ __forceinline__ double ms_rhs(const MsSource* __restrict__ src, uint3
             for (int u = 0; u < U; ++u) {
 #pragma unroll
                 for (int k = 0; k < 6; ++k) dy[k] = __dadd_rn(dy[k], term[u][k]);
-                cap = fmin(cap, fmax(r[u] - sp[u]->rh, 0.01 * sp[u]->m));
+                cap = fmin(cap, fmax(r[u] - sp[u]->rh, 0.01 * (FAST ? sp[u]->m_fast : sp[u]->m)));
                 if (r[u] < cap_scale * sp[u]->rh && in == 0x7fffffff) in = static_cast<int>(base + u);
             }
         }
@@ -210,7 +210,7 @@ __device__ __forceinline__ double ms_rhs(const MsSource* __restrict__ src, uint3
         if (i < n) {
             const MsSource* sp[1] = {src + i};
             ms_terms<1, FAST>(sp, y, term, r);
-            cap = fmin(cap, fmax(r[0] - sp[0]->rh, 0.01 * sp[0]->m));
+            cap = fmin(cap, fmax(r[0] - sp[0]->rh, 0.01 * (FAST ? sp[0]->m_fast : sp[0]->m)));
             if (r[0] < cap_scale * sp[0]->rh && in == 0x7fffffff) in = static_cast<int>(i);
         } else {
 #pragma unroll
@@ -403,7 +403,7 @@ __device__ __forceinline__ double ms_field(const MsSource& s, const double* __re
                          __dmul_rn(__fma_rn(r, x[1], -__dmul_rn(a, x[0])), inv_rpa), __dmul_rn(x[2], inv_r)};
 #pragma unroll
     for (int i = 0; i < 3; ++i) kw[i] = ms_world(s, k, i);
-    return __dmul_rn(__dmul_rn(__dmul_rn(s.m, r2), r), __dmul_rn(rpa, q));
+    return __dmul_rn(__dmul_rn(__dmul_rn(FAST ? s.m_fast : s.m, r2), r), __dmul_rn(rpa, q));
 }
 
 // Projection of p onto H = 0 along n = dH/dp, closest root; returns |H| before (NaN,

@@ -718,7 +718,8 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
             } else {
                 fp64_stages<true, NEAR_PASS>(y, k1, hh, M, a, root, y5, kA, est, dense5, r5, hf5, s5);
                 const double probe = root ? y5[2] : est[2];
-                if (probe != probe) {  // a stage left the fast forms' range (or the state is NaN)
+                // a stage left the fast forms' range (or the state is NaN), or may have unnoticed
+                if (probe != probe || !(Bp->flags & BF_FAST_RANGE)) {
                     double io[39];
 #pragma unroll
                     for (int i = 0; i < 6; ++i) {
