@@ -439,8 +439,7 @@ __device__ __noinline__ void bl_finish(const BlDesc* __restrict__ Bp, BlCold<BLO
 // VOL: hydro model 2, each accepted step's chord through the Fishbone-Moncrief
 // torus gathered into the ray's record (args.cont.vol)
 // FAST: the straight-line reciprocal of the step's right-hand sides, the same values
-// without a special-case test and branch in each (1024^2 Kerr-Newman image 22.7 / 22.0
-// ms); every camera of the launch has BF_FAST_RANGE.
+// (1024^2 Kerr-Newman image 22.0 / 21.5 ms); every camera of the launch has BF_FAST_RANGE.
 // ONE: one camera, its constants read as kernel parameters (BlArgs::one) instead of
 // loads each step waits for (1024^2 Kerr-Newman image 22.05 / 21.44 ms).
 template <int BLOCK, bool VOL, bool FAST, bool ONE>

@@ -8,6 +8,7 @@ import subprocess
 
 import numpy as np
 import pytest
+from test_fast_math_ones_host import close_to_midpoints
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "relativity-simulator_b200", "csrc")
@@ -45,6 +46,12 @@ def _values(lo, hi, n, seed):
 @pytest.mark.parametrize("lo,hi", [(-60, 60), (-900, -860), (960, 1019), (-900, 1019)])
 def test_results_are_the_devices_own(fast, lo, hi):
     rcp, root, rcp_rn, root_rn = fast(_values(lo, hi, 1 << 22, 1000 + hi))
+    np.testing.assert_array_equal(rcp, rcp_rn)
+    np.testing.assert_array_equal(root, root_rn)
+
+
+def test_reciprocals_next_to_midpoints(fast):
+    rcp, root, rcp_rn, root_rn = fast(close_to_midpoints(-900, 1019))
     np.testing.assert_array_equal(rcp, rcp_rn)
     np.testing.assert_array_equal(root, root_rn)
 
