@@ -375,7 +375,8 @@ rt_status rt_set_launch_config(rt_handle* h, const rt_launch_config* cfg);
  * hydro_model 2.  rt_shading_defaults
  * gives the reference's defaults for the disk and the tonemap, GpuSkyProfile's
  * defaults in sky, and sky_enabled = 0 (black behind the disk; set it to 1 for
- * the reference's sky). */
+ * the reference's sky).  rt_set_shading(h, NULL) turns shading off and gives
+ * back the torus's scratch memory (up to 4 GB after hydro_model 2). */
 void rt_shading_defaults(rt_shading* s);
 rt_status rt_set_shading(rt_handle* h, const rt_shading* s);
 /* GpuSkyProfile's defaults, and one field by name (see rt_sky_profile):

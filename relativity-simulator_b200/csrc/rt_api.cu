@@ -111,6 +111,12 @@ rt_status cuda_fail(rt_handle* h, cudaError_t e, const char* where) {
         if (e_ != cudaSuccess) return cuda_fail((h), e_, #call); \
     } while (0)
 
+void release(DevBuf& b) {
+    if (b.ptr) cudaFree(b.ptr);
+    b.ptr = nullptr;
+    b.bytes = 0;
+}
+
 rt_status ensure(rt_handle* h, DevBuf& b, size_t bytes) {
     if (b.bytes >= bytes) return RT_OK;
     if (b.ptr) {
@@ -123,18 +129,18 @@ rt_status ensure(rt_handle* h, DevBuf& b, size_t bytes) {
     b.bytes = 0;
     const size_t grow = std::max(bytes, b.bytes + b.bytes / 2);
     cudaError_t e = cudaMalloc(&b.ptr, grow);
+    if (e == cudaErrorMemoryAllocation && h->path_pages.ptr) {
+        // the torus's points are the one buffer that a dispatch can do without (reserve_path)
+        cudaGetLastError();
+        release(h->path_pages);
+        e = cudaMalloc(&b.ptr, grow);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return cuda_fail(h, e, "cudaMalloc");
     }
     b.bytes = grow;
     return RT_OK;
-}
-
-void release(DevBuf& b) {
-    if (b.ptr) cudaFree(b.ptr);
-    b.ptr = nullptr;
-    b.bytes = 0;
 }
 
 rt_status ensure_host_bundles(rt_handle* h, size_t n) {
@@ -236,20 +242,27 @@ rt_status launch_two_pass(rt_handle* h, uint32_t n_bundles, uint64_t total, cons
 
 // A torus-shaded Kerr-Schild trace in parts whose steps' points fit the page pool: 64
 // points (1.5 KB) a page, five pages a ray at rtol 1e-10 (an edge-on frame of a hole of
-// spin 0.998 uses three), more at a tighter tolerance or step cap, at most 4 GB.  False:
-// the pool could not be had, or the parts would be so small that each is bound by its
-// longest ray (10 ms at spin 0.998; a part of 2^17 rays traces as long).
+// spin 0.998 uses three), more at a tighter tolerance or step cap, at most 4 GB and at most
+// a quarter of the device memory that is free when the pool grows, so that handles and
+// programs that share a GPU leave one another room.  False: the pool could not be had, or
+// the parts would be so small that each is bound by its longest ray (10 ms at spin 0.998; a
+// part of 2^17 rays traces as long).
 constexpr uint64_t kMaxPathPages = 2'600'000, kMinPathPart = 1u << 17;
 bool reserve_path(rt_handle* h, uint64_t total, PathOut& path, uint64_t& part) {
     const BundleDesc& b = h->host_bundles[0];
+    constexpr uint64_t page_bytes = sizeof(double) * kPathPageDoubles;
     const double scale = std::max(1.0, std::pow(1e-10 / std::max(b.rtol, 1e-16), 0.2)) * std::max(1.0, 0.1 / b.cap_c);
     const uint64_t per_ray = static_cast<uint64_t>(std::ceil(5.0 * std::min(scale, 1e3)));
-    part = std::max<uint64_t>(1, std::min<uint64_t>(total, kMaxPathPages / per_ray));
-    if (part < std::min(total, kMinPathPart)) return false;
-    const uint64_t pages = std::min<uint64_t>(part * per_ray, kMaxPathPages);
-    if (ensure(h, h->path_pages, sizeof(double) * kPathPageDoubles * pages) != RT_OK ||
+    uint64_t pages = std::min<uint64_t>(total * per_ray, kMaxPathPages);
+    const uint64_t held = h->path_pages.bytes / page_bytes;
+    size_t free_bytes = 0, all_bytes = 0;
+    if (pages > held && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess)
+        pages = std::min(pages, std::max(held, (free_bytes + h->path_pages.bytes) / 4 / page_bytes));
+    part = std::min<uint64_t>(total, pages / per_ray);
+    if (part == 0 || part < std::min(total, kMinPathPart)) return false;
+    if (ensure(h, h->path_pages, page_bytes * pages) != RT_OK ||
         ensure(h, h->path_rays, sizeof(uint32_t) * 4 * total) != RT_OK ||
-        ensure(h, h->path_cursor, kPathCursorBytes) != RT_OK) {
+        ensure(h, h->path_cursor, kPathCursorBytes) != RT_OK || !h->path_pages.ptr) {
         h->error.clear();  // the tracer that gathers as it goes needs no pool
         return false;
     }
@@ -1148,6 +1161,10 @@ rt_status rt_set_shading(rt_handle* h, const rt_shading* s) {
     if (!h) return RT_ERR_INVALID_ARG;
     if (!s) {
         h->shade_on = false;
+        if (h->path_pages.ptr) {  // up to 4 GB (reserve_path); waits for the device
+            RT_CUDA(h, cudaSetDevice(h->device));
+            release(h->path_pages);
+        }
         return RT_OK;
     }
     rt_camera probe;
