@@ -1033,9 +1033,13 @@ void launch_group(MsArgs args, int sm_count, cudaStream_t s) {
 // ray's chain of attempts, each a chain of source terms) four or eight.  The lanes of
 // a group repeat everything but the source terms, so this pays only while a ray has
 // several sources and the groups about fit on the device at once.  FP64 at 1 / 4 / 8
-// lanes (ms), 5 holes: 64x64 11.4 / 9.4 / 6.8, 160x120 12.7 / 10.8 / 12.4, 200x150
-// 13.5 / 13.7 / 17.2; 16 holes: 64x64 39.0 / 19.0 / 14.3, 160x120 41.8 / 29.9 / 33.1,
-// 200x150 42.2 / 39.9 / 47.6, 240x180 47.6 / 52.4 / 64.5; 2 holes: 160x120 6.8 / 7.2.
+// lanes (ms, means of three scenes):
+//   holes    64x64             128x96            160x120           200x150           240x180
+//    2    7.4 / 7.7 / 8.7   7.7 / 8.1 / 10.6  8.4 / 8.6 / 12.4  8.0 / 10.0 / 14.9 8.4 / 11.3 / 18.7
+//    3    8.8 / 7.1 / 7.9   9.6 / 7.5 / 9.4   9.8 / 8.0 / 11.4  9.8 / 9.0 / 13.6  10.5 / 10.2 / 17.7
+//    4   10.0 / 6.4 / 7.2  10.2 / 6.8 / 9.5  10.9 / 8.1 / 12.2 10.9 / 9.6 / 15.7  12.4 / 11.8 / 20.6
+//    5   11.6 / 9.3 / 7.3  11.9 / 10.2 / 9.7 12.7 / 11.5 / 12.8 12.3 / 14.3 / 17.2 14.1 / 17.6 / 22.2
+//    8   20.8 / 11.7 / 9.3 22.5 / 13.6 / 12.9 23.5 / 15.7 / 17.0 24.0 / 18.8 / 22.3 26.0 / 23.3 / 29.2
 int group_lanes(uint64_t rays, uint32_t sources, int sm_count) {
     const uint64_t sm = static_cast<uint64_t>(sm_count);
     if (sources >= 5 && rays <= 32 * sm) return 8;
