@@ -1025,9 +1025,22 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
 
 // The trace of a small torus-shaded frame is bound by its longest rays' chains of steps
 // (3,700 where the mean is 320): 8 warps per SM, whose steps take less time.  A large one
-// is bound by throughput: 12.  Measured at 8 / 12: 64x36 3.0 / 3.2 ms, 213x119 4.2 / 4.5,
-// 640x360 at spin 0.998 13.6 / 14.6 and at 0.9 9.9 / 9.0, 1920x1080 72.2 / 67.2.
-constexpr uint64_t kTorusLeanRaysPerSm = 2048;
+// is bound by throughput: 12.  Near the largest spin the rays that plunge take several
+// times the steps, and the line lies higher.  Measured at 12 / 8 (ms), each at
+// inclinations of 80, 60 and 17 degrees:
+//   320x180 (389 rays an SM)  spin 0.9   5.2/4.3    5.4/4.9    8.0/8.8
+//                                  0.99  8.9/7.9    7.8/6.9   10.0/9.1
+//   480x270 (876)             spin 0.9   6.8/5.8    6.2/6.9   15.4/16.0
+//                                  0.99  9.5/8.0    9.2/7.7   15.1/16.3
+//   640x360 (1557)            spin 0.9   8.0/8.6    8.9/9.3   25.0/26.0
+//                                  0.98 10.6/10.3  10.3/9.7   24.9/25.7
+//                                  0.99 12.6/10.9  12.1/10.6  24.6/25.6
+//   853x480 (2766)            spin 0.9  13.0/13.8  13.7/13.8  42.2/42.9
+//                                  0.99 17.5/17.4  14.1/16.3  42.4/43.3
+// Spins 0 and 0.6 at 500 rays an SM 3.8/3.6 and 5.2/4.9, at 1,000 5.6/6.1 and 6.5/7.3;
+// spin 0.998 at 2,000 22.4/18.5.
+constexpr uint64_t kTorusLeanRaysPerSm = 640, kTorusLeanRaysPerSmExtremal = 2048;
+constexpr double kTorusExtremalSpin = 0.98;
 constexpr uint32_t kSampleBlock = 64;
 
 // unshaded launches (CONT = 0), shaded ones that follow rays through the
@@ -1593,7 +1606,9 @@ int enqueue_torus(const TraceArgs& base, int sm_count, uint32_t ctas_per_sm, cha
     args.in_queue = args.path.order;
     args.in_count = args.path.cursor + PC_TOTAL;
     void* params[] = {&args};
-    const bool lean = args.total_rays <= kTorusLeanRaysPerSm * static_cast<uint64_t>(sm_count);
+    const bool extremal = std::fabs(args.one.a) >= kTorusExtremalSpin * args.one.m;
+    const bool lean = args.total_rays <=
+                      (extremal ? kTorusLeanRaysPerSmExtremal : kTorusLeanRaysPerSm) * static_cast<uint64_t>(sm_count);
     cudaLaunchKernel(lean ? reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, 8>)
                           : reinterpret_cast<const void*>(&trace_kernel_t<128, false, false, PASS_SINGLE, 3, 12>),
                      dim3(static_cast<uint32_t>(sm_count) * std::min(ctas_per_sm, lean ? 2u : 3u)), dim3(128), params, 0,
