@@ -482,11 +482,9 @@ struct ContinuationScope {
     ~ContinuationScope() { end_continuation_state(h); }
 };
 
-// Enqueue the shading pass over n traced rays (after the trace, same stream).
-rt_status shade_launch(rt_handle* h, const rt_camera* cam, const rt_ray_out& dev, rt_pixel_out* pixels, size_t n,
-                       cudaStream_t s, bool prepared = false) {
-    rt_status st;
-    if (!prepared && (st = shade_prepare(h, cam, s)) != RT_OK) return st;
+// Enqueue the shading pass over n traced rays (after shade_prepare and the trace, same
+// stream).
+rt_status shade_launch(rt_handle* h, rt_pixel_out* pixels, size_t n, cudaStream_t s) {
     launch_shade(static_cast<const ShadeDesc*>(h->shade_desc.ptr), nullptr, nullptr, nullptr, nullptr, h->cur_cont, pixels,
                  n, s);
     RT_CUDA(h, cudaGetLastError());
@@ -1240,7 +1238,7 @@ rt_status rt_dispatch_device(rt_handle* h, const rt_camera* cam, rt_pixel_out* p
         if (shade && (st = shade_prepare(h, cam, s)) != RT_OK) return st;
         if (shade && (st = begin_continuation(h, n, false, false, s)) != RT_OK) return st;
         if ((st = bl_launch(h, cam, 0, cam->screen_width, row0, nrows, 0, OutPtrs{pixels, dev}, s)) != RT_OK) return st;
-        return shade ? shade_launch(h, cam, dev, pixels, n, s, true) : RT_OK;
+        return shade ? shade_launch(h, pixels, n, s) : RT_OK;
     }
     if ((st = ensure_host_bundles(h, 1)) != RT_OK) return st;
     if ((st = ensure(h, h->bundles, sizeof(BundleDesc))) != RT_OK) return st;
@@ -1253,7 +1251,7 @@ rt_status rt_dispatch_device(rt_handle* h, const rt_camera* cam, rt_pixel_out* p
     if (shade && (st = shade_prepare(h, cam, s)) != RT_OK) return st;
     if (shade && (st = begin_continuation(h, n, false, true, s)) != RT_OK) return st;
     if ((st = launch(h, 1, n, OutPtrs{pixels, dev}, cam->precision_mode == RT_PRECISION_MIXED, s)) != RT_OK) return st;
-    return shade ? shade_launch(h, cam, dev, pixels, n, s, true) : RT_OK;
+    return shade ? shade_launch(h, pixels, n, s) : RT_OK;
 }
 
 uint64_t rt_bundle_rays(const rt_camera* cams, uint32_t n) {

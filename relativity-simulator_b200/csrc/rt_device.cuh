@@ -36,112 +36,74 @@ struct DP {
                             D6 = -1453857185.0 / 822651844.0, D7 = 69997945.0 / 29380423.0;
 };
 
-template <typename T>
-__device__ __forceinline__ T rt_rsqrt(T v);
-template <>
-__device__ __forceinline__ double rt_rsqrt<double>(double v) { return rsqrt(v); }
-template <>
-__device__ __forceinline__ float rt_rsqrt<float>(float v) { return rsqrtf(v); }
-
-template <typename T>
-__device__ __forceinline__ T rt_rcp(T v);
-template <>
-__device__ __forceinline__ double rt_rcp<double>(double v) { return 1.0 / v; }
-template <>
-__device__ __forceinline__ float rt_rcp<float>(float v) { return __fdividef(1.0f, v); }  // MUFU rcp
-
-template <typename T>
-__device__ __forceinline__ T rt_sqrt(T v);
-template <>
-__device__ __forceinline__ double rt_sqrt<double>(double v) { return sqrt(v); }
-template <>
-__device__ __forceinline__ float rt_sqrt<float>(float v) {  // MUFU rsqrt based
-    const float w = fmaxf(v, 1e-30f);
-    return w * rsqrtf(w);
-}
-
 // Boyer-Lindquist r of a Kerr-Schild point (kerr_schild_null_integrator.hpp:32-36).
-// FAST (FP64): the root without special cases (rt_fast_math.h); a NaN stays one.
-template <typename T, bool FAST = false>
-__device__ __forceinline__ T bl_r2(T x, T y, T z, T a2) {
-    const T z2 = z * z;
-    const T diff = x * x + y * y + z2 - a2;
+// FAST: the root without special cases (rt_fast_math.h); a NaN stays one.
+template <bool FAST = false>
+__device__ __forceinline__ double bl_r2(double x, double y, double z, double a2) {
+    const double z2 = z * z;
+    const double diff = x * x + y * y + z2 - a2;
     if constexpr (FAST) {
-        const T r2 = T(0.5) * (diff + fast_sqrt(diff * diff + T(4) * a2 * z2));
-        return (r2 < T(1e-24)) ? T(1e-24) : r2;
+        const double r2 = 0.5 * (diff + fast_sqrt(diff * diff + 4.0 * a2 * z2));
+        return (r2 < 1e-24) ? 1e-24 : r2;
     } else {
-        const T r2 = T(0.5) * (diff + rt_sqrt<T>(diff * diff + T(4) * a2 * z2));
-        return fmax(r2, T(1e-24));
+        const double r2 = 0.5 * (diff + sqrt(diff * diff + 4.0 * a2 * z2));
+        return fmax(r2, 1e-24);
     }
 }
 
-// Hamiltonian RHS.  y = (x, y, z, p_x, p_y, p_z); returns r_BL and, through
+// Hamiltonian RHS in FP64.  y = (x, y, z, p_x, p_y, p_z); returns r_BL and, through
 // hf/s, the Kerr-Schild scalar H and s = 1 + k.p at y.
 //   dx/dl = p - 2 H s k
 //   dp/dl = s^2 dH/dx + 2 H s (dk/dx . p)
 // with dk/dx_i . p = dr_i * A + B_i (A, B below) and dH/dx_i = C dr_i (+ D for z).
-// With GRAV = true the position part returns only the gravitational term
-// -2 H s k (the mixed-precision step keeps the free-streaming p in FP64).
-// With FAST = true (FP64) the square root and the reciprocal are the straight-line
+// With FAST = true the square root and the reciprocal are the straight-line
 // forms of rt_fast_math.h: the same values while the reciprocal's argument, about r^6,
 // is below 2^1020, and all six outputs NaN where an argument has no finite seed (sv, a
 // factor of every gravitational term, takes k and with it r, 1/r and 1/(r^2 + a^2)).  A
 // caller looks for that NaN and evaluates again with FAST = false.  It does so too for
 // holes whose field still counts where the reciprocal gives 0 instead (kFastMaxMass).
-template <typename T, bool GRAV = false, bool FAST = false>
-__device__ __forceinline__ T ks_rhs(const T* __restrict__ y, T M, T a, T* __restrict__ dy, T& hf, T& s) {
-    const T x = y[0], yy = y[1], z = y[2], px = y[3], py = y[4], pz = y[5];
-    const T a2 = a * a;
-    const T z2 = z * z;
-    const T r2 = bl_r2<T, FAST>(x, yy, z, a2);
-    const T inv_r = rt_rsqrt<T>(r2);
-    const T r = r2 * inv_r;
-    const T rpa = r2 + a2;
-    const T r4 = r2 * r2;
-    const T den = r4 + a2 * z2;
-    T inv_rpa, inv_den;
-    if constexpr (sizeof(T) == 8) {
-        // one reciprocal for both denominators (r^6 stays far from overflow in FP64)
-        T q;
-        if constexpr (FAST) q = fast_rcp(rpa * den);
-        else q = rt_rcp<T>(rpa * den);
-        inv_rpa = den * q;
-        inv_den = rpa * q;
-    } else {
-        inv_rpa = rt_rcp<T>(rpa);
-        inv_den = rt_rcp<T>(den);
-    }
-    const T r3 = r2 * r;
-    const T H = M * r3 * inv_den;
-    const T k0 = (r * x + a * yy) * inv_rpa;
-    const T k1 = (r * yy - a * x) * inv_rpa;
-    const T k2 = z * inv_r;
-    const T sv = T(1) + k0 * px + k1 * py + k2 * pz;
-    const T two_hs = T(2) * H * sv;
-    if constexpr (GRAV) {
-        dy[0] = -two_hs * k0;
-        dy[1] = -two_hs * k1;
-        dy[2] = -two_hs * k2;
-    } else {
-        dy[0] = px - two_hs * k0;
-        dy[1] = py - two_hs * k1;
-        dy[2] = pz - two_hs * k2;
-    }
-    const T r3d = r3 * inv_den;
-    const T dr0 = r3d * x;
-    const T dr1 = r3d * yy;
-    const T dr2 = r * rpa * z * inv_den;
-    // C = M r^2 (3 a^2 z^2 - r^4) / den^2 and D = -2 M a^2 r^3 z / den^2, grouped so
-    // that FP32 intermediates stay near M / r^2 (no underflow of 1/den^2)
-    const T mr2d = M * r2 * inv_den;
-    const T C = mr2d * ((T(3) * a2 * z2 - r4) * inv_den);
-    const T D = T(-2) * (M * r3 * inv_den) * (a2 * z * inv_den);
-    const T A = inv_rpa * ((x - T(2) * r * k0) * px + (yy - T(2) * r * k1) * py) - inv_r * k2 * pz;
-    const T B0 = inv_rpa * (r * px - a * py);
-    const T B1 = inv_rpa * (r * py + a * px);
-    const T B2 = inv_r * pz;
-    const T s2 = sv * sv;
-    const T G = s2 * C + two_hs * A;
+template <bool FAST = false>
+__device__ __forceinline__ double ks_rhs(const double* __restrict__ y, double M, double a, double* __restrict__ dy,
+                                         double& hf, double& s) {
+    const double x = y[0], yy = y[1], z = y[2], px = y[3], py = y[4], pz = y[5];
+    const double a2 = a * a;
+    const double z2 = z * z;
+    const double r2 = bl_r2<FAST>(x, yy, z, a2);
+    const double inv_r = rsqrt(r2);
+    const double r = r2 * inv_r;
+    const double rpa = r2 + a2;
+    const double r4 = r2 * r2;
+    const double den = r4 + a2 * z2;
+    // one reciprocal for both denominators (r^6 stays far from overflow)
+    double q;
+    if constexpr (FAST) q = fast_rcp(rpa * den);
+    else q = 1.0 / (rpa * den);
+    const double inv_rpa = den * q;
+    const double inv_den = rpa * q;
+    const double r3 = r2 * r;
+    const double H = M * r3 * inv_den;
+    const double k0 = (r * x + a * yy) * inv_rpa;
+    const double k1 = (r * yy - a * x) * inv_rpa;
+    const double k2 = z * inv_r;
+    const double sv = 1.0 + k0 * px + k1 * py + k2 * pz;
+    const double two_hs = 2.0 * H * sv;
+    dy[0] = px - two_hs * k0;
+    dy[1] = py - two_hs * k1;
+    dy[2] = pz - two_hs * k2;
+    const double r3d = r3 * inv_den;
+    const double dr0 = r3d * x;
+    const double dr1 = r3d * yy;
+    const double dr2 = r * rpa * z * inv_den;
+    // C = M r^2 (3 a^2 z^2 - r^4) / den^2 and D = -2 M a^2 r^3 z / den^2
+    const double mr2d = M * r2 * inv_den;
+    const double C = mr2d * ((3.0 * a2 * z2 - r4) * inv_den);
+    const double D = -2.0 * (M * r3 * inv_den) * (a2 * z * inv_den);
+    const double A = inv_rpa * ((x - 2.0 * r * k0) * px + (yy - 2.0 * r * k1) * py) - inv_r * k2 * pz;
+    const double B0 = inv_rpa * (r * px - a * py);
+    const double B1 = inv_rpa * (r * py + a * px);
+    const double B2 = inv_r * pz;
+    const double s2 = sv * sv;
+    const double G = s2 * C + two_hs * A;
     dy[3] = dr0 * G + two_hs * B0;
     dy[4] = dr1 * G + two_hs * B1;
     dy[5] = dr2 * G + two_hs * B2 + s2 * D;
@@ -225,8 +187,8 @@ static __device__ double crossing_fraction(const double* y0, const double* f0, c
                                     double a, double target) {
     const double a2 = a * a;
     double lo = 0.0, hi = 1.0;
-    double flo = sqrt(bl_r2<double>(y0[0], y0[1], y0[2], a2)) - target;
-    double fhi = sqrt(bl_r2<double>(y1[0], y1[1], y1[2], a2)) - target;
+    double flo = sqrt(bl_r2(y0[0], y0[1], y0[2], a2)) - target;
+    double fhi = sqrt(bl_r2(y1[0], y1[1], y1[2], a2)) - target;
     if (!((flo > 0.0) != (fhi > 0.0))) return 1.0;
     int side = 0;
     double t = 1.0, x[3];
@@ -234,7 +196,7 @@ static __device__ double crossing_fraction(const double* y0, const double* f0, c
         t = (lo * fhi - hi * flo) / (fhi - flo);
         if (!(t > lo && t < hi)) t = 0.5 * (lo + hi);
         hermite(y0, f0, y1, f1, h, t, 3, x);
-        const double ft = sqrt(bl_r2<double>(x[0], x[1], x[2], a2)) - target;
+        const double ft = sqrt(bl_r2(x[0], x[1], x[2], a2)) - target;
         if (ft == 0.0 || fabs(hi - lo) < 1e-15 || fabs(ft) < 1e-13 * target) break;
         if ((ft > 0.0) == (fhi > 0.0)) {
             hi = t;
@@ -256,7 +218,7 @@ static __device__ double crossing_fraction(const double* y0, const double* f0, c
 // path hands to its volume tests (boyer_lindquist_from_kerr_schild and
 // spherical_to_cartesian, software_compute_engine.hpp:1063-1066).
 __device__ __forceinline__ void bl_cartesian(const double* x, double a, double* out) {
-    const double r2 = bl_r2<double>(x[0], x[1], x[2], a * a), r = sqrt(r2);
+    const double r2 = bl_r2(x[0], x[1], x[2], a * a), r = sqrt(r2);
     const double k = r / (r2 + a * a);
     out[0] = k * (x[0] * r + x[1] * a);
     out[1] = k * (x[1] * r - x[0] * a);
@@ -272,7 +234,7 @@ __device__ __forceinline__ float pi30_factor(float le, float lp, float order_p1)
 // Kerr-Schild field only (r, H, k) at x.
 __device__ __forceinline__ double ks_field64(const double* x, double M, double a, double* k, double& hf) {
     const double a2 = a * a;
-    const double r2 = bl_r2<double>(x[0], x[1], x[2], a2);
+    const double r2 = bl_r2(x[0], x[1], x[2], a2);
     const double inv_r = rsqrt(r2);
     const double r = r2 * inv_r;
     const double rpa = r2 + a2;

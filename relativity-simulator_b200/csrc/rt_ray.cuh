@@ -52,7 +52,7 @@ struct Cold {
 // from the Kerr-Schild covector through dx^i/dtheta of the map at
 // kerr_schild_null_integrator.hpp:47-53.
 __device__ double carter_q(const double* y, double a) {
-    const double r = sqrt(bl_r2<double>(y[0], y[1], y[2], a * a));
+    const double r = sqrt(bl_r2(y[0], y[1], y[2], a * a));
     const double cos_t = clampd(y[2] / r, -1.0, 1.0);
     const double sin2 = fmax((y[0] * y[0] + y[1] * y[1]) / (r * r + a * a), 1e-30);
     const double sin_t = sqrt(sin2);
@@ -122,7 +122,7 @@ __device__ __noinline__ InitResult init_ray(const BundleDesc* __restrict__ Bp, u
     const double q0 = carter_q(y, B.a);
     double hf, s;
     InitResult res;
-    res.r = ks_rhs<double>(y, B.m, B.a, k1, hf, s);
+    res.r = ks_rhs(y, B.m, B.a, k1, hf, s);
     res.can_early = (B.flags & BF_EARLY_CAPTURE) ? -1 : 0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
@@ -181,7 +181,7 @@ __device__ __noinline__ void finish_ray(const BundleDesc* __restrict__ Bp, ColdT
     if (R.dH) R.dH[o] = S.dH[tid];
     // fields that take work are formed only for callers that asked for them
     if (R.r || R.theta || R.phi) {
-        const double r = sqrt(bl_r2<double>(y[0], y[1], y[2], a * a));
+        const double r = sqrt(bl_r2(y[0], y[1], y[2], a * a));
         if (R.r) R.r[o] = r;
         if (R.theta) R.theta[o] = atan2(sqrt(fmax(__dsub_rn(__dmul_rn(r, r), __dmul_rn(y[2], y[2])), 0.0)), y[2]);
         if (R.phi) {
@@ -254,7 +254,7 @@ __device__ __noinline__ double resume_ray(const BundleDesc* __restrict__ Bp, con
 #pragma unroll
     for (int j = 0; j < PU_COUNT; ++j) uch[j] = pb.u[j * n + ray];
     double hf, sv;
-    const double r = ks_rhs<double>(y, Bp->m, Bp->a, k1, hf, sv);
+    const double r = ks_rhs(y, Bp->m, Bp->a, k1, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         xch[i] = y[i];
@@ -355,7 +355,7 @@ __device__ __forceinline__ void end_continuation(const TraceArgs& args, const Bu
         T[TL_H / 2] = make_double2(hh, interp_target);
         T[TL_M / 2] = make_double2(Bp->m, Bp->a);
     }
-    cont_finish(args.cont, o, n_cross, status, sqrt(bl_r2<double>(yl[0], yl[1], yl[2], Bp->a * Bp->a)), Bp->m);
+    cont_finish(args.cont, o, n_cross, status, sqrt(bl_r2(yl[0], yl[1], yl[2], Bp->a * Bp->a)), Bp->m);
 }
 
 // A ray's end (capture, escape, unfinished): its record and pixel unless it

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(512) shade_kernel(const ShadeDesc* __restrict_
                     // a Kerr-Schild point: r_BL, the azimuth (the pattern is periodic in it)
                     // and the redshift of the circular orbit there
                     const double a = D.disk_spin, x = rk, y = phik;
-                    rk = sqrt(bl_r2<double>(x, y, gk, a * a));
+                    rk = sqrt(bl_r2(x, y, gk, a * a));
                     phik = atan2(y, x) - atan2(a, rk);
                     gk = disk_redshift(D.mass, a, rk, cont.lz[i]);
                 }

@@ -92,7 +92,7 @@ __device__ __forceinline__ void fp64_stages_rolled(const double* __restrict__ y,
             if (root) return;
         }
         double out[6], hf, sv;
-        const double rr = ks_rhs<double>(in, M, a, out, hf, sv);
+        const double rr = ks_rhs(in, M, a, out, hf, sv);
 #pragma unroll
         for (int i = 0; i < 6; ++i) K.k[st][i][tid] = out[i];
         if (st == 5) {
@@ -123,26 +123,26 @@ __device__ __forceinline__ void fp64_stages(const double* __restrict__ y, const 
     double in[6], hf, sv;
 #pragma unroll
     for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A21 * k1[i]);
-    ks_rhs<double, false, FAST>(in, M, a, kA, hf, sv);
+    ks_rhs<FAST>(in, M, a, kA, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A31 * k1[i] + DP::A32 * kA[i]);
-    ks_rhs<double, false, FAST>(in, M, a, k3, hf, sv);
+    ks_rhs<FAST>(in, M, a, k3, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i) in[i] = y[i] + hh * (DP::A41 * k1[i] + DP::A42 * kA[i] + DP::A43 * k3[i]);
-    ks_rhs<double, false, FAST>(in, M, a, k4, hf, sv);
+    ks_rhs<FAST>(in, M, a, k4, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         in[i] = y[i] + hh * (DP::A51 * k1[i] + DP::A52 * kA[i] + DP::A53 * k3[i] + DP::A54 * k4[i]);
-    ks_rhs<double, false, FAST>(in, M, a, k5, hf, sv);
+    ks_rhs<FAST>(in, M, a, k5, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         in[i] = y[i] + hh * (DP::A61 * k1[i] + DP::A62 * kA[i] + DP::A63 * k3[i] + DP::A64 * k4[i] + DP::A65 * k5[i]);
-    ks_rhs<double, false, FAST>(in, M, a, k6, hf, sv);
+    ks_rhs<FAST>(in, M, a, k6, hf, sv);
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         y5[i] = y[i] + hh * (DP::B1 * k1[i] + DP::B3 * k3[i] + DP::B4 * k4[i] + DP::B5 * k5[i] + DP::B6 * k6[i]);
     if (!root) {
-        r5 = ks_rhs<double, false, FAST>(y5, M, a, kA, hf5, s5);
+        r5 = ks_rhs<FAST>(y5, M, a, kA, hf5, s5);
 #pragma unroll
         for (int i = 0; i < 6; ++i)
             est[i] = fabs(hh) * fabs(DP::E1 * k1[i] + DP::E3 * k3[i] + DP::E4 * k4[i] + DP::E5 * k5[i] +
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                                                                            : Be->r_capture;
                     }
                     if (cls == RT_RAY_DISK) {
-                        const double rr = sqrt(bl_r2<double>(xch[12], xch[13], xch[14], Be->a * Be->a));
+                        const double rr = sqrt(bl_r2(xch[12], xch[13], xch[14], Be->a * Be->a));
                         finish_ray(Be, S, tid, RT_RAY_DISK, flags, acc, rej, wind, 0.0, 0.0, rr,
                                    disk_redshift(Be->m, Be->a, rr, S.lz0[tid]), args.out, xch);
                     } else {
@@ -700,21 +700,13 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
             if constexpr (MIXED) {
                 if (k1_fp32) {  // entering the FP64 zone: first stage again in FP64
                     double hf, sv;
-                    ks_rhs<double>(y, M, a, k1, hf, sv);
+                    ks_rhs(y, M, a, k1, hf, sv);
                     k1_fp32 = false;
                     ++n_rhs;
                 }
             }
             if constexpr (ROLLED) {
                 fp64_stages_rolled<BLOCK>(y, k1, hh, M, a, K, tid, root, y5, kA, est, r5, hf5, s5);
-                if constexpr (NEAR_PASS) {
-                    if (y[2] * y5[2] <= 0.0) {  // dense-output term; K holds k2..k7
-#pragma unroll
-                        for (int i = 0; i < 6; ++i)
-                            dense5[i] = hh * (DP::D1 * k1[i] + DP::D3 * K.k[1][i][tid] + DP::D4 * K.k[2][i][tid] +
-                                              DP::D5 * K.k[3][i][tid] + DP::D6 * K.k[4][i][tid] + DP::D7 * kA[i]);
-                    }
-                }
             } else {
                 fp64_stages<true, NEAR_PASS>(y, k1, hh, M, a, root, y5, kA, est, dense5, r5, hf5, s5);
                 const double probe = root ? y5[2] : est[2];
@@ -749,7 +741,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
             const bool done = (ft == 0.0) || (fabs(hi - lo) < 1e-15) ||
                               (fabs(ft) < 1e-13 * (1.0 + fabs(y5[0]) + fabs(y5[1]))) || (rit >= 60);
             if (done) {
-                const double rr = sqrt(bl_r2<double>(y5[0], y5[1], y5[2], a * a));
+                const double rr = sqrt(bl_r2(y5[0], y5[1], y5[2], a * a));
                 if (rr >= Bp->r_in && rr <= Bp->r_out && rr > Bp->rh * 1.02) {
                     // lambda at the root, one rounding in every kernel variant
                     const double lambda_step = S.lambda[tid];
@@ -856,7 +848,7 @@ __global__ void __launch_bounds__(BLOCK, 32 * WARPS / BLOCK) trace_kernel_t(cons
                         // pass); off the disk the step is accepted as it is
                         double xr[18];
                         const double t = dense_disk_root(y, k1, y5, kA, dense5, hh, xr + 12);
-                        const double rr = sqrt(bl_r2<double>(xr[12], xr[13], xr[14], a * a));
+                        const double rr = sqrt(bl_r2(xr[12], xr[13], xr[14], a * a));
                         if (rr >= Bp->r_in && rr <= Bp->r_out && rr > Bp->rh * 1.02) {
                             const int wroot = wind + branch_winding(y[0], y[1], xr[12], xr[13]);
                             if constexpr (!CONT) {
