@@ -57,9 +57,10 @@ RT_FM_FN double refine_rcp(double v, double y) {
 // h = y / 2 to 1 / (2 sqrt(v)): with r = 1/2 - g h, where 2 g h = 1 - 2 r, both are short
 // of their limits by the factor (1 - 2 r)^(1/2) = 1 - r - ..., so g + g r and h + h r
 // leave an error of the order of r^2: 2^-35 and 2^-69.  The correction adds the residual
-// v - g^2 divided by 2 g.
-RT_FM_FN double refine_sqrt(double v, double y) {
-    double g = v * y, h = 0.5 * y;
+// v - g^2 divided by 2 g.  h is left within two ulp of 1 / (2 sqrt(v)).
+RT_FM_FN double refine_sqrt(double v, double y, double& h) {
+    double g = v * y;
+    h = 0.5 * y;
     double r = fma(-g, h, 0.5);
     g = fma(g, r, g);
     h = fma(h, r, h);
@@ -67,6 +68,11 @@ RT_FM_FN double refine_sqrt(double v, double y) {
     g = fma(g, r, g);
     h = fma(h, r, h);
     return fma(fma(-g, g, v), h, g);
+}
+
+RT_FM_FN double refine_sqrt(double v, double y) {
+    double h;
+    return refine_sqrt(v, y, h);
 }
 
 // On the host, which has no such seeds, the operations themselves.
@@ -80,14 +86,22 @@ RT_FM_FN double fast_rcp(double v) {
 #endif
 }
 
-RT_FM_FN double fast_sqrt(double v) {
+// sqrt(v), and 1 / (2 sqrt(v)) within two ulp from the same steps.
+RT_FM_FN double fast_sqrt(double v, double& half_inverse) {
 #ifdef __CUDA_ARCH__
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-    return refine_sqrt(v, y);
+    return refine_sqrt(v, y, half_inverse);
 #else
-    return std::sqrt(v);
+    const double root = std::sqrt(v);
+    half_inverse = 0.5 / root;
+    return root;
 #endif
+}
+
+RT_FM_FN double fast_sqrt(double v) {
+    double half_inverse;
+    return fast_sqrt(v, half_inverse);
 }
 
 }  // namespace relsim

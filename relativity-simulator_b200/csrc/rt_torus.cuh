@@ -94,8 +94,8 @@ RT_FM_HD bool fluid(const Torus& t, const EdgeFactor& e_in, double r, double c2,
     if (denom <= 0.0 || delta <= 0.0) return false;
     const double p = rho2 * delta * s2;
     const double ratio = denom * fast_rcp(p), z = (1e30 < ratio) ? 1e30 : ratio;
-    const double root = fast_sqrt(z);
-    const double rest = fma(-root, root, z) * static_cast<double>(0.5f / static_cast<float>(root));
+    double half_inverse;
+    const double root = fast_sqrt(z, half_inverse), rest = fma(-root, root, z) * half_inverse;
     h_above_1 = fma(e_in.hi, root, -1.0) + fma(e_in.hi, rest, e_in.lo * root);
     if (!(h_above_1 > 1e-9)) return false;
     per = p * root;

@@ -1,14 +1,15 @@
-// Host build of one chord's light through the torus (fm_chord, rt_shade.cuh) beside the
-// chord integral as the reference writes it (hydro_disk_shading.hpp:173-269,
+// One chord's light through the torus (fm_chord, rt_shade.cuh) on the host and on the
+// device, beside the chord integral as the reference writes it (hydro_disk_shading.hpp:173-269,
 // hydro/fishbone_moncrief.hpp:118-224, accretion_disk_model.hpp:71-88 and :218-221),
 // here in double and in extended precision.  Test-only.
 #include <cmath>
+#include <vector>
 
 #include "rt_shade.cuh"
 
 using namespace relsim;
 
-namespace {
+namespace chord_test {
 
 template <class R>
 R within(R v, R lo, R hi) {
@@ -94,16 +95,8 @@ bool chord(const ShadeDesc& D, const double* from, const double* to, double l_ov
     return true;
 }
 
-}  // namespace
-
-// n chords (from and to, l_over_e) through the torus of a unit hole; lambda_um, weight and
-// disk are the spectral table and the disk profile.  err: [2][5][n], the errors of the
-// light (in parts of an opaque chord's), of the opacity and of the redshift against
-// extended precision: fm_chord's, then those of the same integral in double; -1 where no
-// light.  Returns the chords on which the three do not agree whether there is any.
-extern "C" long host_chords(double spin, double gamma, const double* lambda_um, const double* weight, const float* disk,
-                            long n, const double* chords, double* err) {
-    static double table[kPlanckTableDoubles];
+// The descriptor of a unit hole's torus; the table is the caller's.
+ShadeDesc descriptor(double spin, double gamma, const double* lambda_um, const double* weight, const float* disk) {
     ShadeDesc D{};
     const torus::TorusContext c = torus::make_torus(1.0, spin, 6.0, 12.0);
     for (int i = 0; i < 33; ++i) {
@@ -113,24 +106,75 @@ extern "C" long host_chords(double spin, double gamma, const double* lambda_um, 
     for (int i = 0; i < 32; ++i) D.profile[i] = disk[i];
     D.mass = 1.0;
     D.disk_spin = spin;
-    D.fm_valid = c.valid;
     set_torus(D, c, gamma, 0.35, 2.0);
+    return D;
+}
+
+struct Light {
+    double v[5], any;
+};
+
+__host__ __device__ Light light_of(const ShadeDesc& D, const double* v) {
+    ChordLight c{};
+    const bool any = fm_chord(D, v, v + 3, v[6], c);
+    return {{c.rad[0], c.rad[1], c.rad[2], c.opacity, c.z}, any ? 1.0 : 0.0};
+}
+
+__global__ void chord_kernel(const ShadeDesc* D, const double* chords, long n, Light* out) {
+    const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+    if (i < n) out[i] = light_of(*D, chords + 7 * i);
+}
+
+bool on_device(ShadeDesc D, const double* table, const double* chords, long n, Light* out) {
+    char* mem = nullptr;
+    const size_t t = sizeof(double) * kPlanckTableDoubles, d = sizeof(ShadeDesc), c = sizeof(double) * 7 * n;
+    if (cudaMalloc(&mem, t + d + c + sizeof(Light) * n) != cudaSuccess) return false;
+    D.planck = reinterpret_cast<double*>(mem);
+    cudaMemcpy(mem, table, t, cudaMemcpyHostToDevice);
+    cudaMemcpy(mem + t, &D, d, cudaMemcpyHostToDevice);
+    cudaMemcpy(mem + t + d, chords, c, cudaMemcpyHostToDevice);
+    chord_kernel<<<static_cast<unsigned>((n + 63) / 64), 64>>>(reinterpret_cast<ShadeDesc*>(mem + t),
+                                                             reinterpret_cast<double*>(mem + t + d), n,
+                                                             reinterpret_cast<Light*>(mem + t + d + c));
+    const cudaError_t e = cudaMemcpy(out, mem + t + d + c, sizeof(Light) * n, cudaMemcpyDeviceToHost);
+    cudaFree(mem);
+    return e == cudaSuccess;
+}
+
+}  // namespace chord_test
+
+using namespace chord_test;
+
+// n chords (from and to, l_over_e) through the torus of a unit hole, fm_chord on the host or
+// the device; lambda_um, weight and disk are the spectral table and the disk profile.  err:
+// [2][5][n], the errors of the light (in parts of an opaque chord's), of the opacity and of
+// the redshift against extended precision: fm_chord's, then those of the same integral in
+// double; -1 where no light.  Returns the chords on which the three do not agree whether
+// there is any; negative: the device did not run.
+extern "C" long chords(int device, double spin, double gamma, const double* lambda_um, const double* weight,
+                       const float* disk, long n, const double* ends, double* err) {
+    static double table[kPlanckTableDoubles];
+    ShadeDesc D = descriptor(spin, gamma, lambda_um, weight, disk);
     planck_table_fill(D.lambda_um, D.weight, table);
-    D.planck = table;
+    std::vector<Light> ours(n);
+    if (device) {
+        if (!on_device(D, table, ends, n, ours.data())) return -1;
+    } else {
+        D.planck = table;
+        for (long i = 0; i < n; ++i) ours[i] = light_of(D, ends + 7 * i);
+    }
     long odd = 0;
     for (long i = 0; i < n; ++i) {
-        const double* v = chords + 7 * i;
-        ChordLight light{};
+        const double* v = ends + 7 * i;
         double plain[5];
         long double exact[5];
-        const bool a = fm_chord(D, v, v + 3, v[6], light);
+        const bool a = ours[i].any != 0.0;
         const bool b = chord<double>(D, v, v + 3, v[6], plain), e = chord<long double>(D, v, v + 3, v[6], exact);
         odd += a != e || b != e;
-        const double ours[5] = {light.rad[0], light.rad[1], light.rad[2], light.opacity, light.z};
         for (int k = 0; k < 5; ++k) {
             const long double whole = k < 3 ? exact[k] / exact[3] : 1.0L;
             const bool has = a && b && e && whole > 0;
-            err[k * n + i] = has ? static_cast<double>(fabsl(ours[k] - exact[k]) / whole) : -1.0;
+            err[k * n + i] = has ? static_cast<double>(fabsl(ours[i].v[k] - exact[k]) / whole) : -1.0;
             err[(5 + k) * n + i] = has ? static_cast<double>(fabsl(plain[k] - exact[k]) / whole) : -1.0;
         }
     }
