@@ -238,7 +238,7 @@ constexpr double kMinThroughputVol = 0.01;  // the reference's loop condition (t
 // enthalpy, which the powers magnify, outweigh theirs, and a 280x280 frame seen face-on takes
 // 13.1 ms instead of 10.8.
 // Measured, a 640x360 frame with the torus: 68.1 ms before, 32.7 gathered as the
-// tracer goes, 13.9 from the steps' stored points (sample_paths).
+// tracer goes, 13.7 from the steps' stored points (sample_paths).
 struct ChordLight {
     double rad[3], opacity, z;
 };

@@ -2,7 +2,7 @@
 
     python relativity-simulator_b200/trace_once.py [--side 512] [--spin 0.94] [--r-obs 100]
         [--incl 17] [--fov 12] [--precision fp64|mixed] [--repeat 1]
-        [--metric ks|bl] [--charge 0] [--sources N] [--device] [--shade]
+        [--metric ks|bl] [--charge 0] [--sources N] [--device] [--shade] [--hydro 2]
 """
 from __future__ import annotations
 
@@ -49,6 +49,8 @@ def main() -> None:
                     help="shade the pixels (rt_set_shading defaults): rays are followed through the translucent disk")
     ap.add_argument("--sky", action="store_true",
                     help="shade with the procedural sky on (the default sky profile; implies --shade)")
+    ap.add_argument("--hydro", type=int, default=0, choices=[0, 1, 2],
+                    help="hydro model of the shading: 1 Novikov-Thorne, 2 the Fishbone-Moncrief torus (implies --shade)")
     ap.add_argument("--record", choices=["minimal", "bench"], default="minimal",
                     help="outputs written: class and step counts, or the bench's record (class, r, theta, "
                          "phi, r_hit, g) plus the 32-byte pixels")
@@ -71,8 +73,8 @@ def main() -> None:
         srcs = scenes.rt_sources(req.sources)
     with relsim.Tracer(0) as tr:
         tr.set_launch_config(a.block, 0, a.refill, a.rays_per_thread, a.fp64_rolled, a.mixed_single)
-        if a.shade or a.sky:
-            tr.set_shading(relsim.shading(sky_enabled=1) if a.sky else relsim.shading())
+        if a.shade or a.sky or a.hydro:
+            tr.set_shading(relsim.shading(sky_enabled=1 if a.sky else 0, hydro_model=a.hydro))
         dev = None
         if a.device:
             import torch
