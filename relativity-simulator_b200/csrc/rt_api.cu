@@ -243,7 +243,7 @@ rt_status launch_two_pass(rt_handle* h, uint32_t n_bundles, uint64_t total, cons
 // A torus-shaded Kerr-Schild trace in parts whose steps' points fit the page pool: 64
 // points (1.5 KB) a page, five pages a ray at rtol 1e-10 (an edge-on frame of a hole of
 // spin 0.998 uses three), more at a tighter tolerance or step cap, at most 4 GB and at most
-// a quarter of the device memory that is free when the pool grows, so that handles and
+// half of the device memory that is free when the pool grows, so that handles and
 // programs that share a GPU leave one another room.  False: the pool could not be had, or
 // the parts would be so small that each is bound by its longest ray (10 ms at spin 0.998; a
 // part of 2^17 rays traces as long).
@@ -257,7 +257,7 @@ bool reserve_path(rt_handle* h, uint64_t total, PathOut& path, uint64_t& part) {
     const uint64_t held = h->path_pages.bytes / page_bytes;
     size_t free_bytes = 0, all_bytes = 0;
     if (pages > held && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess)
-        pages = std::min(pages, std::max(held, (free_bytes + h->path_pages.bytes) / 4 / page_bytes));
+        pages = std::min(pages, std::max(held, (free_bytes + h->path_pages.bytes) / 2 / page_bytes));
     part = std::min<uint64_t>(total, pages / per_ray);
     if (part == 0 || part < std::min(total, kMinPathPart)) return false;
     if (ensure(h, h->path_pages, page_bytes * pages) != RT_OK ||
